@@ -37,7 +37,7 @@ ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
                 "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr"]
 
-CORE_SOURCES = ["errors.cu", "elementwise.cu", "gemm_simt.cu", "gemm_tcgen05.cu", "gemm_pair.cu",
+CORE_SOURCES = ["errors.cu", "elementwise.cu", "gemm_simt.cu", "gemm_f32.cu", "gemm_tcgen05.cu", "gemm_pair.cu",
                 "sampling.cu", "sampling_cluster.cu", "embed_position.cu", "attention_window_bias.cu",
                 "attention_latent.cu", "attention_latent_decode.cu", "attention_latent_prefill.cu", "ssm.cu", "moe.cu",
                 "stream.cu", "linear_attention.cu", "postnorm.cu", "hyper_connections.cu"]

@@ -1,14 +1,19 @@
 // C[M,N] = A[M,K] * W[N,K]^T on the CUDA cores with 32-bit accumulation.
 //
-// This is the true 32-bit matrix product of the engine (no tensor cores, so no
-// reduced-precision operand mode) and the fallback for bfloat16 shapes the
-// tensor-core kernel refuses.  Each output element is one thread's sequential sum
+// The entry of the engine's true 32-bit matrix product (no tensor cores, so no reduced-precision
+// operand mode): rows of whole 16-byte runs go to gemm_f32.cu.  The kernel here takes the rest and the
+// mixed types, and is the fallback for bfloat16 shapes the tensor-core kernel refuses.  Each output element is one thread's sequential sum
 // over k in ascending order, so a row's result does not depend on which other
 // rows are in the batch.
 //
 // Reference counterpart: gemm_nt_kernel, one thread per output with a scalar K
 // loop (cuda/src/kernels.cu:431-459).
 #include "common.cuh"
+
+// gemm_f32.cu: 32-bit products whose rows are whole 16-byte runs
+bool gemm_f32_takes(const void* a, const void* w, long long K, long long lda, long long ldw);
+int gemm_f32(const float* a, const float* w, float* out, int M, int N, int K, long long lda, long long ldw, long long ldc,
+             cudaStream_t stream);
 
 #define BM 64
 #define BN 64
@@ -76,6 +81,8 @@ AP_EXPORT int ap_gemm_simt(const void* a, int a_dtype, const void* w, int w_dtyp
     AP_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm: bad sizes M=%d N=%d K=%d", M, N, K);
     AP_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm: a leading dimension is below its row length");
     if (M == 0) return AP_OK;
+    if (a_dtype == AP_F32 && w_dtype == AP_F32 && out_dtype == AP_F32 && gemm_f32_takes(a, w, K, lda, ldw))
+        return gemm_f32((const float*)a, (const float*)w, (float*)out, M, N, K, lda, ldw, ldc, stream);
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     AP_REQUIRE(grid.y <= 65535, "gemm: %d rows exceed the grid of the CUDA-core kernel", M);
 #define LAUNCH(TA, TW, TO)                                                      \

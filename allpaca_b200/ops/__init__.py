@@ -775,6 +775,9 @@ def check_kernel_status() -> None:
         raise KernelError(f"the tensor-core matrix product on pairs of SMs gave up waiting (code "
                           f"{int(lib.ap_gemm_tc_pair_status())}: 1 free stage, 2 operands, 3 accumulator, 4 the two "
                           f"CTAs' tensor memory differs); its results are void")
+    if hasattr(lib, "ap_gemm_f32_status") and int(lib.ap_gemm_f32_status()) != 0:
+        raise KernelError(f"the 32-bit matrix product gave up waiting (code {int(lib.ap_gemm_f32_status())}: 1 free stage, "
+                          f"2 operands); its results are void")
     code = gemm_tc_status()
     if code != 0:
         raise KernelError(f"the tensor-core matrix product gave up waiting (code {code}: "

@@ -144,6 +144,7 @@ _OPTIONAL_CORE_SIGNATURES = {
     "ap_gemm_tc_prefers_dual": [_I, _I, _I],
     "ap_gemm_tc_prefers_pair": [_I, _I, _I],
     "ap_gemm_tc_prefers_persistent": [_I, _I, _I],
+    "ap_gemm_f32_status": [],
     "ap_gemm_tc_status": [],
     "ap_gemm_tc_reset_status": [],
 }
