@@ -30,21 +30,22 @@
 #include "common.cuh"
 #include <cooperative_groups.h>
 #include <float.h>
+#include "window_bias.cuh"
 namespace cg = cooperative_groups;
 
 #define QKN_THREADS 128
 #define MAX_HEAD 256              // head sizes the kernels take at full speed (8 value columns per lane)
 #define WIDE_NC 20                // value columns per lane of the kernels built for wider values ...
 #define MAX_WIDE_HEAD (32 * WIDE_NC)   // ... up to 640 (a latent of 512 with 64 rotated dimensions is 576 wide)
-#define BIAS_NONE 0
-#define BIAS_LOG 1
-#define BIAS_LINEAR 2
 
-__device__ __forceinline__ float awb_bias(int kind, float b1, float b2, float dist) {
-    return kind == BIAS_LOG ? b1 * log1pf(b2 * dist) : (kind == BIAS_LINEAR ? b1 * dist : 0.f);
-}
-// the scaled score, bounded by a soft cap where there is one: cap * tanh(score / cap)
-__device__ __forceinline__ float awb_cap(float score, float cap) { return cap > 0.f ? cap * tanhf(score / cap) : score; }
+// attention_window_decode.cu: single rows in bfloat16 whose keys and values are whole 16-byte runs
+bool attention_window_decode_takes(const void* q, const void* cache, int D, int VD, long long page_stride, int RS, int voff);
+int attention_window_decode(const void* q, void* out, const void* cache, const int* block_table, int max_blocks,
+                            const int* seq_start, const int* positions, int nseq, int nh, int nkv, int D, int VD, int P,
+                            long long page_stride, float scale, float softcap, int window, const float* r1, const float* r2,
+                            int RS, int voff, int bias_kind, int keep_first, const float* gate, long long gate_ld,
+                            const float* sink, int max_context, cudaStream_t stream);
+
 // Key tiles a row tile walks: the tiles that hold kept first tokens (0 .. tiles_kept-1), then the
 // tiles from the window's first (tile_win) on; where the two meet or overlap, all tiles from 0.
 __device__ __forceinline__ int awb_next_tile(int tile, int tiles_kept, int tile_win) {
@@ -805,7 +806,12 @@ AP_EXPORT int ap_attention_window_bias(const void* q, void* out, const void* cac
         single_rows = 0;
         other_rows = 1;
     }
-    if (single_rows == 1) {
+    if (single_rows == 1 && dtype == AP_BF16 && attention_window_decode_takes(q, cache, D, VD, page_stride, RS, voff)) {
+        const int rc = attention_window_decode(q, out, cache, block_table, max_blocks, seq_start, positions, nseq, nh, nkv, D, VD,
+                                               P, page_stride, scale, softcap, window, r1, r2, RS, voff, bias_kind, keep_first,
+                                               gate, gate_ld, sink, max_context, stream);
+        if (rc != AP_OK || !other_rows) return rc;
+    } else if (single_rows == 1) {
         const int rep = nh / nkv;
         // all query heads of a key/value head in one CTA (every key read once) where that still fills the
         // GPU; else fewer heads per CTA and the keys read again from L2
