@@ -40,11 +40,11 @@ COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",
 CORE_SOURCES = ["errors.cu", "elementwise.cu", "gemm_simt.cu", "gemm_f32.cu", "gemm_tcgen05.cu", "gemm_pair.cu",
                 "sampling.cu", "sampling_cluster.cu", "embed_position.cu", "attention_window_bias.cu",
                 "attention_window_decode.cu",
-                "attention_latent.cu", "attention_latent_decode.cu", "attention_latent_prefill.cu", "ssm.cu", "moe.cu",
+                "attention_latent.cu", "attention_latent_decode.cu", "attention_latent_prefill.cu", "ssm.cu", "moe.cu", "moe_tcgen05.cu",
                 "stream.cu", "linear_attention.cu", "postnorm.cu", "hyper_connections.cu"]
 ATTN_SOURCES = ["errors.cu", "attention.cu", "attention_tc.cu", "attention_tcgen05.cu",
                 "attention_tcgen05_wide.cu"]
-HEADERS = ["common.cuh", "tcgen05.cuh", "window_bias.cuh", "attention_noalloc.h"]
+HEADERS = ["common.cuh", "tcgen05.cuh", "window_bias.cuh", "gated_activation.cuh", "attention_noalloc.h"]
 
 
 class BuildError(RuntimeError):

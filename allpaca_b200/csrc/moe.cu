@@ -16,39 +16,13 @@
 //   moe_combine    delta[t] = sum_k weight[t,k] * o[place(t,k)], in the order of k, on top of `base` where given
 //   gated_act      the activation alone, for a dense feed-forward whose product left [gate | up]
 //
-// Activations (g = gate, u = up):
-//   0 silu:   g / (1 + exp(-g)) * u
-//   1 relu:   max(g, 0) * u
-//   2 clamped sigmoid gate: g' = min(g, limit), u' = clamp(u, -limit, limit); g' * sigmoid(alpha g') * (u' + shift)
-//   3 the tanh form of GELU on g, times u
-//   4 relu2:  max(g, 0)^2 * u
-// Without a gate the same functions of the one sum, with nothing to multiply (all but 2).
-//
-// The products run on the CUDA cores with 32-bit accumulation (every output element one
+// Steps of many pairs in bfloat16 form both products on the tensor cores (moe_tcgen05.cu).  The products here run on the CUDA cores with 32-bit accumulation (every output element one
 // thread's sum over k in ascending order), so a row's result does not depend on where the
 // sort placed it or on what else is in the batch.  Nothing is decided on the host: counts and
 // tiles stay on the device, grids are planned for the worst case and surplus CTAs return.
 #include "common.cuh"
+#include "gated_activation.cuh"
 #include <float.h>
-
-#define ACT_SILU 0
-#define ACT_RELU 1
-#define ACT_CLAMPED 2
-#define ACT_GELU_TANH 3
-#define ACT_RELU2 4
-
-__device__ __forceinline__ float gated_activation(float g, float u, int act, float limit, float alpha, float shift) {
-    if (act == ACT_RELU) return fmaxf(g, 0.f) * u;
-    if (act == ACT_RELU2) { const float r = fmaxf(g, 0.f); return r * r * u; }
-    if (act == ACT_GELU_TANH)        // 0.5 g (1 + tanh(sqrt(2/pi) (g + 0.044715 g^3))) u
-        return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
-    if (act == ACT_CLAMPED) {
-        g = fminf(g, limit);
-        u = fminf(fmaxf(u, -limit), limit);
-        return g / (1.0f + expf(-alpha * g)) * (u + shift);
-    }
-    return g / (1.0f + expf(-g)) * u;
-}
 
 // ---- the activation alone ------------------------------------------------------------
 template <typename TI, typename TO>

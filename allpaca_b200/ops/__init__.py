@@ -778,6 +778,9 @@ def check_kernel_status() -> None:
     if hasattr(lib, "ap_gemm_f32_status") and int(lib.ap_gemm_f32_status()) != 0:
         raise KernelError(f"the 32-bit matrix product gave up waiting (code {int(lib.ap_gemm_f32_status())}: 1 free stage, "
                           f"2 operands); its results are void")
+    if hasattr(lib, "ap_moe_tc_status") and int(lib.ap_moe_tc_status()) != 0:
+        raise KernelError(f"the experts' products on the tensor cores gave up waiting (code {int(lib.ap_moe_tc_status())}: "
+                          f"1 free stage, 2 operands, 3 accumulator); their results are void")
     code = gemm_tc_status()
     if code != 0:
         raise KernelError(f"the tensor-core matrix product gave up waiting (code {code}: "
@@ -788,7 +791,7 @@ from .mixers import (attention_window_bias, causal_conv, embed_sinusoid_norm, ga
                      head_project, latent_decode, latent_decode_takes, latent_gather, latent_prefill,
                      latent_prefill_takes, latent_prepare, qk_norm_store, ssm_scan)
 from . import routed  # noqa: E402,F401
-from .routed import (gated_act, moe_combine, moe_down, moe_gate_up, moe_gather, moe_max_tiles,  # noqa: E402
+from .routed import (gated_act, moe_combine, moe_down, moe_gate_up, moe_gather, moe_max_tiles, moe_products, moe_products_taken,  # noqa: E402
                      moe_route, moe_route_rows, moe_sort)
 from .stream import add_dyt, bias_act, dyt_shift, stream_mix, stream_norm  # noqa: E402
 from .recurrent import exp_gates, gated_postnorm, gated_row_add, head_norm_gate, linear_scan  # noqa: E402

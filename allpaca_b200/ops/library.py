@@ -87,6 +87,10 @@ _CORE_SIGNATURES = {
     "ap_moe_max_tiles": [_I, _I],
     # int ap_moe_sort(chosen, perm, place, tiles, offsets, pairs, E, real, stream)
     "ap_moe_sort": [_P, _P, _P, _P, _P, _I, _I, _I, _P],
+    # int ap_moe_tc_takes(a, w, pairs, E, N, K)
+    "ap_moe_tc_takes": [_P, _P, _I, _I, _I, _I],
+    # int ap_moe_tc(a, w, out, out_dtype, first, pairs, E, N, K, gated, act, limit, alpha, shift, pair_scale, perm, stream)
+    "ap_moe_tc": [_P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _F, _F, _P, _P, _P],
     "ap_moe_gather": [_P, _P, _P, _I, _I, _I, _P],
     # int ap_moe_gate_up(a, a_dtype, w, w_dtype, y, y_dtype, perm, top, tiles, pairs, E, F, K, gated, act, limit,
     #                    alpha, shift, pair_scale, stream)
@@ -145,6 +149,7 @@ _OPTIONAL_CORE_SIGNATURES = {
     "ap_gemm_tc_prefers_pair": [_I, _I, _I],
     "ap_gemm_tc_prefers_persistent": [_I, _I, _I],
     "ap_gemm_f32_status": [],
+    "ap_moe_tc_status": [],
     "ap_gemm_tc_status": [],
     "ap_gemm_tc_reset_status": [],
 }

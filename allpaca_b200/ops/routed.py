@@ -166,6 +166,43 @@ def moe_down(y: torch.Tensor, w: torch.Tensor, o: torch.Tensor, tiles: torch.Ten
          tiles.data_ptr(), pairs, int(experts or E), H, F, stream_handle())
 
 
+def moe_products_taken(a: torch.Tensor, w: torch.Tensor, pairs: int) -> bool:
+    """Whether :func:`moe_products` is the way for ``pairs`` rows of ``a``'s width and ``w [E, N, K]``."""
+    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or not w.is_cuda:
+        return False
+    E, N, K = w.shape
+    return bool(core().ap_moe_tc_takes(a.data_ptr(), w.data_ptr(), int(pairs), E, N, K))
+
+
+def moe_products(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, first: torch.Tensor, gated: bool = False,
+                 activation: Optional[str] = None, limit: float = 0.0, alpha: float = 1.0, shift: float = 0.0,
+                 pair_scale: Optional[torch.Tensor] = None, perm: Optional[torch.Tensor] = None) -> None:
+    """``out[p] = a[p] W[e]^T`` for the rows ``first[e] <= p < first[e + 1]`` of every expert, on the tensor cores:
+    bfloat16 ``a [pairs, K]`` in grouped order, ``w [E, N, K]``, ``first`` int32 of at least ``E + 1``; rows from
+    ``first[E]`` on are left alone.  ``activation``: of the 32-bit sums (:func:`gated_act`); with ``gated`` ``w`` is
+    ``[E, 2N, K]`` (gate rows, then up rows of each expert) and ``out[p] = act(gate, up)``.  ``pair_scale`` (32-bit, by
+    ``perm[p]``): multiplies the sums before the activation."""
+    _check(a, "a", torch.bfloat16, 2)
+    _check(w, "w", torch.bfloat16, 3)
+    _check(out, "out", dims=2)
+    _check(first, "first", torch.int32, 1)
+    pairs, N = out.shape
+    E, NW, K = w.shape
+    if NW != (2 * N if gated else N) or tuple(a.shape) != (pairs, K) or first.shape[0] < E + 1:
+        raise KernelError(f"moe_products: shapes disagree: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    if pair_scale is not None:
+        _check(pair_scale, "pair_scale", torch.float32, 1)
+        if perm is None or perm.shape[0] < pairs or pair_scale.shape[0] < pairs:
+            raise KernelError("moe_products: scales need one entry per pair and the permutation")
+        _check(perm, "perm", torch.int32, 1)
+    if gated and activation is None:
+        raise KernelError("moe_products: gated experts need an activation")
+    call(core(), "ap_moe_tc", a.data_ptr(), w.data_ptr(), out.data_ptr(), dtype_code(out.dtype), first.data_ptr(), pairs, E,
+         N, K, 1 if gated else 0, -1 if activation is None else activation_code(activation), float(limit), float(alpha),
+         float(shift), pair_scale.data_ptr() if pair_scale is not None else 0, perm.data_ptr() if perm is not None else 0,
+         stream_handle())
+
+
 def moe_combine(o: torch.Tensor, place: torch.Tensor, weight: torch.Tensor, delta: torch.Tensor,
                 chosen: Optional[torch.Tensor] = None, real: int = 0, rows: Optional[torch.Tensor] = None,
                 unweighted: bool = False, base: Optional[torch.Tensor] = None) -> None:

@@ -30,12 +30,8 @@ its two products in tiles, and a last pass adds each row's weighted results in t
 its choices.  Counts and tiles never leave the device, so a step can be replayed from a CUDA
 graph, and a row's result does not depend on what else is in the batch.
 
-A bfloat16 step that brings a prompt portion and many pairs takes another way: the experts'
-first positions come to the host (one small copy, and the only wait on the device in the
-step), the rows are gathered in grouped order, and every expert's rows run through the
-tcgen05 products the dense layers use, one pair of launches per expert.  Such a step is never
-recorded as a CUDA graph (only steps of one row per request are), so deciding on the host
-is safe there.
+In bfloat16 the rows are gathered in grouped order and both products of all experts run on the tensor cores, a launch
+each; a step of very few pairs, other types and sizes that TMA cannot address take kernels on the CUDA cores.
 """
 from __future__ import annotations
 
@@ -45,7 +41,6 @@ import torch
 
 from .. import ops
 from .base import BuildEnv, FeedForward, PartError, PartSpec, WeightSpec, build, register
-from .linear import Linear
 
 
 @register("feed_forward", "routed_experts")
@@ -146,13 +141,9 @@ class RoutedExperts(FeedForward):
             self.gate_up = self.router.new_zeros((1, self.first_rows, self.hidden))
             self.down = self.router.new_zeros((1, self.hidden, self.inter))
 
-    #: pairs from which a prompt step's experts run on the tensor cores, one product per expert
-    TENSOR_CORE_MIN_PAIRS = 512
-
-    def _per_expert_on_tensor_cores(self, h, step, pairs: int) -> bool:
-        return (self.env.dtype == torch.bfloat16 and step is not None and step.max_query_len > 1
-                and pairs >= self.TENSOR_CORE_MIN_PAIRS and self.gate_up.dtype == torch.bfloat16
-                and self.hidden % 8 == 0 and self.inter % 8 == 0 and ops.tensor_core_gemm_available())
+    def _on_tensor_cores(self, h, pairs: int) -> bool:
+        return (self.env.dtype == torch.bfloat16 and self.experts > 0 and self.hidden % 8 == 0 and self.inter % 8 == 0
+                and ops.moe_products_taken(h, self.gate_up, pairs))
 
     def forward(self, h: torch.Tensor, step) -> torch.Tensor:
         T = h.shape[0]
@@ -168,30 +159,14 @@ class RoutedExperts(FeedForward):
         tiles = ws.get("moe.tiles", (ops.moe_max_tiles(pairs, self.outputs) + 1, 3), torch.int32)
         y = ws.get("moe.act", (pairs, self.inter), self.env.dtype)
         o = ws.get("moe.out", (pairs, self.hidden), torch.float32)
-        if self._per_expert_on_tensor_cores(h, step, pairs):
-            offsets = ws.get("moe.offsets", (self.outputs + 1,), torch.int32)
-            ops.moe_sort(chosen, perm, place, tiles, self.outputs, offsets, real=self.experts)
-            first = offsets.tolist()                                   # the step waits for the device here
+        if self._on_tensor_cores(h, pairs):
+            first = ws.get("moe.offsets", (self.outputs + 1,), torch.int32)
+            ops.moe_sort(chosen, perm, place, tiles, self.outputs, first, real=self.experts)
             rows = ws.get("moe.rows", (pairs, self.hidden), torch.bfloat16)
             ops.moe_gather(h, rows, perm, self.top)
-            # without a gate the square of relu is applied in the products' epilogues; else by a pass over all pairs
-            fused = not self.gated and self.activation in ops.EPILOGUE_ACTIVATIONS
-            gu = y if fused else ws.get("moe.gate_up", (pairs, self.first_rows),
-                                        torch.bfloat16 if self.gated else torch.float32)
-            for e in range(self.experts):
-                a, b = first[e], first[e + 1]
-                if b > a:
-                    Linear.tensor_core_product(rows[a:b], self.gate_up[e], gu[a:b],
-                                               activation=self.activation if fused else None)
-            if self.gated:
-                ops.gated_act(gu, y, self.activation, False, self.limit, self.alpha, self.shift,
-                              row_scale=weight.view(-1) if on_input else None, scale_index=perm if on_input else None)
-            elif not fused:
-                ops.bias_act(gu, None, y, self.activation)
-            for e in range(self.experts):
-                a, b = first[e], first[e + 1]
-                if b > a:
-                    Linear.tensor_core_product(y[a:b], self.down[e], o[a:b])
+            ops.moe_products(rows, self.gate_up, y, first, gated=self.gated, activation=self.activation, limit=self.limit,
+                             alpha=self.alpha, shift=self.shift, pair_scale=weight.view(-1) if on_input else None, perm=perm)
+            ops.moe_products(y, self.down, o, first)
         else:
             ops.moe_sort(chosen, perm, place, tiles, self.outputs, real=self.experts)
             ops.moe_gate_up(h, self.gate_up, y, perm, self.top, tiles, self.activation, self.limit, self.alpha,
