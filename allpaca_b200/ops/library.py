@@ -56,8 +56,8 @@ _CORE_SIGNATURES = {
     #                       token_seq, block_table, max_blocks, P, page_stride, cos_sin, eps, T, stream)
     "ap_latent_prepare": [_P, _L, _I, _I, _P, _P, _I, _I, _I, _I, _P, _P, _I, _P, _P, _P, _I, _I, _L, _P, _F, _I, _P],
     # int ap_head_project(in, in_dtype, in_ld, in_hs, w, w_dtype, out, out_dtype, out_ld, out_hs, T, H, K, N, tail,
-    #                     tail_dims, cos_sin, stream)
-    "ap_head_project": [_P, _I, _L, _I, _P, _I, _P, _I, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    #                     tail_dims, cos_sin, seq_start, nseq, stream)
+    "ap_head_project": [_P, _I, _L, _I, _P, _I, _P, _I, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P],
     # int ap_latent_gather(cache, dtype, page_stride, P, record, block_table, max_blocks, seq_start, context_lens,
     #                      nseq, out, where, width, total, window, stream)
     "ap_latent_gather": [_P, _I, _L, _I, _I, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _P],

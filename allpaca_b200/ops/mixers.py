@@ -226,12 +226,15 @@ def latent_prepare(proj: torch.Tensor, q_col: int, q_rank: int, q_weight: Option
 
 
 def head_project(inp: torch.Tensor, weight: Optional[torch.Tensor], out: torch.Tensor, heads: int, tail: int = 0,
-                 tail_dims: int = 0, cos_sin: Optional[torch.Tensor] = None) -> None:
-    """``out[t, h, :N] = inp[t, h, :K] @ weight[h]`` for ``weight [heads, K, N]``, every sum 32-bit in
-    ascending ``k``.  ``inp [T, heads*(K + tail)]`` and ``out [T, heads*(N + tail)]``: the ``tail``
+                 tail_dims: int = 0, cos_sin: Optional[torch.Tensor] = None,
+                 singles: Optional[torch.Tensor] = None, num_seqs: int = 0) -> None:
+    """``out[t, h, :N] = inp[t, h, :K] @ weight[h]`` for ``weight [heads, K, N]``, every sum 32-bit in a
+    fixed order.  ``inp [T, heads*(K + tail)]`` and ``out [T, heads*(N + tail)]``: the ``tail``
     numbers behind a head's ``K`` inputs go behind its ``N`` outputs, the first ``tail_dims`` of them
     rotated by ``cos_sin [T, tail_dims/2, 2]`` (entry ``i`` paired with ``i + tail_dims/2``).  With
-    ``weight`` None the ``K`` numbers are copied (``out`` has ``inp``'s shape): a rotation alone."""
+    ``weight`` None the ``K`` numbers are copied (``out`` has ``inp``'s shape): a rotation alone.  ``singles`` (the
+    step's ``seq_start``, of ``num_seqs`` sequences): only the rows of sequences that bring one row are needed; what
+    becomes of the others is not said."""
     if inp.dim() != 2 or not inp.is_cuda or inp.stride(1) != 1:
         raise KernelError("head_project: inp must be a CUDA matrix with contiguous rows (it may be a view of wider rows)")
     _check(out, "out", dims=2)
@@ -255,9 +258,15 @@ def head_project(inp: torch.Tensor, weight: Optional[torch.Tensor], out: torch.T
         if tuple(cos_sin.shape) != (T, tail_dims // 2, 2):
             raise KernelError("head_project: cos_sin must be [T, tail_dims/2, 2]")
         csptr = cos_sin.data_ptr()
+    ssptr = 0
+    if singles is not None:
+        _check(singles, "singles", torch.int32, 1)
+        if singles.shape[0] < num_seqs + 1:
+            raise KernelError("head_project: seq_start is shorter than the sequences")
+        ssptr = singles.data_ptr()
     call(core(), "ap_head_project", inp.data_ptr(), dtype_code(inp.dtype), inp.stride(0), K + tail, weight_ptr,
          weight_code, out.data_ptr(), dtype_code(out.dtype), out.stride(0), N + tail, T, H, K, N,
-         int(tail), int(tail_dims), csptr, stream_handle())
+         int(tail), int(tail_dims), csptr, ssptr, int(num_seqs), stream_handle())
 
 
 CONV_ACTIVATIONS = {None: 0, "silu": 1}

@@ -203,7 +203,9 @@ class LatentAttention(Mixer):
         if singles or not per_head:
             # in the latent space: every row, or (beside the per-head form) the sequences that bring one row
             qa = ws.get("lattn.qa", (T, self.nh * rec), dt)
-            ops.head_project(q, self.uk, qa, self.nh, tail=self.rot, tail_dims=self.rot_dims, cos_sin=cos_sin)
+            only = step.seq_start if per_head else None      # the portions' rows take the per-head form below
+            ops.head_project(q, self.uk, qa, self.nh, tail=self.rot, tail_dims=self.rot_dims, cos_sin=cos_sin,
+                             singles=only, num_seqs=step.num_seqs)
             ol = ws.get("lattn.ol", (T, self.nh * self.R), dt)
             # sequences that bring one row: all heads together against shared key tiles on the tensor cores
             fast = dt == torch.bfloat16 and singles and ops.latent_decode_takes(rec, self.R)
@@ -217,7 +219,7 @@ class LatentAttention(Mixer):
                                           self.nh, 1, rec, self.R, self.scale, W, None, None,
                                           single_rows="skip" if fast else (dt == torch.bfloat16 and singles),
                                           other_rows=others, bias=None, gate=gate, record=rec, value_offset=0, sink=sink)
-            ops.head_project(ol, self.uv, ov, self.nh)
+            ops.head_project(ol, self.uv, ov, self.nh, singles=only, num_seqs=step.num_seqs)
         if per_head:
             # the sequences that bring several rows, on per-head keys and values of all their tokens so far
             # (behind a window: from the first token that the sequence's first row still sees)
