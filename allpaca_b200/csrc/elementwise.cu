@@ -461,6 +461,31 @@ AP_EXPORT int ap_clear_page_tails(void* pages, int elem_bytes, long long run_str
     return AP_OK;
 }
 
+// A step's metadata from pinned host memory (read once each, past the caches) into the device's block: the numbers first ..
+// first + n - 1.  The count numbers from `off` on are token ids: where `tokens` is given number i takes tokens[i - off], or (with
+// `index`, pinned as well) tokens[index[i - off]] where that is not negative.  Plain stream order: later kernels may read the
+// block early.
+__global__ void __launch_bounds__(256)
+stage_step_kernel(const int* __restrict__ host, int* __restrict__ dev, int first, int n, const int* __restrict__ tokens, int off,
+                  int count, const int* __restrict__ index) {
+    const int i = first + blockIdx.x * 256 + threadIdx.x;
+    if (i >= first + n) return;
+    int from = -1;
+    if (tokens != nullptr && i >= off && i < off + count) from = index != nullptr ? __ldcv(index + (i - off)) : i - off;
+    dev[i] = from >= 0 ? tokens[from] : __ldcv(host + i);
+}
+
+AP_EXPORT int ap_stage_step(const int* host, int* dev, int first, int n, const int* tokens, int off, int count,
+                            const int* index, cudaStream_t stream) {
+    AP_REQUIRE(first >= 0 && n >= 0 && off >= 0 && count >= 0, "stage_step: bad sizes first=%d n=%d off=%d count=%d", first, n,
+               off, count);
+    if (n == 0) return AP_OK;
+    AP_REQUIRE(host && dev, "stage_step: a pointer is missing");
+    stage_step_kernel<<<(n + 255) / 256, 256, 0, stream>>>(host, dev, first, n, tokens, off, count, index);
+    AP_CHECK_LAUNCH("stage_step");
+    return AP_OK;
+}
+
 // One thread per pair of elements: (nh + nkv) * half rotated pairs, then nkv * half pairs of V.
 #define ROPE_THREADS 256
 template <typename TI, typename TO>

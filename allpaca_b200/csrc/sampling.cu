@@ -26,10 +26,12 @@ __device__ __forceinline__ unsigned ordered_key(float f) {
 __device__ __forceinline__ bool finite_f(float f) { return fabsf(f) <= FLT_MAX; }
 
 // ---------------------------------------------------------------------------
-// arg-max: first maximum wins; rows with no finite value give token 0.
+// arg-max: first maximum wins; rows with no finite value give token 0.  host_out (here and below; or null): pinned host
+// memory that gets the tokens too, so that no copy of its own stands between this step and the next (5 us of a stream's time for
+// the copy engine to start, 3 for 4 bytes a row).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(SAMP_THREADS)
-argmax_kernel(const float* __restrict__ logits, long long row_stride, int V, int* __restrict__ out) {
+argmax_kernel(const float* __restrict__ logits, long long row_stride, int V, int* __restrict__ out, int* __restrict__ host_out) {
     __shared__ float best_v[32];
     __shared__ int best_i[32];
     const float* row = logits + (size_t)blockIdx.x * row_stride;
@@ -52,16 +54,18 @@ argmax_kernel(const float* __restrict__ logits, long long row_stride, int V, int
     if (threadIdx.x == 0) {
         for (int w = 1; w < SAMP_THREADS / 32; ++w)
             if (best_v[w] > bv || (best_v[w] == bv && best_i[w] < bi)) { bv = best_v[w]; bi = best_i[w]; }
-        out[blockIdx.x] = (bi == 0x7fffffff) ? 0 : bi;
+        const int token = (bi == 0x7fffffff) ? 0 : bi;
+        out[blockIdx.x] = token;
+        if (host_out) host_out[blockIdx.x] = token;
     }
 }
 
-AP_EXPORT int ap_argmax(const float* logits, long long row_stride, int R, int V, int* out,
+AP_EXPORT int ap_argmax(const float* logits, long long row_stride, int R, int V, int* out, int* host_out,
                         cudaStream_t stream) {
     AP_REQUIRE(R >= 0 && V > 0 && row_stride >= V, "argmax: bad sizes R=%d V=%d", R, V);
     if (R == 0) return AP_OK;
     AP_CHECK_PDL_LAUNCH("argmax", ap_launch_pdl(argmax_kernel, dim3(R), dim3(SAMP_THREADS), 0, stream, logits,
-                                                row_stride, V, out));
+                                                row_stride, V, out, host_out));
     return AP_OK;
 }
 
@@ -191,12 +195,17 @@ __device__ int nth_equal(const float* row, int V, float tdiv, const Cut& c0, con
 __global__ void __launch_bounds__(SAMP_THREADS)
 sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
               const float* __restrict__ temperature, const int* __restrict__ top_k,
-              const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out) {
+              const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out,
+              int* __restrict__ host_out) {
     __shared__ SampShared sh;
     __shared__ float red[32];
     const int r = blockIdx.x;
     const float* row = logits + (size_t)r * row_stride;
     const float temp = temperature[r];
+    auto choose = [&](int token) {
+        out[r] = token;
+        if (host_out) host_out[r] = token;
+    };
 
     // maximum (first index) over finite logits; also the greedy answer
     float bv = -INFINITY;
@@ -218,7 +227,7 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
     const int arg = sh.i0 == 0x7fffffff ? 0 : sh.i0;
     __syncthreads();
     if (cnt == 0.f || temp <= 1e-5f) {           // nothing finite -> token 0; greedy -> first maximum
-        if (threadIdx.x == 0) out[r] = arg;
+        if (threadIdx.x == 0) choose(arg);
         return;
     }
     const float tdiv = fmaxf(temp, 1e-5f);
@@ -297,19 +306,19 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
     if (sh.i0 == 0x7fffffff) {       // rounding left the walk short: the last survivor
         if (last >= 0) atomicMax(&sh.i1, last);
         __syncthreads();
-        if (threadIdx.x == 0) out[r] = sh.i1 < 0 ? arg : sh.i1;
+        if (threadIdx.x == 0) choose(sh.i1 < 0 ? arg : sh.i1);
     } else if (threadIdx.x == 0) {
-        out[r] = sh.i0;
+        choose(sh.i0);
     }
 }
 
 // The kernel above: one CTA per row, any vocabulary.
 AP_EXPORT int ap_sample_rows(const float* logits, long long row_stride, int R, int V, const float* temperature,
-                             const int* top_k, const float* top_p, const float* uniform, int* out,
+                             const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out,
                              cudaStream_t stream) {
     AP_REQUIRE(R >= 0 && V > 0 && row_stride >= V, "sample: bad sizes R=%d V=%d", R, V);
     if (R == 0) return AP_OK;
-    sample_kernel<<<R, SAMP_THREADS, 0, stream>>>(logits, row_stride, V, temperature, top_k, top_p, uniform, out);
+    sample_kernel<<<R, SAMP_THREADS, 0, stream>>>(logits, row_stride, V, temperature, top_k, top_p, uniform, out, host_out);
     AP_CHECK_LAUNCH("sample");
     return AP_OK;
 }
@@ -317,15 +326,15 @@ AP_EXPORT int ap_sample_rows(const float* logits, long long row_stride, int R, i
 // sampling_cluster.cu: a cluster of CTAs per row, the row in registers
 extern "C" int ap_sample_cluster_max_vocab(void);
 extern "C" int ap_sample_cluster(const float* logits, long long row_stride, int R, int V, const float* temperature,
-                                 const int* top_k, const float* top_p, const float* uniform, int* out,
+                                 const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out,
                                  cudaStream_t stream);
 
 // One token per row: the cluster kernel where the vocabulary fits its registers (up to 262144
 // entries), else one CTA per row.
 AP_EXPORT int ap_sample(const float* logits, long long row_stride, int R, int V, const float* temperature,
-                        const int* top_k, const float* top_p, const float* uniform, int* out,
+                        const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out,
                         cudaStream_t stream) {
     if (V > 0 && V <= ap_sample_cluster_max_vocab() && R <= 65535)
-        return ap_sample_cluster(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, stream);
-    return ap_sample_rows(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, stream);
+        return ap_sample_cluster(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
+    return ap_sample_rows(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
 }

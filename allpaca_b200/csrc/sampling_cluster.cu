@@ -416,14 +416,28 @@ template <int E>
 __global__ void __launch_bounds__(SC_THREADS, 1)
 sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, int V,
                       const float* __restrict__ temperature, const int* __restrict__ top_k,
-                      const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out) {
+                      const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out,
+                      int* __restrict__ host_out) {
     cg::cluster_group cl = cg::this_cluster();
     __shared__ ScShared sh;
     const int rank = (int)cl.block_rank();
     const int r = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float* src = logits + (size_t)r * row_stride;
-    const float temp = temperature[r];
+    // the row's options may lie in pinned host memory: each is asked for once, while the logits are still being formed
+    __shared__ float option_s[4];
+    ap_pdl_trigger();
+    if (threadIdx.x < 4)
+        option_s[threadIdx.x] = threadIdx.x == 0 ? temperature[r] : threadIdx.x == 1 ? __int_as_float(top_k[r])
+                                : threadIdx.x == 2 ? top_p[r] : uniform[r];
+    ap_pdl_wait();
+    __syncthreads();
+    const float temp = option_s[0], opt_top_p = option_s[2], opt_uniform = option_s[3];
+    const int opt_top_k = __float_as_int(option_s[1]);
+    auto choose = [&](int token) {
+        out[r] = token;
+        if (host_out) host_out[r] = token;
+    };
     const float tdiv = fmaxf(temp, 1e-5f);
     int parity = 0;
 
@@ -496,14 +510,14 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, in
         n_cand += (int)sh.all[c][3];
     }
     if (n_cand == 0 || temp <= 1e-5f) {          // nothing finite -> token 0; greedy -> first maximum
-        if (rank == 0 && threadIdx.x == 0) out[r] = n_cand == 0 ? 0 : arg;
+        if (rank == 0 && threadIdx.x == 0) choose(n_cand == 0 ? 0 : arg);
         cl.sync();
         return;
     }
 
-    const int k = top_k[r];
-    const float pth = top_p[r];
-    const float u = uniform[r];
+    const int k = opt_top_k;
+    const float pth = opt_top_p;
+    const float u = opt_uniform;
     const bool use_k = k > 0 && k < n_cand;
     const bool use_p = pth >= 0.f && pth < 1.f;
     const ScCut none = {0u, 0, 0};
@@ -537,7 +551,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, in
                 const float z = sc_prefix_weights(sh, kept);
                 int i = sc_first_reaching(sh, kept, u * z);
                 if (i >= kept) i = kept - 1;             // rounding left the walk short: the last survivor
-                if (threadIdx.x == 0) out[r] = (int)(sh.list[i] >> 32);
+                if (threadIdx.x == 0) choose((int)(sh.list[i] >> 32));
             }
             cl.sync();
             return;
@@ -616,7 +630,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, in
                     if (token < 0 && run >= target) token = last;
                 }
             }
-            out[r] = token >= 0 ? token : last;
+            choose(token >= 0 ? token : last);
         }
     }
     cl.sync();
@@ -624,21 +638,23 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, in
 
 template <int E>
 static int sc_launch(const float* logits, long long row_stride, int R, int V, const float* temperature,
-                     const int* top_k, const float* top_p, const float* uniform, int* out, cudaStream_t stream) {
+                     const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(SC_CLUSTER, R);
     cfg.blockDim = dim3(SC_THREADS);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = SC_CLUSTER;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = ap_pdl_enabled() ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<E>, logits, row_stride, V, temperature, top_k,
-                                       top_p, uniform, out);
+                                       top_p, uniform, out, host_out);
     AP_REQUIRE(e == cudaSuccess, "sample (cluster): launch failed: %s", cudaGetErrorString(e));
     return AP_OK;
 }
@@ -647,7 +663,7 @@ static int sc_launch(const float* logits, long long row_stride, int R, int V, co
 AP_EXPORT int ap_sample_cluster_max_vocab(void) { return SC_CLUSTER * SC_THREADS * 64; }
 
 AP_EXPORT int ap_sample_cluster(const float* logits, long long row_stride, int R, int V, const float* temperature,
-                                const int* top_k, const float* top_p, const float* uniform, int* out,
+                                const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out,
                                 cudaStream_t stream) {
     AP_REQUIRE(R >= 0 && V > 0 && row_stride >= V, "sample: bad sizes R=%d V=%d", R, V);
     AP_REQUIRE(V <= ap_sample_cluster_max_vocab(), "sample (cluster): a vocabulary of %d exceeds %d", V,
@@ -655,8 +671,8 @@ AP_EXPORT int ap_sample_cluster(const float* logits, long long row_stride, int R
     AP_REQUIRE(R <= 65535, "sample (cluster): %d rows exceed the grid", R);
     if (R == 0) return AP_OK;
     const int per = (V + SC_CLUSTER * SC_THREADS - 1) / (SC_CLUSTER * SC_THREADS);
-    if (per <= 4) return sc_launch<4>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, stream);
-    if (per <= 16) return sc_launch<16>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, stream);
-    if (per <= 32) return sc_launch<32>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, stream);
-    return sc_launch<64>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, stream);
+    if (per <= 4) return sc_launch<4>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
+    if (per <= 16) return sc_launch<16>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
+    if (per <= 32) return sc_launch<32>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
+    return sc_launch<64>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
 }

@@ -10,7 +10,7 @@ concatenated token list of ``forward_batch`` (crates/allpaca-core/src/model.rs:3
 from __future__ import annotations
 
 from dataclasses import dataclass, field
-from typing import Hashable, List, Sequence
+from typing import Hashable, List, Optional, Sequence
 
 import torch
 
@@ -22,6 +22,7 @@ class BatchEntry:
     request: Hashable
     tokens: Sequence[int]
     want: Sequence[int] = ()        # indices into `tokens` whose logits are asked for
+    device_row: Optional[int] = None     # a single row whose token id the device has: its place among the step's device tokens
 
 
 @dataclass

@@ -104,9 +104,9 @@ class LLM:
         """Launch one batch; returns the requests found finished.
 
         One step is kept in flight: while the GPU runs the batch launched here, the host reads
-        the tokens of the batch before it, appends them and decides who is done.  In steady
-        decoding (the same requests, one row each, as in the step before) the new step takes
-        its token ids straight from the device, where the step before left them, so the GPU
+        the tokens of the batch before it, appends them and decides who is done.  Rows that
+        decode take their token ids straight from the device, where the step before left them
+        (:meth:`_device_rows`), beside portions of prompts, whose tokens the host has, so the GPU
         never waits for the host.  A request that a stop token ended is therefore known one
         step late: the row it still had in the step in flight is run for nothing and its
         token dropped.  Requests reach the caller one call after the step that finished them;
@@ -128,12 +128,10 @@ class LLM:
                 finished = finished + self._resolve(prev)
             return self._outputs(finished)
         sampling = [r.request for r in out.rows if r.samples]
-        steady = (prev is not None and len(sampling) == len(out.rows) and len(sampling) == len(prev.sampling)
-                  and all(r.count == 1 for r in out.rows)
-                  and all(a is b for a, b in zip(sampling, prev.sampling)))
-        if steady:
-            entries = [BatchEntry(r.request.request_id, [0], [0]) for r in out.rows]
-            logits = self.runner.step(entries, device_tokens=prev.pending.device)
+        ahead = self._device_rows(prev, out) if prev is not None else None
+        if ahead is not None:
+            entries, tokens = ahead
+            logits = self.runner.step(entries, device_tokens=tokens)
         else:
             if prev is not None:
                 finished = finished + self._resolve(prev)          # the rows planned need the token values
@@ -145,16 +143,45 @@ class LLM:
             # row is dropped; the scheduler still counts it among the planned ones)
             logits = self.runner.step(entries) if entries else None
         seed_default = self.runner.engine.seed
-        live = [q for q in sampling if q.status is not RequestStatus.FINISHED] if not steady else sampling
+        live = [q for q in sampling if q.status is not RequestStatus.FINISHED] if ahead is None else sampling
         us = [uniform(q.params.seed if q.params.seed is not None else seed_default,
                       len(q.output_token_ids) + q.num_pending) for q in live]
         pending = self.sampler.launch(logits, [q.params for q in live], us) if logits is not None else None
         self.stats["steps"] += 1
         self.stats["batched_rows"] += out.num_tokens
-        if steady:
+        if ahead is not None:
             finished = finished + self._resolve(prev)   # while the GPU runs the step just launched
         self._inflight = _InFlight(out, sampling, live, pending)
         return self._outputs(finished)
+
+    @staticmethod
+    def _device_rows(prev: "_InFlight", out):
+        """The entries of the planned rows where these can run before the tokens of the step in flight are here, and those
+        tokens on the device (None where no row needs one): rows that decode name their place among them.  None where the
+        values are needed first: a request was preempted (it will run again from all its tokens), or a portion reaches
+        into tokens that are not here yet."""
+        if prev.pending is None or out.preempted:
+            return None
+        place = {id(q): i for i, q in enumerate(prev.live)}
+        entries, steady = [], len(out.rows) == len(prev.live)
+        for r in out.rows:
+            q = r.request
+            known = q.num_tokens
+            if r.start + r.count <= known:
+                entries.append(BatchEntry(q.request_id, q.token_slice(r.start, r.count), [r.count - 1] if r.samples else []))
+                steady = False
+                continue
+            i = place.get(id(q))
+            if r.count != 1 or r.start != known or q.num_pending != 1 or i is None or not r.samples:
+                return None
+            steady = steady and i == len(entries)
+            entries.append(BatchEntry(q.request_id, [0], [0], i))
+        if steady:                       # the same rows as in the step before: the tokens as they lie there
+            for en in entries:
+                en.device_row = None
+        elif all(en.device_row is None for en in entries):
+            return entries, None
+        return entries, prev.pending.device
 
     def _at_length_limit(self, q: Request) -> bool:
         n = len(q.output_token_ids) + q.num_pending

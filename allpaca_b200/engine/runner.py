@@ -21,6 +21,7 @@ from ..config import EngineConfig
 from ..models import DecoderModel, load_config
 from ..parts import BuildEnv, Workspace
 from ..weights import load_checkpoint
+from .. import ops
 from ..ops import library
 from .batch import BatchEntry, StepBatch
 from .step_builder import build_step
@@ -118,7 +119,8 @@ class ModelRunner:
         ``device_tokens`` (int32 on the device, one per row): the step's token ids are taken
         from there instead of from the entries, whose tokens are then placeholders.  With it a
         caller that chooses the next tokens on the GPU can launch the next step without
-        bringing them to the host first."""
+        bringing them to the host first.  Where an entry names a ``device_row``, such entries take
+        that one of the tokens and all others their own."""
         if self._graphable(entries):
             logits = self._graph_step(entries, device_tokens)
         else:
@@ -188,6 +190,11 @@ class ModelRunner:
         gs.generation = self.workspace.generation
         return logits
 
+    #: numbers of a step's metadata up to which a kernel fetches them from the pinned block (with the device's tokens in their
+    #: place): a copy keeps the stream waiting 5 us for the copy engine before its first byte and a second one for the tokens,
+    #: the kernel takes 3 us for a few hundred numbers; beyond, the copy engine's rate counts
+    STAGE_BY_KERNEL = 8192
+
     def prepare(self, entries: Sequence[BatchEntry], staging=None, widths=None,
                 device_tokens: Optional[torch.Tensor] = None) -> StepBatch:
         """Check the batch, allocate its pages and upload its metadata (into ``staging``'s
@@ -200,7 +207,7 @@ class ModelRunner:
         T = sum(len(en.tokens) for en in entries)
         R = sum(len(en.want) for en in entries)
         widest = -(-self.max_model_len // min(g.page_size for g in self.cache.groups)) if G else 0
-        total_cap = 3 * T + 3 * nseq + 1 + R + nseq * widest * G
+        total_cap = 4 * T + 3 * nseq + 1 + R + nseq * widest * G
         if staging is None:
             host, dev = self._staging(total_cap)
             host_tensor, copied = self._host_tensor, self._copied
@@ -212,12 +219,28 @@ class ModelRunner:
         layout, firsts, slots, lens, tok_off = built.layout, built.first_position, built.state_slot, \
             built.query_lens, built.seq_start
         total = int(layout.total)
-        dev[:total].copy_(host_tensor[:total], non_blocking=True)
-        copied.record()
+        off = int(layout.off_tokens)
+        indexed = device_tokens is not None and any(en.device_row is not None for en in entries)
         if device_tokens is not None:
-            if device_tokens.dtype != torch.int32 or device_tokens.numel() < T or not device_tokens.is_cuda:
+            if device_tokens.dtype != torch.int32 or not device_tokens.is_cuda or \
+                    (not indexed and device_tokens.numel() < T):
                 raise ValueError("device_tokens must be int32 on the device, one per row of the step")
-            dev[layout.off_tokens:layout.off_tokens + T].copy_(device_tokens.reshape(-1)[:T], non_blocking=True)
+            device_tokens = device_tokens.reshape(-1).contiguous()
+        if indexed:
+            index = host[total:total + T]                  # the block has room for them behind the step's numbers
+            index[:] = -1
+            for en, at in zip(entries, tok_off):
+                if en.device_row is not None:
+                    if len(en.tokens) != 1 or not 0 <= en.device_row < device_tokens.numel():
+                        raise ValueError(f"device_row {en.device_row} is not a token on the device for a single row")
+                    index[at] = en.device_row
+        if total <= self.STAGE_BY_KERNEL:
+            ops.stage_step(host_tensor, dev, 0, total, device_tokens, off, T, total if indexed else -1)
+        else:
+            dev[:total].copy_(host_tensor[:total], non_blocking=True)
+            if device_tokens is not None:
+                ops.stage_step(host_tensor, dev, off, T, device_tokens, off, T, total if indexed else -1)
+        copied.record()
 
         def view(off, n):
             return dev[off:off + n]
@@ -270,7 +293,7 @@ class _DecodeGraph:
 
     def __init__(self, runner: ModelRunner, B: int):
         self.widths = [-(-runner.max_model_len // g.page_size) for g in runner.cache.groups]
-        total = 3 * B + (B + 1) + 2 * B + B + sum(B * w for w in self.widths)
+        total = 4 * B + (B + 1) + 2 * B + B + sum(B * w for w in self.widths)
         self.host_tensor = torch.empty(total, dtype=torch.int32, pin_memory=True)
         self.host = self.host_tensor.numpy()
         self.dev = torch.empty(total, dtype=torch.int32, device=runner.device)

@@ -695,33 +695,71 @@ def _decode_splits(rows: int, num_heads: int, num_kv_heads: int, max_context: in
     return best
 
 
-def argmax(logits: torch.Tensor, out: torch.Tensor) -> None:
-    """First maximum of every row of 32-bit ``logits [R,V]`` into int32 ``out [R]``."""
+def _host_tokens(host: Optional[torch.Tensor], rows: int) -> int:
+    """The address of pinned int32 host memory that gets a choice's tokens beside the device (0: none)."""
+    if host is None:
+        return 0
+    if host.dtype != torch.int32 or not host.is_contiguous() or host.numel() < rows or not host.is_pinned():
+        raise KernelError(f"host tokens must be pinned int32 memory of at least {rows} entries")
+    return host.data_ptr()
+
+
+def argmax(logits: torch.Tensor, out: torch.Tensor, host: Optional[torch.Tensor] = None) -> None:
+    """First maximum of every row of 32-bit ``logits [R,V]`` into int32 ``out [R]``.  ``host`` (pinned int32): gets them
+    too; they are there once an event recorded behind the call has passed."""
     _check(logits, "logits", torch.float32, 2)
     _check(out, "out", torch.int32, 1)
     R, V = logits.shape
-    call(core(), "ap_argmax", logits.data_ptr(), V, R, V, out.data_ptr(), stream_handle())
+    call(core(), "ap_argmax", logits.data_ptr(), V, R, V, out.data_ptr(), _host_tokens(host, R), stream_handle())
 
 
 def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
-           top_p: torch.Tensor, uniform: torch.Tensor, out: torch.Tensor, method: str = "auto") -> None:
+           top_p: torch.Tensor, uniform: torch.Tensor, out: torch.Tensor, method: str = "auto",
+           host: Optional[torch.Tensor] = None) -> None:
     """One token per row: greedy where temperature <= 1e-5, else temperature/top-k/top-p.
 
     ``method``: "cluster" (eight CTAs hold a row in registers; vocabularies of up to 262144
-    entries), "rows" (one CTA per row, any vocabulary) or "auto" (the first where it fits)."""
+    entries), "rows" (one CTA per row, any vocabulary) or "auto" (the first where it fits).
+    The options may lie in pinned host memory, which must stay as it is until the call has run.  ``host``: as for
+    :func:`argmax`."""
     _check(logits, "logits", torch.float32, 2)
+    _check(out, "out", torch.int32, 1)
     R, V = logits.shape
     for t, n, dt in ((temperature, "temperature", torch.float32), (top_k, "top_k", torch.int32),
-                     (top_p, "top_p", torch.float32), (uniform, "uniform", torch.float32),
-                     (out, "out", torch.int32)):
-        _check(t, n, dt, 1)
+                     (top_p, "top_p", torch.float32), (uniform, "uniform", torch.float32)):
+        if t.is_cuda:
+            _check(t, n, dt, 1)
+        elif not t.is_pinned() or t.dtype != dt or t.dim() != 1 or not t.is_contiguous():
+            raise KernelError(f"sample: {n} must be a contiguous vector of {dt} on the device or in pinned memory")
+    for t, n in ((temperature, "temperature"), (top_k, "top_k"), (top_p, "top_p"), (uniform, "uniform"), (out, "out")):
         if t.shape[0] < R:
             raise KernelError(f"sample: {n} has fewer than {R} entries")
     entry = {"auto": "ap_sample", "cluster": "ap_sample_cluster", "rows": "ap_sample_rows"}.get(method)
     if entry is None:
         raise KernelError(f"sample: unknown method {method!r}")
     call(core(), entry, logits.data_ptr(), V, R, V, temperature.data_ptr(), top_k.data_ptr(),
-         top_p.data_ptr(), uniform.data_ptr(), out.data_ptr(), stream_handle())
+         top_p.data_ptr(), uniform.data_ptr(), out.data_ptr(), _host_tokens(host, R), stream_handle())
+
+
+def stage_step(host: torch.Tensor, dev: torch.Tensor, first: int, n: int, device_tokens: Optional[torch.Tensor] = None,
+               off_tokens: int = 0, tokens: int = 0, index_at: int = -1) -> None:
+    """Numbers ``first`` .. ``first + n - 1`` of pinned int32 ``host`` into the same places of ``dev``, in one kernel;
+    ``device_tokens`` (int32) take the place of the ``tokens`` numbers from ``off_tokens`` on, one after another, or, where
+    ``index_at`` is not negative, as the ``tokens`` numbers of ``host`` from there on say (negative: the host's number stays).
+    ``host`` must stay as it is until the call has run."""
+    end = max(first + n, index_at + tokens)
+    if host.dtype != torch.int32 or not host.is_contiguous() or host.numel() < end or not host.is_pinned():
+        raise KernelError(f"stage_step: the source must be pinned int32 memory of at least {end} entries")
+    _check(dev, "dev", torch.int32, 1)
+    if first < 0 or n < 0 or tokens < 0 or off_tokens < 0 or dev.numel() < first + n:
+        raise KernelError("stage_step: the device's block is shorter than what it is to hold")
+    if device_tokens is not None:
+        _check(device_tokens, "device_tokens", torch.int32, 1)
+        if index_at < 0 and device_tokens.numel() < tokens:
+            raise KernelError("stage_step: fewer tokens on the device than the step takes")
+    call(core(), "ap_stage_step", host.data_ptr(), dev.data_ptr(), int(first), int(n),
+         device_tokens.data_ptr() if device_tokens is not None else 0, int(off_tokens), int(tokens),
+         host.data_ptr() + 4 * index_at if device_tokens is not None and index_at >= 0 else 0, stream_handle())
 
 
 def gemm_tc_splits(M: int, N: int, K: int) -> int:

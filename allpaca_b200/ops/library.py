@@ -34,10 +34,12 @@ _CORE_SIGNATURES = {
     "ap_norm_residual": [_P, _P, _I, _L, _P, _I, _F, _F, _P, _I, _I, _I, _P],
     "ap_swiglu": [_P, _I, _I, _L, _P, _I, _I, _I, _I, _P],
     "ap_gemm_simt": [_P, _I, _P, _I, _P, _I, _I, _I, _I, _L, _L, _L, _P],
-    "ap_argmax": [_P, _L, _I, _I, _P, _P],
-    "ap_sample": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P],
-    "ap_sample_rows": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P],
-    "ap_sample_cluster": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P],
+    # int ap_stage_step(host, dev, first, n, device_tokens, off_tokens, tokens, index, stream)
+    "ap_stage_step": [_P, _P, _I, _I, _P, _I, _I, _P, _P],
+    "ap_argmax": [_P, _L, _I, _I, _P, _P, _P],
+    "ap_sample": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P, _P],
+    "ap_sample_rows": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P, _P],
+    "ap_sample_cluster": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P, _P],
     # int ap_embed_sinusoid_norm(tokens, positions, table, table_dtype, inv_freq, norm_w, norm_dtype, eps, scale,
     #                            x, T, H, V, stream)
     "ap_embed_sinusoid_norm": [_P, _P, _P, _I, _P, _P, _I, _F, _F, _P, _I, _I, _I, _P],
