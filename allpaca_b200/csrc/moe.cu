@@ -63,7 +63,7 @@ AP_EXPORT int ap_gated_act(const void* in, int in_dtype, void* out, int out_dtyp
 }
 
 // ---- routing ---------------------------------------------------------------------------
-#define ROUTE_MAX_PER_LANE 8          // experts <= 256
+#define ROUTE_MAX_EXPERTS 256
 #define ROUTE_MAX_TOP 16
 #define ROUTE_TOP_SOFTMAX 0           // the `top` largest z + bias; shares: their softmax
 #define ROUTE_SOFTMAX_ALL 1           // s = softmax(z) over all; the `top` largest s + bias; shares: their s / sum
@@ -72,59 +72,109 @@ AP_EXPORT int ap_gated_act(const void* in, int in_dtype, void* out, int out_dtyp
 
 // One CTA per RPB rows: eight warps, or, for a CTA of one row, a warp per router output (at most 32: a step of
 // few rows is a chain of loads per warp, which more warps shorten).  With `rows` the warps first form the rows' router logits: E dot
-// products of each row with the router's rows, the experts dealt to the warps in turn, 32-bit sums
+// products of each row with the router's rows, EB experts to a warp at a time, 32-bit sums
 // (every lane a strided part of K, 16-byte loads where the types and alignment allow, then a
 // butterfly over the lanes: one fixed order per row, whatever the batch and whichever rows share its CTA;
-// a part of the router that a warp has loaded meets all RPB rows before the next is loaded, so that a step of
-// many rows reads the router RPB times less often); else the logits are read from `logits` [T, E].  The bias is
-// added; warp r takes the `top` largest of row r and their shares.
+// a part of the router that a warp has loaded meets all RPB rows, and a part of a row all EB experts, before the next is
+// loaded: conversions to 32 bits are half of the arithmetic otherwise); else the logits are read from `logits` [T, E].  The bias is
+// added; warp r takes the `top` largest of row r and their shares.  A CTA of one row asks for the router's first 2048 columns
+// before the kernel that makes the row ends.  NL: experts per lane in the choice (E <= 32 NL).
+// Measured (one B200, in a step, us; in brackets with one expert at a time, eight experts per lane and nothing ahead of the
+// wait): 1 row of 2048 against 16 in four groups 5.4 (10.2), 32 rows of 4096 against 32 9.1 (12.0), 2048 rows 12.5 (26) and 23 (71).
 #define ROUTE_THREADS 256            // a CTA of several rows; a CTA of one row has up to ROUTE_MAX_THREADS
 #define ROUTE_MAX_THREADS 1024
-template <typename TA, typename TW, int RPB>
-__global__ void __launch_bounds__(ROUTE_MAX_THREADS)
+#define ROUTE_AHEAD 8                // 16-byte runs of a router row that a lane asks for ahead of the wait
+template <typename TA, typename TW, int RPB, int EB, int NL>
+__global__ void __launch_bounds__(RPB == 1 ? ROUTE_MAX_THREADS : ROUTE_THREADS)
 moe_route_kernel(const float* __restrict__ logits, const TA* __restrict__ rows, const TW* __restrict__ router, int K,
                  const float* __restrict__ bias, int* __restrict__ chosen, float* __restrict__ weight, int T, int E,
                  int top, int mode, int groups, int keep, float share_scale) {
-    __shared__ float z_all[RPB][32 * ROUTE_MAX_PER_LANE];
+    constexpr int ROUTE_MAX_PER_LANE = NL;
+    __shared__ float z_all[RPB][32 * NL];
     ap_pdl_trigger();
-    ap_pdl_wait();
     const int t0 = blockIdx.x * RPB, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nrows = min(RPB, T - t0);
-    if (rows != nullptr) {
-        const TA* a = rows + (size_t)t0 * K;
-        const bool vec = sizeof(TA) == 2 && sizeof(TW) == 2 && K % 8 == 0 &&
-                         ((((uintptr_t)rows) | ((uintptr_t)router)) & 15) == 0;
+    const TA* a = rows + (size_t)t0 * K;
+    const bool vec = sizeof(TA) == 2 && sizeof(TW) == 2 && K % 8 == 0 && rows != nullptr &&
+                     ((((uintptr_t)rows) | ((uintptr_t)router)) & 15) == 0;
+    if (vec && RPB == 1) {
+        uint4 ahead[ROUTE_AHEAD];
+        auto run = [&](const uint4& wv, int k, float& sum) {
+            const uint4 av = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(a) + k);
+            const __nv_bfloat162 *w2 = reinterpret_cast<const __nv_bfloat162*>(&wv), *a2 = reinterpret_cast<const __nv_bfloat162*>(&av);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 x = __bfloat1622float2(a2[q]), y = __bfloat1622float2(w2[q]);
+                sum = fmaf(x.y, y.y, fmaf(x.x, y.x, sum));
+            }
+        };
+        for (int e = warp; e < E; e += (int)blockDim.x / 32) {
+            const bf16* w = reinterpret_cast<const bf16*>(router) + (size_t)e * K;
+#pragma unroll
+            for (int i = 0; i < ROUTE_AHEAD; ++i)
+                if (lane * 8 + 256 * i < K) ahead[i] = *reinterpret_cast<const uint4*>(w + lane * 8 + 256 * i);
+            if (e == warp) ap_pdl_wait();
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < ROUTE_AHEAD; ++i)
+                if (lane * 8 + 256 * i < K) run(ahead[i], lane * 8 + 256 * i, sum);
+#pragma unroll 4
+            for (int k = lane * 8 + 256 * ROUTE_AHEAD; k < K; k += 256) run(*reinterpret_cast<const uint4*>(w + k), k, sum);
+            sum = ap_warp_sum(sum);
+            if (lane == 0) z_all[0][e] = sum + ((bias && mode == ROUTE_TOP_SOFTMAX) ? bias[e] : 0.f);
+        }
+        if (warp >= E) ap_pdl_wait();
+    } else if (vec) {
+        ap_pdl_wait();
+        for (int e0 = warp * EB; e0 < E; e0 += (int)blockDim.x / 32 * EB) {
+            float sum[RPB][EB];
+#pragma unroll
+            for (int r = 0; r < RPB; ++r)
+#pragma unroll
+                for (int j = 0; j < EB; ++j) sum[r][j] = 0.f;
+            const bf16* w = reinterpret_cast<const bf16*>(router) + (size_t)e0 * K;
+#pragma unroll 2
+            for (int k = lane * 8; k < K; k += 256) {
+                uint4 wv[EB], av[RPB];
+#pragma unroll
+                for (int j = 0; j < EB; ++j) wv[j] = *reinterpret_cast<const uint4*>(w + (size_t)(e0 + j < E ? j : 0) * K + k);
+#pragma unroll
+                for (int r = 0; r < RPB; ++r)
+                    av[r] = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(a) + (size_t)(r < nrows ? r : 0) * K + k);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    float2 y[EB];
+#pragma unroll
+                    for (int j = 0; j < EB; ++j) y[j] = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&wv[j])[q]);
+#pragma unroll
+                    for (int r = 0; r < RPB; ++r) {
+                        const float2 x = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&av[r])[q]);
+#pragma unroll
+                        for (int j = 0; j < EB; ++j) sum[r][j] = fmaf(x.y, y[j].y, fmaf(x.x, y[j].x, sum[r][j]));
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RPB; ++r)
+#pragma unroll
+                for (int j = 0; j < EB; ++j) {
+                    const float v = ap_warp_sum(sum[r][j]);
+                    if (lane == 0 && e0 + j < E) z_all[r][e0 + j] = v + ((bias && mode == ROUTE_TOP_SOFTMAX) ? bias[e0 + j] : 0.f);
+                }
+        }
+    } else if (rows != nullptr) {
+        ap_pdl_wait();
         for (int e = warp; e < E; e += (int)blockDim.x / 32) {
             const TW* w = router + (size_t)e * K;
             float sum[RPB];
 #pragma unroll
             for (int r = 0; r < RPB; ++r) sum[r] = 0.f;
-            if (vec) {
 #pragma unroll 4
-                for (int k = lane * 8; k < K; k += 256) {
-                    const uint4 wv = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(w) + k);
-                    const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(&wv);
+            for (int k = lane; k < K; k += 32) {
+                const float wk = ap_to_float(w[k]);
 #pragma unroll
-                    for (int r = 0; r < RPB; ++r) {
-                        if (r < nrows) {
-                            const uint4 av = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(a) + (size_t)r * K + k);
-                            const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&av);
-#pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                const float2 x = __bfloat1622float2(a2[q]), y = __bfloat1622float2(w2[q]);
-                                sum[r] = fmaf(x.y, y.y, fmaf(x.x, y.x, sum[r]));
-                            }
-                        }
-                    }
-                }
-            } else {
-#pragma unroll 4
-                for (int k = lane; k < K; k += 32) {
-                    const float wk = ap_to_float(w[k]);
-#pragma unroll
-                    for (int r = 0; r < RPB; ++r)
-                        if (r < nrows) sum[r] = fmaf(ap_to_float(a[(size_t)r * K + k]), wk, sum[r]);
-                }
+                for (int r = 0; r < RPB; ++r)
+                    if (r < nrows) sum[r] = fmaf(ap_to_float(a[(size_t)r * K + k]), wk, sum[r]);
             }
 #pragma unroll
             for (int r = 0; r < RPB; ++r) {
@@ -133,6 +183,7 @@ moe_route_kernel(const float* __restrict__ logits, const TA* __restrict__ rows, 
             }
         }
     } else {
+        ap_pdl_wait();
         for (int r = 0; r < nrows; ++r)
             for (int e = threadIdx.x; e < E; e += (int)blockDim.x)
                 z_all[r][e] = logits[(size_t)(t0 + r) * E + e] + ((bias && mode == ROUTE_TOP_SOFTMAX) ? bias[e] : 0.f);
@@ -218,8 +269,8 @@ moe_route_kernel(const float* __restrict__ logits, const TA* __restrict__ rows, 
         for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i)
             if (!((open >> i) & 1u)) z[i] = -INFINITY;
     }
-    float best[ROUTE_MAX_TOP];
-    int who[ROUTE_MAX_TOP];
+    float best = 0.f;                                        // lane k: the k-th choice
+    int who = 0;
     for (int k = 0; k < top; ++k) {
         float v = -INFINITY;
         int idx = 0x7fffffff;
@@ -243,42 +294,39 @@ moe_route_kernel(const float* __restrict__ logits, const TA* __restrict__ rows, 
                 if (lane + 32 * i == idx) own = sc[i];
             v = __shfl_sync(0xffffffffu, own, idx & 31);
         }
-        best[k] = v;
-        who[k] = idx;
+        if (lane == k) {
+            best = v;
+            who = idx;
+        }
 #pragma unroll
         for (int i = 0; i < ROUTE_MAX_PER_LANE; ++i)
             if (lane + 32 * i == idx) z[i] = -INFINITY;       // taken
     }
-    if (lane == 0 && (mode == ROUTE_SIGMOID || mode == ROUTE_SOFTMAX_SCORES)) {
-        for (int k = 0; k < top; ++k) {
-            chosen[(size_t)t * top + k] = who[k];
-            weight[(size_t)t * top + k] = best[k] * share_scale;
-        }
-    } else if (lane == 0 && mode == ROUTE_SOFTMAX_ALL) {
-        float sum = 0.f;
-        for (int k = 0; k < top; ++k) sum += best[k];
-        for (int k = 0; k < top; ++k) {
-            chosen[(size_t)t * top + k] = who[k];
-            weight[(size_t)t * top + k] = best[k] / (sum + 1e-20f) * share_scale;
-        }
-    } else if (lane == 0) {
-        float sum = 0.f;
-        for (int k = 0; k < top; ++k) sum += expf(best[k] - best[0]);      // best[0] is the largest
-        for (int k = 0; k < top; ++k) {
-            chosen[(size_t)t * top + k] = who[k];
-            weight[(size_t)t * top + k] = expf(best[k] - best[0]) / sum * share_scale;
-        }
+    float share = best, sum = 0.f;
+    if (mode == ROUTE_SOFTMAX_ALL || mode == ROUTE_TOP_SOFTMAX) {
+        if (mode == ROUTE_TOP_SOFTMAX) share = expf(best - __shfl_sync(0xffffffffu, best, 0));      // the first is the largest
+        for (int k = 0; k < top; ++k) sum += __shfl_sync(0xffffffffu, share, k);
+        share = mode == ROUTE_SOFTMAX_ALL ? share / (sum + 1e-20f) : share / sum;
+    }
+    if (lane < top) {
+        chosen[(size_t)t * top + lane] = who;
+        weight[(size_t)t * top + lane] = share * share_scale;
     }
 }
 
+#define ROUTE_NL(CALL) do { if (E <= 32) CALL(1); else if (E <= 64) CALL(2); else if (E <= 128) CALL(4); else CALL(8); } while (0)
+
 AP_EXPORT int ap_moe_route(const float* logits, const float* bias, int* chosen, float* weight, int T, int E, int top,
                            cudaStream_t stream) {
-    AP_REQUIRE(T >= 0 && E > 0 && E <= 32 * ROUTE_MAX_PER_LANE && top > 0 && top <= E && top <= ROUTE_MAX_TOP,
-               "moe_route: %d experts (at most %d), %d chosen (at most %d)", E, 32 * ROUTE_MAX_PER_LANE, top, ROUTE_MAX_TOP);
+    AP_REQUIRE(T >= 0 && E > 0 && E <= ROUTE_MAX_EXPERTS && top > 0 && top <= E && top <= ROUTE_MAX_TOP,
+               "moe_route: %d experts (at most %d), %d chosen (at most %d)", E, ROUTE_MAX_EXPERTS, top, ROUTE_MAX_TOP);
     if (T == 0) return AP_OK;
-    AP_CHECK_PDL_LAUNCH("moe_route", ap_launch_pdl(moe_route_kernel<float, float, 1>, dim3((unsigned)T), dim3(ROUTE_THREADS),
-                                                   0, stream, logits, (const float*)nullptr, (const float*)nullptr, 0, bias,
-                                                   chosen, weight, T, E, top, ROUTE_TOP_SOFTMAX, 1, 1, 1.0f));
+#define LAUNCH(NL)                                                                                                    \
+    AP_CHECK_PDL_LAUNCH("moe_route", ap_launch_pdl(moe_route_kernel<float, float, 1, 1, NL>, dim3((unsigned)T), dim3(ROUTE_THREADS), \
+                                                   0, stream, logits, (const float*)nullptr, (const float*)nullptr, 0, bias, \
+                                                   chosen, weight, T, E, top, ROUTE_TOP_SOFTMAX, 1, 1, 1.0f))
+    ROUTE_NL(LAUNCH);
+#undef LAUNCH
     return AP_OK;
 }
 
@@ -289,23 +337,27 @@ AP_EXPORT int ap_moe_route_rows(const void* rows, int rows_dtype, const void* ro
     AP_REQUIRE(mode >= ROUTE_TOP_SOFTMAX && mode <= ROUTE_SOFTMAX_SCORES, "moe_route: unknown mode %d", mode);
     AP_REQUIRE(groups > 0 && E % groups == 0 && keep > 0 && keep <= groups && top <= E / groups * keep,
                "moe_route: %d experts in %d groups, %d of them kept, %d chosen", E, groups, keep, top);
-    AP_REQUIRE(T >= 0 && K > 0 && E > 0 && E <= 32 * ROUTE_MAX_PER_LANE && top > 0 && top <= E && top <= ROUTE_MAX_TOP,
-               "moe_route: %d experts (at most %d), %d chosen (at most %d)", E, 32 * ROUTE_MAX_PER_LANE, top, ROUTE_MAX_TOP);
+    AP_REQUIRE(T >= 0 && K > 0 && E > 0 && E <= ROUTE_MAX_EXPERTS && top > 0 && top <= E && top <= ROUTE_MAX_TOP,
+               "moe_route: %d experts (at most %d), %d chosen (at most %d)", E, ROUTE_MAX_EXPERTS, top, ROUTE_MAX_TOP);
     if (T == 0) return AP_OK;
     // four rows to a CTA in a step of many rows
     const bool four = T >= 512;
     const unsigned threads1 = (unsigned)(32 * (E < 8 ? 8 : E > 32 ? 32 : E));
-#define LAUNCH_R(TA, TW, R)                                                                                        \
-    AP_CHECK_PDL_LAUNCH("moe_route", ap_launch_pdl(moe_route_kernel<TA, TW, R>, dim3((unsigned)((T + R - 1) / R)),   \
-                                                   dim3(R == 1 ? threads1 : ROUTE_THREADS), 0, stream, (const float*)nullptr,           \
+#define LAUNCH_R(TA, TW, R, EB, NL)                                                                                \
+    AP_CHECK_PDL_LAUNCH("moe_route", ap_launch_pdl(moe_route_kernel<TA, TW, R, EB, NL>, dim3((unsigned)((T + R - 1) / R)), \
+                                                   dim3(R == 1 ? threads1 : ROUTE_THREADS), 0, stream, (const float*)nullptr, \
                                                    (const TA*)rows, (const TW*)router, K, bias, chosen, weight, T, E, \
                                                    top, mode, groups, keep, share_scale))
-#define LAUNCH(TA, TW) do { if (four) LAUNCH_R(TA, TW, 4); else LAUNCH_R(TA, TW, 1); } while (0)
-    if (rows_dtype == AP_F32 && router_dtype == AP_F32) LAUNCH(float, float);
-    else if (rows_dtype == AP_BF16 && router_dtype == AP_BF16) LAUNCH(bf16, bf16);
-    else if (rows_dtype == AP_BF16 && router_dtype == AP_F32) LAUNCH(bf16, float);
+#define LAUNCH_BF(NL) do { if (!four) LAUNCH_R(bf16, bf16, 1, 1, NL); else if (E <= 16) LAUNCH_R(bf16, bf16, 4, 2, NL); else LAUNCH_R(bf16, bf16, 4, 4, NL); } while (0)
+#define LAUNCH_FF(NL) do { if (!four) LAUNCH_R(float, float, 1, 1, NL); else LAUNCH_R(float, float, 4, 1, NL); } while (0)
+#define LAUNCH_BW(NL) do { if (!four) LAUNCH_R(bf16, float, 1, 1, NL); else LAUNCH_R(bf16, float, 4, 1, NL); } while (0)
+    if (rows_dtype == AP_F32 && router_dtype == AP_F32) ROUTE_NL(LAUNCH_FF);
+    else if (rows_dtype == AP_BF16 && router_dtype == AP_BF16) ROUTE_NL(LAUNCH_BF);
+    else if (rows_dtype == AP_BF16 && router_dtype == AP_F32) ROUTE_NL(LAUNCH_BW);
     else AP_REQUIRE(false, "moe_route: unsupported dtypes rows=%d router=%d", rows_dtype, router_dtype);
-#undef LAUNCH
+#undef LAUNCH_BF
+#undef LAUNCH_FF
+#undef LAUNCH_BW
 #undef LAUNCH_R
     return AP_OK;
 }
@@ -322,34 +374,62 @@ AP_EXPORT int ap_moe_route_rows(const void* rows, int rows_dtype, const void* ro
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int* __restrict__ chosen, int* __restrict__ perm, int* __restrict__ place, int3* __restrict__ tiles,
                 int* __restrict__ offsets, int pairs, int E, int max_tiles, int real) {
+    // every warp counts and places its pairs on counters of its own: the counters of a few experts would meet all 32
+    // (8192 pairs on 16 experts 7.0 us; one set of counters and one thread for the tiles 10, a match over each warp 12.5)
+    extern __shared__ int mine_s[];                          // [warps][E]
     __shared__ int count[SORT_MAX_EXPERTS];
     __shared__ int first[SORT_MAX_EXPERTS + 1];
+    __shared__ int tile_of[SORT_MAX_EXPERTS + 1];
     ap_pdl_trigger();
     ap_pdl_wait();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    int* mine = mine_s + warp * E;
+    for (int i = threadIdx.x; i < warps * E; i += blockDim.x) mine_s[i] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < pairs; i += blockDim.x) atomicAdd(&count[chosen[i]], 1);
+    for (int i = threadIdx.x; i < pairs; i += blockDim.x) atomicAdd(&mine[chosen[i]], 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int at = 0, nt = 0;
-        for (int e = 0; e < E; ++e) {
-            first[e] = at;
-            // experts from `real` on have no weights (their result is their input): no tiles for the products
-            for (int r = 0; e < real && r < count[e] && nt < max_tiles; r += MOE_BM)
-                tiles[nt++] = make_int3(e, at + r, min(MOE_BM, count[e] - r));
-            at += count[e];
+    // a warp's counters become the places before its own pairs of an expert
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+        int before = 0;
+        for (int w = 0; w < warps; ++w) {
+            const int n = mine_s[w * E + e];
+            mine_s[w * E + e] = before;
+            before += n;
         }
-        first[E] = at;
-        tiles[max_tiles] = make_int3(nt, 0, 0);
+        count[e] = before;
     }
     __syncthreads();
+    if (threadIdx.x < 32) {
+        // running sums over the experts, 32 at a time: pairs, and row tiles (none for experts from `real` on, which have no
+        // weights: their result is their input)
+        int at = 0, nt = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane;
+            const int n = e < E ? count[e] : 0, k = e < real ? (n + MOE_BM - 1) / MOE_BM : 0;
+            int sn = n, sk = k;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int un = __shfl_up_sync(0xffffffffu, sn, o), uk = __shfl_up_sync(0xffffffffu, sk, o);
+                if (lane >= o) { sn += un; sk += uk; }
+            }
+            if (e < E) { first[e] = at + sn - n; tile_of[e] = nt + sk - k; }
+            at += __shfl_sync(0xffffffffu, sn, 31);
+            nt += __shfl_sync(0xffffffffu, sk, 31);
+        }
+        if (lane == 0) {
+            first[E] = at;
+            tiles[max_tiles] = make_int3(min(nt, max_tiles), 0, 0);
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += blockDim.x)
+        for (int k = 0, n = count[e]; e < real && k * MOE_BM < n && tile_of[e] + k < max_tiles; ++k)
+            tiles[tile_of[e] + k] = make_int3(e, first[e] + k * MOE_BM, min(MOE_BM, n - k * MOE_BM));
     if (offsets != nullptr)
         for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = first[e];
-    for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
-    __syncthreads();
     for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
         const int e = chosen[i];
-        const int p = first[e] + atomicAdd(&count[e], 1);
+        const int p = first[e] + atomicAdd(&mine[e], 1);
         perm[p] = i;
         place[i] = p;
     }
@@ -362,7 +442,9 @@ AP_EXPORT int ap_moe_sort(const int* chosen, int* perm, int* place, int* tiles, 
     AP_REQUIRE(pairs >= 0 && E > 0 && E <= SORT_MAX_EXPERTS, "moe_sort: %d experts (at most %d)", E, SORT_MAX_EXPERTS);
     AP_REQUIRE(real >= 0 && real <= E, "moe_sort: %d of %d experts have weights", real, E);
     if (pairs == 0) return AP_OK;
-    AP_CHECK_PDL_LAUNCH("moe_sort", ap_launch_pdl(moe_sort_kernel, dim3(1), dim3(1024), 0, stream, chosen, perm, place,
+    const int threads = pairs >= 1024 ? 1024 : (pairs + 31) / 32 * 32;
+    AP_CHECK_PDL_LAUNCH("moe_sort", ap_launch_pdl(moe_sort_kernel, dim3(1), dim3((unsigned)threads),
+                                                  (size_t)(threads / 32) * E * sizeof(int), stream, chosen, perm, place,
                                                   (int3*)tiles, offsets, pairs, E, ap_moe_max_tiles(pairs, E), real));
     return AP_OK;
 }
@@ -690,12 +772,51 @@ __global__ void moe_combine_kernel(const float* __restrict__ o, const int* __res
     }
 }
 
+// The same for rows of whole 16-byte runs without identity experts: a CTA takes a row's run of 1024 columns, so that places and
+// weights are read once per thread and all of the row's results are in flight together.  Traffic bounds it: 2048 rows of 2048,
+// four results and a base 20 us (5.0 TB/s), 25 with an element to a thread; 4096 wide 31 and 48.
+#define COMBINE_TOP 8
+__global__ void __launch_bounds__(256)
+moe_combine_runs_kernel(const float* __restrict__ o, const int* __restrict__ place, const float* __restrict__ weight,
+                        float* __restrict__ delta, int H, int top, const float* __restrict__ base) {
+    ap_pdl_trigger();
+    ap_pdl_wait();
+    const size_t t = blockIdx.x;
+    const int c = (int)(blockIdx.y * 256 + threadIdx.x) * 4;
+    if (c >= H) return;
+    float4 v = base ? *reinterpret_cast<const float4*>(base + t * H + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k0 = 0; k0 < top; k0 += COMBINE_TOP) {
+        float4 r[COMBINE_TOP];
+        float w[COMBINE_TOP];
+#pragma unroll
+        for (int k = 0; k < COMBINE_TOP; ++k)
+            if (k0 + k < top) {
+                w[k] = weight ? weight[t * top + k0 + k] : 1.0f;
+                r[k] = *reinterpret_cast<const float4*>(o + (size_t)place[t * top + k0 + k] * H + c);
+            }
+#pragma unroll
+        for (int k = 0; k < COMBINE_TOP; ++k)
+            if (k0 + k < top) {
+                v.x = fmaf(w[k], r[k].x, v.x);
+                v.y = fmaf(w[k], r[k].y, v.y);
+                v.z = fmaf(w[k], r[k].z, v.z);
+                v.w = fmaf(w[k], r[k].w, v.w);
+            }
+    }
+    *reinterpret_cast<float4*>(delta + t * H + c) = v;
+}
+
 AP_EXPORT int ap_moe_combine(const float* o, const int* place, const float* weight, float* delta, int T, int H, int top,
                              const int* chosen, int real, const void* rows, int rows_dtype, const float* base,
                              cudaStream_t stream) {
     AP_REQUIRE(T >= 0 && H > 0 && top > 0, "moe_combine: bad sizes");
     AP_REQUIRE(chosen == nullptr || rows != nullptr, "moe_combine: identity experts need the rows' input");
     if (T == 0) return AP_OK;
+    if (chosen == nullptr && H % 4 == 0 && (((uintptr_t)o | (uintptr_t)delta | (uintptr_t)base) & 15) == 0) {
+        AP_CHECK_PDL_LAUNCH("moe_combine", ap_launch_pdl(moe_combine_runs_kernel, dim3((unsigned)T, (unsigned)((H + 1023) / 1024)),
+                                                         dim3(256), 0, stream, o, place, weight, delta, H, top, base));
+        return AP_OK;
+    }
     long long blocks = ((long long)T * H + 255) / 256;
     if (blocks > 148 * 32) blocks = 148 * 32;
     if (chosen != nullptr && rows_dtype == AP_BF16)
