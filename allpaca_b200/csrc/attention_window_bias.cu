@@ -325,15 +325,21 @@ attention_window_bias_kernel(const TA* __restrict__ q, TA* __restrict__ out, con
 }
 
 // ---------------------------------------------------------------------------------------
-// bfloat16, sequences of several rows, head sizes up to 128: the same attention on the tensor
+// bfloat16, sequences of several rows, head sizes up to 128 (keys up to 192): the same attention on the tensor
 // cores (mma.sync m16n8k16, 32-bit accumulators).  A CTA of four warps takes 64 consecutive rows
 // of one sequence and one query head, 16 rows to a warp, whose queries stay in registers as the
-// first product's A operand; keys come 64 at a time through shared memory ([key][d], the B
-// operand as it lies), values transposed ([d][key]) for the second product.  Scores leave the
+// first product's A operand; keys and values come 64 at a time through two buffers of shared memory, each asked for a tile
+// ahead by cp.async (a lane finds the page of a key, eight lanes share its record), and are read as B operands
+// by ldmatrix, values transposed on the way.  Scores leave the
 // first product as 32-bit sums; scale, distance bias, window and the online softmax act on them
 // in registers; the weights are rounded to bfloat16 only as the second product's A operand,
-// their sum is kept in 32-bit.  DK, DV: the head sizes rounded up to a size the kernel is
-// built for (operands are zero beyond the real sizes).
+// their sum is kept in 32-bit.  A tile that all of a warp's rows see whole skips the masks.  DK, DV: the head sizes rounded up
+// to a size the kernel is built for (operands are zero beyond the real sizes).
+//
+// What bounds it is the arithmetic between the products (a score's bias, maximum, exponential) and the products' own
+// instructions, two CTAs to an SM hiding each other's waits.  Measured (one B200, 2048 rows, 16 heads on 4, head size 128, window
+// 512, in the step): 49 us with a logarithmic bias, 66 without one and a second layer's keys; values stored transposed by two
+// bytes, key fragments by 32-bit loads and no load ahead took 125 and 195.
 // ---------------------------------------------------------------------------------------
 #define MQ 64
 #define MK 64
@@ -348,9 +354,25 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&v);
 }
+__device__ __forceinline__ void awb_ldsm_x4(uint32_t (&r)[4], const void* p) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s) : "memory");
+}
+__device__ __forceinline__ void awb_ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s) : "memory");
+}
+
+template <int DK, int DV> struct AwbMma {
+    static constexpr int kKPitch = DK + 8, kVPitch = DV + 8;             // 16 bytes more than a row: ldmatrix meets no bank twice
+    static constexpr int kStage = MK * (kKPitch + kVPitch);              // elements
+    static constexpr int kSmem = 2 * kStage * 2 + MMA_BIAS_TABLE * 4;
+};
 
 template <int DK, int DV>
-__global__ void __launch_bounds__(AWB_THREADS)
+__global__ void __launch_bounds__(AWB_THREADS, 2)
 attention_window_bias_mma_kernel(const bf16* __restrict__ q, bf16* __restrict__ out, const bf16* __restrict__ cache,
                                  const int* __restrict__ block_table, int max_blocks, const int* __restrict__ seq_start,
                                  const int* __restrict__ positions, int nseq, int nh, int nkv, int D, int VD, int P,
@@ -358,11 +380,9 @@ attention_window_bias_mma_kernel(const bf16* __restrict__ q, bf16* __restrict__ 
                                  const float* __restrict__ r2, int skip_single, int RS, int voff, int bias_kind,
                                  int keep_first, const float* __restrict__ gate, long long gate_ld,
                                  const float* __restrict__ sink) {
-    // the widest keys leave room for a shorter table (48 KB of static shared memory in all)
-    constexpr int BIAS_TABLE = DK > 128 ? MMA_BIAS_TABLE / 2 : MMA_BIAS_TABLE;
-    __shared__ __align__(16) bf16 k_s[MK][DK + 8];
-    __shared__ __align__(16) bf16 vt_s[DV][MK + 8];
-    __shared__ float bias_s[BIAS_TABLE];                   // r1 ln(1 + r2 d) for the distances this CTA meets
+    using Cfg = AwbMma<DK, DV>;
+    extern __shared__ __align__(16) bf16 awb_smem[];       // [2][keys | values], then the bias of the distances this CTA meets
+    float* bias_s = reinterpret_cast<float*>(awb_smem + 2 * Cfg::kStage);
     ap_pdl_trigger();
     ap_pdl_wait();
     int b = blockIdx.x, seq = -1, row0 = 0, nrows = 0;
@@ -382,153 +402,194 @@ attention_window_bias_mma_kernel(const bf16* __restrict__ q, bf16* __restrict__ 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
     const int* table = block_table + (size_t)seq * max_blocks;
     const int pos_first = positions[row0], pos_last = pos_first + nrows - 1;
+    const int klo = (window > 0 && pos_first - window + 1 > 0) ? pos_first - window + 1 : 0;
+    const int kfe = keep_first < klo ? keep_first : klo;       // kept first tokens before the first row's window
+    const int tiles_kept = (kfe + MK - 1) / MK, tile_win = klo / MK;
+    const bool vec = D % 8 == 0 && VD % 8 == 0 && RS % 8 == 0 && voff % 8 == 0 && page_stride % 8 == 0 &&
+                     ((uintptr_t)cache & 15) == 0;
+    // a warp brings sixteen keys of a tile with their values
+    auto load_tile = [&](int tile, int stage) {
+        bf16* ks = awb_smem + stage * Cfg::kStage;
+        bf16* vs = ks + MK * Cfg::kKPitch;
+        long long mine = -1;
+        const int kp = tile * MK + warp * 16 + lane;
+        if (lane < 16 && (kp >= klo || kp < kfe) && kp <= pos_last) {
+            const int pg = kp / P;
+            mine = (long long)((size_t)table[pg] * page_stride + ((size_t)kvh * P + (kp - pg * P)) * RS);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int key = warp * 16 + 4 * j + (lane >> 3);
+            const long long at = __shfl_sync(0xffffffffu, mine, 4 * j + (lane >> 3));
+#pragma unroll
+            for (int c0 = 0; c0 < (DK + DV) / 8; c0 += 8) {
+                const int c = c0 + (lane & 7);
+                if (c >= (DK + DV) / 8) continue;              // (sizes of 32: half of the lanes)
+                const bool is_k = c < DK / 8;
+                const int d = is_k ? c * 8 : c * 8 - DK, n = is_k ? D : VD;
+                bf16* dst = is_k ? ks + key * Cfg::kKPitch + d : vs + key * Cfg::kVPitch + d;
+                if (at >= 0 && vec && d < n) {
+                    const unsigned sm = (unsigned)__cvta_generic_to_shared(dst);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sm), "l"(cache + at + (is_k ? d : voff + d)) : "memory");
+                } else {
+                    uint4 val = make_uint4(0, 0, 0, 0);
+                    if (at >= 0) {
+                        bf16* e8 = reinterpret_cast<bf16*>(&val);
+                        for (int e = 0; e < 8; ++e)
+                            if (d + e < n) e8[e] = cache[at + (is_k ? 0 : voff) + d + e];
+                    }
+                    *reinterpret_cast<uint4*>(dst) = val;
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int tile = tiles_kept > 0 ? 0 : tile_win, stage = 0;
+    load_tile(tile, 0);
     // this warp's queries as A fragments: rows g and g + 8 of its 16
     uint32_t qa[DK / 16][4];
     {
         const int ra = warp * 16 + g, rb = ra + 8;
         const bf16* qra = q + ((size_t)(row0 + ra) * nh + h) * D;
         const bf16* qrb = q + ((size_t)(row0 + rb) * nh + h) * D;
+        const bool pairs = D % 2 == 0 && ((uintptr_t)q & 3) == 0;
         const bf16 zero = __float2bfloat16_rn(0.f);
+        auto two = [&](const bf16* src, bool in, int c) -> uint32_t {
+            if (!in || c >= D) return 0u;
+            if (pairs) return *reinterpret_cast<const uint32_t*>(src + c);
+            const bf16 lo = src[c], hi = c + 1 < D ? src[c + 1] : zero;
+            return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+        };
 #pragma unroll
-        for (int ks = 0; ks < DK / 16; ++ks) {
+        for (int ks = 0; ks < DK / 16; ++ks)
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 const int c = ks * 16 + half * 8 + 2 * t4;
-                const bf16 a0 = (ra < nrows && c < D) ? qra[c] : zero, a1 = (ra < nrows && c + 1 < D) ? qra[c + 1] : zero;
-                const bf16 b0 = (rb < nrows && c < D) ? qrb[c] : zero, b1 = (rb < nrows && c + 1 < D) ? qrb[c + 1] : zero;
-                qa[ks][half * 2] = (uint32_t)__bfloat16_as_ushort(a0) | ((uint32_t)__bfloat16_as_ushort(a1) << 16);
-                qa[ks][half * 2 + 1] = (uint32_t)__bfloat16_as_ushort(b0) | ((uint32_t)__bfloat16_as_ushort(b1) << 16);
+                qa[ks][half * 2] = two(qra, ra < nrows, c);
+                qa[ks][half * 2 + 1] = two(qrb, rb < nrows, c);
             }
-        }
     }
     const float b1h = r1 ? r1[h] : 0.f, b2h = r2 ? r2[h] : 0.f;
-    const int klo = (window > 0 && pos_first - window + 1 > 0) ? pos_first - window + 1 : 0;
     // the largest distance any row of this CTA has to a key it may see
     const int span = pos_last - klo + 1;
-    const bool tabled = bias_kind == BIAS_LOG && span <= BIAS_TABLE;
+    const bool tabled = bias_kind == BIAS_LOG && span <= MMA_BIAS_TABLE;
     if (tabled)
         for (int d = threadIdx.x; d < span; d += AWB_THREADS) bias_s[d] = b1h * log1pf(b2h * (float)d);
-    const int kfe = keep_first < klo ? keep_first : klo;       // kept first tokens before the first row's window
-    const int tiles_kept = (kfe + MK - 1) / MK, tile_win = klo / MK;
     float o[DV / 8][4];
 #pragma unroll
     for (int i = 0; i < DV / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
     float m[2] = {-FLT_MAX, -FLT_MAX}, l[2] = {0.f, 0.f};
-    const bool vec = D % 8 == 0 && VD % 8 == 0 && RS % 8 == 0 && voff % 8 == 0 && page_stride % 8 == 0 &&
-                     ((uintptr_t)cache & 15) == 0;
     const int row_a = warp * 16 + g;                        // this lane's rows: row_a and row_a + 8
-    for (int tile = tiles_kept > 0 ? 0 : tile_win; tile * MK <= pos_last; tile = awb_next_tile(tile, tiles_kept, tile_win)) {
+    const int warp_first = pos_first + warp * 16, warp_last = min(warp_first + 15, pos_last);
+    while (tile * MK <= pos_last) {
+        const int next = awb_next_tile(tile, tiles_kept, tile_win);
+        if (next * MK <= pos_last) {
+            load_tile(next, stage ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();                                     // the tile (and, the first time, the table) is there
         const int k0 = tile * MK;
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < MK * (DK / 8); idx += AWB_THREADS) {
-            const int j = idx / (DK / 8), d0 = (idx - j * (DK / 8)) * 8;
-            const int kp = k0 + j;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if ((kp >= klo || kp < kfe) && kp <= pos_last && d0 < D) {
-                const bf16* src = cache + (size_t)table[kp / P] * page_stride + ((size_t)kvh * P + kp % P) * RS + d0;
-                if (vec) {
-                    val = *reinterpret_cast<const uint4*>(src);
-                } else {
-                    bf16* dst = reinterpret_cast<bf16*>(&val);
-                    for (int e = 0; e < 8; ++e)
-                        if (d0 + e < D) dst[e] = src[e];
+        // a warp whose rows see none of the tile's keys (before its last row's window, behind its last row) has nothing to do
+        const bool work = warp * 16 < nrows && k0 <= warp_last &&
+                          (window <= 0 || k0 + MK - 1 > warp_first - window || k0 < keep_first);
+        if (work) {
+            const bf16* ks = awb_smem + stage * Cfg::kStage;
+            const bf16* vs = ks + MK * Cfg::kKPitch;
+            float sc[MK / 8][4];
+#pragma unroll
+            for (int nb = 0; nb < MK / 8; ++nb) sc[nb][0] = sc[nb][1] = sc[nb][2] = sc[nb][3] = 0.f;
+            // fragments of eight keys and 32 coordinates at a time
+            const bf16* kb = ks + (lane & 7) * Cfg::kKPitch + (lane >> 3) * 8;
+#pragma unroll
+            for (int kk = 0; kk < DK / 32; ++kk)
+#pragma unroll
+                for (int nb = 0; nb < MK / 8; ++nb) {
+                    uint32_t f[4];
+                    awb_ldsm_x4(f, kb + nb * 8 * Cfg::kKPitch + kk * 32);
+                    mma_bf16_16816(sc[nb], qa[2 * kk], f[0], f[1]);
+                    mma_bf16_16816(sc[nb], qa[2 * kk + 1], f[2], f[3]);
                 }
-            }
-            *reinterpret_cast<uint4*>(&k_s[j][d0]) = val;
+            // scale, bias, window; the tile's row maxima
+            const bool whole = k0 + MK - 1 <= warp_first && warp * 16 + 15 < nrows && (window <= 0 || warp_last - k0 < window);
+            // (one kind of work to a loop, the choice outside it: with all kinds in the body of one unrolled loop the code of
+            // a tile was many times what it runs, and the warps waited for instructions)
+            float mx[2] = {-FLT_MAX, -FLT_MAX};
+            const int far = pos_first + row_a - k0 - 2 * t4;         // distance of this lane's first row and key
+#define EACH_SCORE(...)                                                  \
+    _Pragma("unroll") for (int nb = 0; nb < MK / 8; ++nb)                \
+        _Pragma("unroll") for (int e = 0; e < 4; ++e) {                  \
+            const int dist = far + (e >> 1) * 8 - nb * 8 - (e & 1);      \
+            float& v = sc[nb][e];                                        \
+            __VA_ARGS__;                                                 \
+            (void)dist;                                                  \
         }
-        for (int idx = threadIdx.x; idx < MK * (DV / 8); idx += AWB_THREADS) {
-            const int j = idx % MK, d0 = (idx / MK) * 8;
-            const int kp = k0 + j;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if ((kp >= klo || kp < kfe) && kp <= pos_last && d0 < VD) {
-                const bf16* src = cache + (size_t)table[kp / P] * page_stride + ((size_t)kvh * P + kp % P) * RS + voff + d0;
-                if (vec) {
-                    val = *reinterpret_cast<const uint4*>(src);
-                } else {
-                    bf16* dst = reinterpret_cast<bf16*>(&val);
-                    for (int e = 0; e < 8; ++e)
-                        if (d0 + e < VD) dst[e] = src[e];
-                }
+            // (a tile that begins behind the kept tokens has no key in sight beyond the table)
+            EACH_SCORE(v *= scale)
+            if (softcap > 0.f) { EACH_SCORE(v = softcap * tanhf(v / softcap)) }
+            if (bias_kind == BIAS_LINEAR) { EACH_SCORE(v -= b1h * (float)dist) }
+            else if (bias_kind == BIAS_LOG && tabled && k0 >= kfe) { EACH_SCORE(v -= bias_s[min(max(dist, 0), span - 1)]) }
+            else if (bias_kind == BIAS_LOG) { EACH_SCORE(v -= b1h * log1pf(b2h * fmaxf((float)dist, 0.f))) }
+            if (!whole) {
+                EACH_SCORE(const int r = row_a + (e >> 1) * 8;
+                           if (!(r < nrows && dist >= 0 && (window <= 0 || dist < window || k0 + nb * 8 + 2 * t4 + (e & 1) < keep_first)))
+                               v = -FLT_MAX)
             }
-            const bf16* ve = reinterpret_cast<const bf16*>(&val);
+            EACH_SCORE(mx[e >> 1] = fmaxf(mx[e >> 1], v))
+#undef EACH_SCORE
+            float alpha[2];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) vt_s[d0 + e][j] = ve[e];
-        }
-        __syncthreads();
-        if (warp * 16 >= nrows) continue;                   // this warp has no rows (it helped loading)
-        float sc[MK / 8][4];
-#pragma unroll
-        for (int nb = 0; nb < MK / 8; ++nb) sc[nb][0] = sc[nb][1] = sc[nb][2] = sc[nb][3] = 0.f;
-#pragma unroll
-        for (int ks = 0; ks < DK / 16; ++ks) {
+            for (int i = 0; i < 2; ++i) {
+                mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
+                mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
+                const float m_new = fmaxf(m[i], mx[i]);
+                alpha[i] = __expf(m[i] - m_new);
+                m[i] = m_new;
+                l[i] *= alpha[i];
+            }
 #pragma unroll
             for (int nb = 0; nb < MK / 8; ++nb) {
-                const uint32_t kb0 = *reinterpret_cast<const uint32_t*>(&k_s[nb * 8 + g][ks * 16 + 2 * t4]);
-                const uint32_t kb1 = *reinterpret_cast<const uint32_t*>(&k_s[nb * 8 + g][ks * 16 + 8 + 2 * t4]);
-                mma_bf16_16816(sc[nb], qa[ks], kb0, kb1);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    // the weight is rounded to bfloat16 for the second product: the fast exponential's error is far below that
+                    const float p = sc[nb][e] > -FLT_MAX ? __expf(sc[nb][e] - m[e >> 1]) : 0.f;
+                    sc[nb][e] = p;
+                    l[e >> 1] += p;                          // this lane's share; the quad's shares meet at the end
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < DV / 8; ++i) {
+                o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
+                o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
+            }
+            const bf16* vb = vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * Cfg::kVPitch + (lane >> 4) * 8;
+#pragma unroll
+            for (int kk = 0; kk < MK / 16; ++kk) {
+                uint32_t pa[4];
+                pa[0] = pack_bf16(sc[2 * kk][0], sc[2 * kk][1]);
+                pa[1] = pack_bf16(sc[2 * kk][2], sc[2 * kk][3]);
+                pa[2] = pack_bf16(sc[2 * kk + 1][0], sc[2 * kk + 1][1]);
+                pa[3] = pack_bf16(sc[2 * kk + 1][2], sc[2 * kk + 1][3]);
+#pragma unroll
+                for (int nb = 0; nb < DV / 8; nb += 2) {
+                    uint32_t f[4];
+                    awb_ldsm_x4_trans(f, vb + kk * 16 * Cfg::kVPitch + nb * 8);
+                    mma_bf16_16816(o[nb], pa, f[0], f[1]);
+                    mma_bf16_16816(o[nb + 1], pa, f[2], f[3]);
+                }
             }
         }
-        // scale, bias, window; the tile's row maxima
-        float mx[2] = {-FLT_MAX, -FLT_MAX};
-#pragma unroll
-        for (int nb = 0; nb < MK / 8; ++nb) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int r = row_a + (e >> 1) * 8;
-                const int kp = k0 + nb * 8 + 2 * t4 + (e & 1);
-                const int dist = pos_first + r - kp;
-                const bool seen = r < nrows && dist >= 0 && (window <= 0 || dist < window || kp < keep_first);
-                float v = -FLT_MAX;
-                if (seen) v = awb_cap(sc[nb][e] * scale, softcap) - ((tabled && dist < span) ? bias_s[dist] : awb_bias(bias_kind, b1h, b2h, (float)dist));
-                sc[nb][e] = v;
-                mx[e >> 1] = fmaxf(mx[e >> 1], v);
-            }
-        }
-        float alpha[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
-            mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
-            const float m_new = fmaxf(m[i], mx[i]);
-            alpha[i] = __expf(m[i] - m_new);
-            m[i] = m_new;
-            l[i] *= alpha[i];
-        }
-#pragma unroll
-        for (int nb = 0; nb < MK / 8; ++nb) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                // the weight is rounded to bfloat16 for the second product: the fast exponential's error is far below that
-                const float p = sc[nb][e] > -FLT_MAX ? __expf(sc[nb][e] - m[e >> 1]) : 0.f;
-                sc[nb][e] = p;
-                l[e >> 1] += p;                              // this lane's share; the quad's shares meet at the end
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < DV / 8; ++i) {
-            o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
-            o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
-        }
-#pragma unroll
-        for (int kb = 0; kb < MK / 16; ++kb) {
-            uint32_t pa[4];
-            pa[0] = pack_bf16(sc[2 * kb][0], sc[2 * kb][1]);
-            pa[1] = pack_bf16(sc[2 * kb][2], sc[2 * kb][3]);
-            pa[2] = pack_bf16(sc[2 * kb + 1][0], sc[2 * kb + 1][1]);
-            pa[3] = pack_bf16(sc[2 * kb + 1][2], sc[2 * kb + 1][3]);
-#pragma unroll
-            for (int nb = 0; nb < DV / 8; ++nb) {
-                const uint32_t vb0 = *reinterpret_cast<const uint32_t*>(&vt_s[nb * 8 + g][kb * 16 + 2 * t4]);
-                const uint32_t vb1 = *reinterpret_cast<const uint32_t*>(&vt_s[nb * 8 + g][kb * 16 + 8 + 2 * t4]);
-                mma_bf16_16816(o[nb], pa, vb0, vb1);
-            }
-        }
+        __syncthreads();                                     // this buffer is loaded again in the next round
+        tile = next;
+        stage ^= 1;
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
         l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
     }
+    const bool two_out = VD % 2 == 0 && ((uintptr_t)out & 3) == 0;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int r = row_a + i * 8;
@@ -539,8 +600,12 @@ attention_window_bias_mma_kernel(const bf16* __restrict__ q, bf16* __restrict__ 
 #pragma unroll
         for (int nb = 0; nb < DV / 8; ++nb) {
             const int c = nb * 8 + 2 * t4;
-            if (c < VD) dst[c] = __float2bfloat16_rn(o[nb][2 * i] * inv);
-            if (c + 1 < VD) dst[c + 1] = __float2bfloat16_rn(o[nb][2 * i + 1] * inv);
+            if (two_out && c < VD) {
+                *reinterpret_cast<uint32_t*>(dst + c) = pack_bf16(o[nb][2 * i] * inv, o[nb][2 * i + 1] * inv);
+            } else {
+                if (c < VD) dst[c] = __float2bfloat16_rn(o[nb][2 * i] * inv);
+                if (c + 1 < VD) dst[c + 1] = __float2bfloat16_rn(o[nb][2 * i + 1] * inv);
+            }
         }
     }
 }
@@ -552,8 +617,12 @@ static int launch_awb_mma(const void* q, void* out, const void* cache, const int
                           int skip_single, int RS, int voff, int bias_kind, int keep_first, const float* gate,
                           long long gate_ld, const float* sink, cudaStream_t stream) {
     const dim3 grid((unsigned)(T / MQ + nseq), (unsigned)nh);
+    constexpr int smem = AwbMma<DK, DV>::kSmem;
+    auto kern = attention_window_bias_mma_kernel<DK, DV>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    AP_REQUIRE(e == cudaSuccess, "attention_window_bias: cannot reserve %d bytes of shared memory", smem);
     AP_CHECK_PDL_LAUNCH("attention_window_bias_mma",
-                        ap_launch_pdl(attention_window_bias_mma_kernel<DK, DV>, grid, dim3(AWB_THREADS), 0, stream,
+                        ap_launch_pdl(kern, grid, dim3(AWB_THREADS), smem, stream,
                                       (const bf16*)q, (bf16*)out, (const bf16*)cache, block_table, max_blocks, seq_start,
                                       positions, nseq, nh, nkv, D, VD, P, (size_t)page_stride, scale, softcap, window, r1, r2,
                                       skip_single, RS, voff, bias_kind, keep_first, gate, gate_ld, sink));
