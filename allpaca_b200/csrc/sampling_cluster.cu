@@ -412,8 +412,12 @@ __device__ ScCut sc_search(cg::cluster_group& cl, ScShared& sh, int& parity, con
     return cut;
 }
 
-template <int E>
-__global__ void __launch_bounds__(SC_THREADS, 1)
+// PER_SM 2: two CTAs to an SM, for more rows than find room for their clusters at one (some 14: a cluster stays within a GPC); a
+// row is a chain of cluster barriers, and two rows hide each other's, though the registers are then tight.  Measured (one B200, top-k 40,
+// top-p 0.95, us, one and two to an SM): 8 rows of 32000 logits 32 and 35, 16 rows 49 and 35, 32 rows 69 and 37; of 128256 logits 8 rows 45
+// and 60, 16 rows 78 and 63, 24 rows 79 and 63, 64 rows 161 and 113.
+template <int E, int PER_SM>
+__global__ void __launch_bounds__(SC_THREADS, PER_SM)
 sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, int V,
                       const float* __restrict__ temperature, const int* __restrict__ top_k,
                       const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out,
@@ -653,8 +657,9 @@ static int sc_launch(const float* logits, long long row_stride, int R, int V, co
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ap_pdl_enabled() ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<E>, logits, row_stride, V, temperature, top_k,
-                                       top_p, uniform, out, host_out);
+    const bool many = E <= 32 && R > 12;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, many ? sample_cluster_kernel<E, E <= 32 ? 2 : 1> : sample_cluster_kernel<E, 1>, logits,
+                                       row_stride, V, temperature, top_k, top_p, uniform, out, host_out);
     AP_REQUIRE(e == cudaSuccess, "sample (cluster): launch failed: %s", cudaGetErrorString(e));
     return AP_OK;
 }
@@ -672,6 +677,7 @@ AP_EXPORT int ap_sample_cluster(const float* logits, long long row_stride, int R
     if (R == 0) return AP_OK;
     const int per = (V + SC_CLUSTER * SC_THREADS - 1) / (SC_CLUSTER * SC_THREADS);
     if (per <= 4) return sc_launch<4>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
+    if (per <= 8) return sc_launch<8>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
     if (per <= 16) return sc_launch<16>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
     if (per <= 32) return sc_launch<32>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
     return sc_launch<64>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
