@@ -564,34 +564,54 @@ __device__ __forceinline__ float moe_rows_sum8(const float* acc, int lane) {
     return a1;
 }
 
+// A shared expert (rows 0: none): all rows of the step, a [rows, K], w [N or 2 N, K], out [rows, N], riding in the same launch.
+template <typename TO> struct MoeShared {
+    const bf16 *a, *w;
+    TO* out;
+    int rows, N, K;
+};
 template <bool FIRST, bool GATED, typename TO>
 __global__ void __launch_bounds__(256)
 moe_rows_kernel(const bf16* __restrict__ A, long long lda, const bf16* __restrict__ W, long long w_expert_stride,
                 TO* __restrict__ C, long long ldc, const int* __restrict__ perm, int top, const int3* __restrict__ tiles,
                 int max_tiles, int N, int K, int act, float limit, float alpha, float shift,
-                const float* __restrict__ pair_scale) {
+                const float* __restrict__ pair_scale, const MoeShared<TO> X) {
     extern __shared__ __align__(16) bf16 a_s[];            // [ROWS_MAX][K]
     ap_pdl_trigger();
     ap_pdl_wait();
-    if ((int)blockIdx.y >= tiles[max_tiles].x) return;
-    const int3 tile = tiles[blockIdx.y];
+    // the last row of CTAs: the shared expert, every row of the step in its place
+    const bool shared = (int)blockIdx.y == max_tiles;
+    if (!shared && (int)blockIdx.y >= tiles[max_tiles].x) return;
+    const int3 tile = shared ? make_int3(0, 0, X.rows) : tiles[blockIdx.y];
     const int e = tile.x, p0 = tile.y, rows = tile.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bf16* We = W + (size_t)e * w_expert_stride;
+    if (shared) {
+        We = X.w;
+        A = X.a;
+        C = X.out;
+        N = X.N;
+        K = X.K;
+        lda = K;
+        ldc = N;
+    }
+    if (blockIdx.x * ROWS_COLS >= N) return;
+    const bool gathered = FIRST && !shared, scaled = !shared && pair_scale != nullptr;
     const int K8 = K / 8;
+    const int n_warp = blockIdx.x * ROWS_COLS + warp * (ROWS_COLS / 8);
     for (int r0 = 0; r0 < rows; r0 += ROWS_MAX) {
         const int R = min(ROWS_MAX, rows - r0);
         __syncthreads();
         for (int i = threadIdx.x; i < R * K8; i += 256) {
             const int r = i / K8, c = i - r * K8;
-            const int src = FIRST ? perm[p0 + r0 + r] / top : p0 + r0 + r;
+            const int src = gathered ? perm[p0 + r0 + r] / top : p0 + r0 + r;
             *reinterpret_cast<uint4*>(a_s + (size_t)r * K + c * 8) = *reinterpret_cast<const uint4*>(A + (size_t)src * lda + c * 8);
         }
         __syncthreads();
         // two weight rows at a time, so that what is read of the tile's rows serves both: a gate's and its up's, or (no
         // gate) two neighbouring columns'
         for (int cc = 0; cc < ROWS_COLS / 8; cc += GATED ? 1 : 2) {
-            const int n = blockIdx.x * ROWS_COLS + warp * (ROWS_COLS / 8) + cc;
+            const int n = n_warp + cc;
             if (n >= N) break;
             float acc[ROWS_MAX], acc2[ROWS_MAX];
 #pragma unroll
@@ -633,7 +653,7 @@ moe_rows_kernel(const bf16* __restrict__ A, long long lda, const bf16* __restric
             float v = moe_rows_sum8(acc, lane), v2 = moe_rows_sum8(acc2, lane);
             if ((lane & 3) == 0 && out_row < R) {
                 if constexpr (FIRST) {
-                    const float sc = pair_scale ? pair_scale[perm[p0 + r0 + out_row]] : 1.0f;
+                    const float sc = scaled ? pair_scale[perm[p0 + r0 + out_row]] : 1.0f;
                     if constexpr (GATED) v = gated_activation(v * sc, v2 * sc, act, limit, alpha, shift);
                     else {
                         v = gated_activation(v * sc, 1.0f, act, 0.f, 0.f, 0.f);
@@ -648,16 +668,27 @@ moe_rows_kernel(const bf16* __restrict__ A, long long lda, const bf16* __restric
     }
 }
 
+// the shared expert of a call, for the kernel above; false where it cannot take it
+template <typename TO> static bool moe_shared_args(MoeShared<TO>& X, const void* a, const void* w, void* out, int rows, int N, int K) {
+    X = MoeShared<TO>{(const bf16*)a, (const bf16*)w, (TO*)out, rows, N, K};
+    return rows == 0 || (rows > 0 && a && w && out && N > 0 && K > 0 && K % 8 == 0 && (size_t)ROWS_MAX * K * 2 <= 160 * 1024 &&
+                         ((((uintptr_t)a) | ((uintptr_t)w)) & 15) == 0);
+}
+
 // whether a step of `pairs` (row, choice) pairs in bfloat16 is one for the kernel above
 static bool moe_few_rows(int pairs, int E, int K, const void* a, const void* w) {
     return pairs <= 16 * E && K % 8 == 0 && (size_t)ROWS_MAX * K * 2 <= 160 * 1024 &&
            ((((uintptr_t)a) | ((uintptr_t)w)) & 15) == 0;
 }
 
-// a: [T, K]; w_gate_up: [E, 2 F, K], or (not `gated`) [E, F, K]; y: [pairs, F] in the activation type
+AP_EXPORT int ap_moe_rows_takes(const void* a, const void* w, int pairs, int E, int K) { return moe_few_rows(pairs, E, K, a, w); }
+
+// a: [T, K]; w_gate_up: [E, 2 F, K], or (not `gated`) [E, F, K]; y: [pairs, F] in the activation type.  x_rows > 0 (only where
+// ap_moe_rows_takes says so, all bfloat16): a shared expert beside them, x_a [x_rows, x_K], x_w [2 x_N or x_N, x_K] -> x_y [x_rows, x_N]
 AP_EXPORT int ap_moe_gate_up(const void* a, int a_dtype, const void* w, int w_dtype, void* y, int y_dtype,
                              const int* perm, int top, const int* tiles, int pairs, int E, int F, int K, int gated, int act,
-                             float limit, float alpha, float shift, const float* pair_scale, cudaStream_t stream) {
+                             float limit, float alpha, float shift, const float* pair_scale, const void* x_a, const void* x_w,
+                             void* x_y, int x_rows, int x_N, int x_K, cudaStream_t stream) {
     AP_REQUIRE(pairs >= 0 && E > 0 && F > 0 && K > 0 && top > 0 && act >= 0 && act <= ACT_RELU2, "moe_gate_up: bad sizes");
     AP_REQUIRE(gated || act != ACT_CLAMPED, "moe_gate_up: activation %d needs a gate", act);
     if (pairs == 0) return AP_OK;
@@ -672,8 +703,11 @@ AP_EXPORT int ap_moe_gate_up(const void* a, int a_dtype, const void* w, int w_dt
                                                      (TO*)y, (long long)F, perm, top, (const int3*)tiles, max_tiles, F, K, \
                                                      act, limit, alpha, shift, pair_scale))
     if (a_dtype == AP_BF16 && w_dtype == AP_BF16 && y_dtype == AP_BF16 && moe_few_rows(pairs, E, K, a, w)) {
-        const dim3 rgrid((unsigned)((F + ROWS_COLS - 1) / ROWS_COLS), (unsigned)max_tiles);
-        const size_t smem = (size_t)ROWS_MAX * K * sizeof(bf16);
+        MoeShared<bf16> X;
+        AP_REQUIRE(moe_shared_args(X, x_a, x_w, x_y, x_rows, x_N, x_K), "moe_gate_up: bad shared expert");
+        const int widest = x_rows > 0 && x_N > F ? x_N : F;
+        const dim3 rgrid((unsigned)((widest + ROWS_COLS - 1) / ROWS_COLS), (unsigned)(max_tiles + (x_rows > 0)));
+        const size_t smem = (size_t)ROWS_MAX * (x_rows > 0 && x_K > K ? x_K : K) * sizeof(bf16);
         auto kern = gated ? moe_rows_kernel<true, true, bf16> : moe_rows_kernel<true, false, bf16>;
         if (smem > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -681,9 +715,10 @@ AP_EXPORT int ap_moe_gate_up(const void* a, int a_dtype, const void* w, int w_dt
         }
         AP_CHECK_PDL_LAUNCH("moe_gate_up", ap_launch_pdl(kern, rgrid, dim3(256), smem, stream, (const bf16*)a, (long long)K,
                                                          (const bf16*)w, expert_stride, (bf16*)y, (long long)F, perm,
-                                                         top, (const int3*)tiles, max_tiles, F, K, act, limit, alpha, shift, pair_scale));
+                                                         top, (const int3*)tiles, max_tiles, F, K, act, limit, alpha, shift, pair_scale, X));
         return AP_OK;
     }
+    AP_REQUIRE(x_rows == 0, "moe_gate_up: a shared expert rides along only where few rows do");
     if (a_dtype == AP_F32 && w_dtype == AP_F32 && y_dtype == AP_F32) LAUNCH(float, float, float);
     else if (a_dtype == AP_BF16 && w_dtype == AP_BF16 && y_dtype == AP_BF16) LAUNCH(bf16, bf16, bf16);
     else if (a_dtype == AP_BF16 && w_dtype == AP_F32 && y_dtype == AP_BF16) LAUNCH(bf16, float, bf16);
@@ -695,7 +730,8 @@ AP_EXPORT int ap_moe_gate_up(const void* a, int a_dtype, const void* w, int w_dt
 
 // y: [pairs, F]; w_down: [E, H, F]; o: [pairs, H] 32-bit
 AP_EXPORT int ap_moe_down(const void* y, int y_dtype, const void* w, int w_dtype, float* o, const int* tiles, int pairs,
-                          int E, int H, int F, cudaStream_t stream) {
+                          int E, int H, int F, const void* x_y, const void* x_w, float* x_o, int x_rows, int x_N, int x_K,
+                          cudaStream_t stream) {
     AP_REQUIRE(pairs >= 0 && E > 0 && F > 0 && H > 0, "moe_down: bad sizes");
     if (pairs == 0) return AP_OK;
     const int max_tiles = ap_moe_max_tiles(pairs, E);
@@ -707,8 +743,11 @@ AP_EXPORT int ap_moe_down(const void* y, int y_dtype, const void* w, int w_dtype
                                                   (long long)H, (const int*)nullptr, 1, (const int3*)tiles, max_tiles, H, \
                                                   F, 0, 0.f, 0.f, 0.f, (const float*)nullptr))
     if (y_dtype == AP_BF16 && w_dtype == AP_BF16 && moe_few_rows(pairs, E, F, y, w)) {
-        const dim3 rgrid((unsigned)((H + ROWS_COLS - 1) / ROWS_COLS), (unsigned)max_tiles);
-        const size_t smem = (size_t)ROWS_MAX * F * sizeof(bf16);
+        MoeShared<float> X;
+        AP_REQUIRE(moe_shared_args(X, x_y, x_w, x_o, x_rows, x_N, x_K), "moe_down: bad shared expert");
+        const int widest = x_rows > 0 && x_N > H ? x_N : H;
+        const dim3 rgrid((unsigned)((widest + ROWS_COLS - 1) / ROWS_COLS), (unsigned)(max_tiles + (x_rows > 0)));
+        const size_t smem = (size_t)ROWS_MAX * (x_rows > 0 && x_K > F ? x_K : F) * sizeof(bf16);
         auto kern = moe_rows_kernel<false, false, float>;
         if (smem > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -717,9 +756,10 @@ AP_EXPORT int ap_moe_down(const void* y, int y_dtype, const void* w, int w_dtype
         AP_CHECK_PDL_LAUNCH("moe_down", ap_launch_pdl(kern, rgrid, dim3(256), smem, stream, (const bf16*)y, (long long)F,
                                                       (const bf16*)w, (long long)H * F, o, (long long)H,
                                                       (const int*)nullptr, 1, (const int3*)tiles, max_tiles, H, F, 0, 0.f,
-                                                      0.f, 0.f, (const float*)nullptr));
+                                                      0.f, 0.f, (const float*)nullptr, X));
         return AP_OK;
     }
+    AP_REQUIRE(x_rows == 0, "moe_down: a shared expert rides along only where few rows do");
     if (y_dtype == AP_F32 && w_dtype == AP_F32) LAUNCH(float, float);
     else if (y_dtype == AP_BF16 && w_dtype == AP_BF16) LAUNCH(bf16, bf16);
     else if (y_dtype == AP_BF16 && w_dtype == AP_F32) LAUNCH(bf16, float);

@@ -19,6 +19,10 @@
 // 8192 pairs 185 (743 TFLOP/s) and 168.  What was before: on the CUDA cores 41 and 21, 76 and 39; prompts a launch per expert and product
 // behind a copy of first[] to the host, 37 and 29 us per expert of the latter.
 //
+// A shared expert that all rows use (rows, sizes, matrix and result of its own) may ride along: its items follow the routed
+// ones, so it costs its bytes and no launch (4 rows, 10 of 16 experts of 2048 x 1024 with gates and a shared one of the same size: 21.4 and
+// 12.8 us; 20.1 and 12.5 without it, whose own two products took 4.4 and 3.9).
+//
 // A row's sums run over K in one order whatever tile it lies in: its result does not depend on the other rows.
 //
 // Every barrier wait has a time limit; on expiry the status word is raised, loads in flight are let land, tensor memory is
@@ -54,21 +58,32 @@ struct MoeTcArgs {
     int experts, NT, N, K, act;
     long long ldc;
     float limit, alpha, shift;
+    int x_rows, x_NT, x_N, x_K;        // the shared expert (x_rows 0: none); its results are x_N wide
 };
 
 struct MoeItem {
-    int e, j, p0, rows, width;  // expert, weight tile, first row, rows, rows rounded up to 16
+    int e, j, p0, rows, width;  // expert (-1: the shared one), weight tile, first row, rows, rows rounded up to 16
 };
 
 // item `it` of the walk; first[] and the experts' row tiles before each (cum) lie in shared memory
-template <int BN> __device__ __forceinline__ MoeItem moe_item(const int* first, const int* cum, int experts, int NT, int it) {
+template <int BN> __device__ __forceinline__ MoeItem moe_item(const int* first, const int* cum, const MoeTcArgs& g, int it) {
+    const int experts = g.experts, NT = g.NT;
+    MoeItem w;
+    if (it >= cum[experts] * NT) {
+        const int x = it - cum[experts] * NT, tiles = (g.x_rows + BN - 1) / BN;
+        w.e = -1;
+        w.j = x / tiles;
+        w.width = ((g.x_rows + tiles - 1) / tiles + 15) & ~15;
+        w.p0 = (x - w.j * tiles) * w.width;
+        w.rows = min(w.width, g.x_rows - w.p0);
+        return w;
+    }
     int lo = 0, hi = experts;                    // cum[lo] NT <= it < cum[hi] NT
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
         if (cum[mid] * NT <= it) lo = mid;
         else hi = mid;
     }
-    MoeItem w;
     w.e = lo;
     const int tiles = cum[lo + 1] - cum[lo], local = it - cum[lo] * NT;
     w.j = local / tiles;
@@ -144,8 +159,9 @@ template <typename TO> __device__ __forceinline__ void mt_store(TO* o, long long
 
 template <int BN, int SUB, bool GATED, typename TO>
 __global__ void __launch_bounds__(MT_THREADS)
-moe_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, TO* __restrict__ out,
-              const MoeTcArgs g) {
+moe_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
+              const __grid_constant__ CUtensorMap tmap_xw, const __grid_constant__ CUtensorMap tmap_xa, TO* __restrict__ out,
+              TO* __restrict__ x_out, const MoeTcArgs g) {
     using Cfg = MoeTile<BN, SUB>;
     constexpr int STAGES = Cfg::kStages;
     extern __shared__ uint8_t smem_raw[];
@@ -200,22 +216,24 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     }
     __syncthreads();
     const uint32_t tmem_base = *tmem_slot;
-    const int items = *abort_flag ? 0 : cum[g.experts] * g.NT;
-    const int nkb = (g.K + MT_K - 1) / MT_K;
+    const int items = *abort_flag ? 0 : cum[g.experts] * g.NT + (g.x_rows + BN - 1) / BN * g.x_NT;
     if (SUB == 1) ap_pdl_trigger();
 
     if (warp == 0) {
         if (lane == 0) {
             int b = 0;                           // blocks asked for so far
             for (int it = blockIdx.x; it < items && !*abort_flag; it += gridDim.x) {
-                const MoeItem w = moe_item<BN>(first, cum, g.experts, g.NT, it);
-                const int w_rows = GATED ? 2 * g.N : g.N;
+                const MoeItem w = moe_item<BN>(first, cum, g, it);
+                const bool shared = w.e < 0;
+                const int N = shared ? g.x_N : g.N, nkb = ((shared ? g.x_K : g.K) + MT_K - 1) / MT_K;
+                const CUtensorMap *mw = shared ? &tmap_xw : &tmap_w, *ma = shared ? &tmap_xa : &tmap_a;
+                const int w_rows = shared ? 0 : GATED ? 2 * N : N;
                 int row[2 * SUB];
 #pragma unroll
                 for (int s = 0; s < 2 * SUB; ++s) {
-                    if (GATED) row[s] = SUB == 1 ? w.j * 64 + s * g.N : w.j * 128 + (s >> 1) * g.N + (s & 1) * 64;
+                    if (GATED) row[s] = SUB == 1 ? w.j * 64 + s * N : w.j * 128 + (s >> 1) * N + (s & 1) * 64;
                     else row[s] = w.j * 128 * SUB + s * 64;
-                    row[s] += w.e * w_rows;
+                    row[s] += (shared ? 0 : w.e) * w_rows;
                 }
                 const int boxes = (w.width + Cfg::kABox - 1) / Cfg::kABox;
                 const uint32_t bytes = Cfg::kWBytes + boxes * Cfg::kABox * MT_K * 2;
@@ -230,9 +248,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
                     uint8_t* stage = smem + s * Cfg::kStageBytes;
                     tc::mbar_expect_tx(&full[s], bytes);
 #pragma unroll
-                    for (int i = 0; i < 2 * SUB; ++i) tc::tma_load_2d(stage + i * MT_BOX, &tmap_w, k * MT_K, row[i], &full[s]);
+                    for (int i = 0; i < 2 * SUB; ++i) tc::tma_load_2d(stage + i * MT_BOX, mw, k * MT_K, row[i], &full[s]);
                     for (int i = 0; i < boxes; ++i)
-                        tc::tma_load_2d(stage + Cfg::kWBytes + i * Cfg::kABox * MT_K * 2, &tmap_a, k * MT_K,
+                        tc::tma_load_2d(stage + Cfg::kWBytes + i * Cfg::kABox * MT_K * 2, ma, k * MT_K,
                                         w.p0 + i * Cfg::kABox, &full[s]);
                 }
             }
@@ -243,7 +261,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
         if (lane == 0) {
             int b = 0, n = 0;
             for (int it = blockIdx.x; it < items && !*abort_flag; it += gridDim.x, ++n) {
-                const MoeItem w = moe_item<BN>(first, cum, g.experts, g.NT, it);
+                const MoeItem w = moe_item<BN>(first, cum, g, it);
+                const int nkb = ((w.e < 0 ? g.x_K : g.K) + MT_K - 1) / MT_K;
                 const uint32_t idesc = tc::instr_desc_bf16_f32(128, w.width);
                 const int buf = n & 1;
                 const uint32_t acc = tmem_base + (uint32_t)(buf * SUB * BN);
@@ -284,7 +303,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
         const int q = warp & 3, row = q * 32 + lane;
         int n = 0;
         for (int it = blockIdx.x; it < items; it += gridDim.x, ++n) {
-            const MoeItem w = moe_item<BN>(first, cum, g.experts, g.NT, it);
+            const MoeItem w = moe_item<BN>(first, cum, g, it);
             const int buf = n & 1;
             const bool have = !*abort_flag && tc::mbar_wait(&acc_full[buf], (n >> 1) & 1);
             if (!have && !*abort_flag) {
@@ -294,10 +313,14 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
             if (!mt_all(have)) break;                                 // all four warps agree, as they meet at barriers below
             tc::fence_after_sync();
             const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * SUB * BN);
+            const int N = w.e < 0 ? g.x_N : g.N;
+            const long long ldc = w.e < 0 ? g.x_N : g.ldc;
+            TO* to = w.e < 0 ? x_out : out;
+            const bool scaled = g.pair_scale != nullptr && w.e >= 0;
 #pragma unroll 1
             for (int c = 0; c < w.rows; c += 16) {
                 float scale = 1.0f;                                  // of row c + lane % 16
-                if (g.pair_scale != nullptr && c + (lane & 15) < w.rows) scale = g.pair_scale[g.perm[w.p0 + c + (lane & 15)]];
+                if (scaled && c + (lane & 15) < w.rows) scale = g.pair_scale[g.perm[w.p0 + c + (lane & 15)]];
                 uint32_t v[16], u[16];
                 tc::tmem_ld_x16(acc + (uint32_t)c, v);
                 if (SUB == 2) tc::tmem_ld_x16(acc + (uint32_t)(BN + c), u);
@@ -321,7 +344,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
                     x[i] = __uint_as_float(v[i]);
                     y[i] = SUB == 2 || GATED ? __uint_as_float(u[i]) : 1.0f;
                 }
-                if (g.pair_scale != nullptr) {
+                if (scaled) {
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const float sc = __shfl_sync(0xffffffffu, scale, i);
@@ -333,12 +356,12 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
                 const int left = w.rows - c;
                 if constexpr (GATED) {
                     const int n0 = SUB == 1 ? w.j * 64 + row : w.j * 128 + row;
-                    if ((SUB == 2 || row < 64) && n0 < g.N) mt_store(out + (size_t)(w.p0 + c) * g.ldc + n0, g.ldc, x, left);
+                    if ((SUB == 2 || row < 64) && n0 < N) mt_store(to + (size_t)(w.p0 + c) * ldc + n0, ldc, x, left);
                 } else {
                     const int n0 = w.j * 128 * SUB + row;
-                    TO* o = out + (size_t)(w.p0 + c) * g.ldc + n0;
-                    if (n0 < g.N) mt_store(o, g.ldc, x, left);
-                    if (SUB == 2 && n0 + 128 < g.N) mt_store(o + 128, g.ldc, y, left);
+                    TO* o = to + (size_t)(w.p0 + c) * ldc + n0;
+                    if (n0 < N) mt_store(o, ldc, x, left);
+                    if (SUB == 2 && n0 + 128 < N) mt_store(o + 128, ldc, y, left);
                 }
             }
             tc::fence_before_sync();
@@ -378,23 +401,31 @@ static bool moe_map(CUtensorMap* map, const void* base, long long rows, long lon
 }
 
 template <int BN, int SUB, bool GATED, typename TO>
-static int moe_launch(const void* a, const void* w, void* out, const MoeTcArgs& args, int pairs, cudaStream_t stream) {
+static int moe_launch(const void* a, const void* w, void* out, const MoeTcArgs& args, int pairs, const void* x_a,
+                      const void* x_w, void* x_out, cudaStream_t stream) {
     using Cfg = MoeTile<BN, SUB>;
-    CUtensorMap tw, ta;
+    CUtensorMap tw, ta, txw, txa;
     AP_REQUIRE(moe_map(&tw, w, (long long)args.experts * (GATED ? 2 : 1) * args.N, args.K, 64) &&
                    moe_map(&ta, a, pairs, args.K, Cfg::kABox),
                "moe_tc: cannot encode the tensor maps");
+    txw = tw;
+    txa = ta;
+    AP_REQUIRE(args.x_rows == 0 || (moe_map(&txw, x_w, (long long)(GATED ? 2 : 1) * args.x_N, args.x_K, 64) &&
+                                    moe_map(&txa, x_a, args.x_rows, args.x_K, Cfg::kABox)),
+               "moe_tc: cannot encode the shared expert's tensor maps");
     auto kern = moe_tc_kernel<BN, SUB, GATED, TO>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
     AP_REQUIRE(e == cudaSuccess, "moe_tc: cannot reserve %d bytes of shared memory: %s", Cfg::kSmem, cudaGetErrorString(e));
     MoeTcArgs g = args;
     const int cols = (GATED ? 64 : 128) * SUB;                // results per weight tile
     g.NT = (g.N + cols - 1) / cols;
-    const long long most = (long long)((pairs < g.experts ? pairs : g.experts) + pairs / BN) * g.NT;
+    g.x_NT = (g.x_N + cols - 1) / cols;
+    const long long most = (long long)((pairs < g.experts ? pairs : g.experts) + pairs / BN) * g.NT +
+                           (long long)((g.x_rows + BN - 1) / BN) * g.x_NT;
     AP_REQUIRE(most < 0x7fffffffLL, "moe_tc: too many tiles");
     const long long room = SUB == 1 ? 2 * 148 : 148;
     AP_CHECK_PDL_LAUNCH("moe_tc", ap_launch_pdl(kern, dim3((unsigned)(most < room ? most : room)), dim3(MT_THREADS), Cfg::kSmem,
-                                                stream, tw, ta, (TO*)out, g));
+                                                stream, tw, ta, txw, txa, (TO*)out, (TO*)x_out, g));
     return AP_OK;
 }
 
@@ -412,10 +443,15 @@ AP_EXPORT int ap_moe_tc_takes(const void* a, const void* w, int pairs, int E, in
            (long long)E * N < 0x7fffffffLL;
 }
 
-// a: [pairs, K] in grouped order; w: [E, 2 N, K] (gated) or [E, N, K]; out: [pairs, N]; first: [E + 1]; act: -1 for none
+// a: [pairs, K] in grouped order; w: [E, 2 N, K] (gated) or [E, N, K]; out: [pairs, N]; first: [E + 1]; act: -1 for none.
+// x_rows > 0: the shared expert, x_a [x_rows, x_K], x_w [2 x_N or x_N, x_K], x_out [x_rows, x_N], the same activation, unscaled
 AP_EXPORT int ap_moe_tc(const void* a, const void* w, void* out, int out_dtype, const int* first, int pairs, int E, int N,
                         int K, int gated, int act, float limit, float alpha, float shift, const float* pair_scale,
-                        const int* perm, cudaStream_t stream) {
+                        const int* perm, const void* x_a, const void* x_w, void* x_out, int x_rows, int x_N, int x_K,
+                        cudaStream_t stream) {
+    AP_REQUIRE(x_rows == 0 || (x_rows > 0 && x_a && x_w && x_out && x_N > 0 && x_K > 0 && x_K % 8 == 0 &&
+                               (((uintptr_t)x_a | (uintptr_t)x_w) & 15) == 0),
+               "moe_tc: bad shared expert of %d rows, %d x %d", x_rows, x_N, x_K);
     AP_REQUIRE(pairs >= 0 && E > 0 && E <= MT_MAX_EXPERTS && N > 0 && K > 0 && K % 8 == 0, "moe_tc: bad sizes pairs=%d experts=%d N=%d K=%d",
                pairs, E, N, K);
     AP_REQUIRE(act >= (gated ? 0 : -1) && act <= ACT_RELU2 && (gated || act != ACT_CLAMPED), "moe_tc: activation %d", act);
@@ -423,13 +459,13 @@ AP_EXPORT int ap_moe_tc(const void* a, const void* w, void* out, int out_dtype, 
     AP_REQUIRE(pair_scale == nullptr || perm != nullptr, "moe_tc: scales go by the permutation");
     AP_REQUIRE((long long)E * (gated ? 2 : 1) * N < 0x7fffffffLL, "moe_tc: too many weight rows");
     if (pairs == 0) return AP_OK;
-    const MoeTcArgs g{first, pair_scale, perm, E, 0, N, K, act, (long long)N, limit, alpha, shift};
+    const MoeTcArgs g{first, pair_scale, perm, E, 0, N, K, act, (long long)N, limit, alpha, shift, x_rows, 0, x_N, x_K};
     const int mean = (pairs + E - 1) / E;
 #define LAUNCH(BN, SUB)                                                                                                \
     do {                                                                                                               \
-        if (gated && out_dtype == AP_BF16) return moe_launch<BN, SUB, true, bf16>(a, w, out, g, pairs, stream);        \
-        if (!gated && out_dtype == AP_BF16) return moe_launch<BN, SUB, false, bf16>(a, w, out, g, pairs, stream);      \
-        if (!gated && out_dtype == AP_F32) return moe_launch<BN, SUB, false, float>(a, w, out, g, pairs, stream);      \
+        if (gated && out_dtype == AP_BF16) return moe_launch<BN, SUB, true, bf16>(a, w, out, g, pairs, x_a, x_w, x_out, stream);        \
+        if (!gated && out_dtype == AP_BF16) return moe_launch<BN, SUB, false, bf16>(a, w, out, g, pairs, x_a, x_w, x_out, stream);      \
+        if (!gated && out_dtype == AP_F32) return moe_launch<BN, SUB, false, float>(a, w, out, g, pairs, x_a, x_w, x_out, stream);      \
         AP_REQUIRE(false, "moe_tc: unsupported out dtype %d", out_dtype);                                              \
     } while (0)
     if (2 * mean <= 16) LAUNCH(16, 1);

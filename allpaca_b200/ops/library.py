@@ -91,14 +91,17 @@ _CORE_SIGNATURES = {
     "ap_moe_sort": [_P, _P, _P, _P, _P, _I, _I, _I, _P],
     # int ap_moe_tc_takes(a, w, pairs, E, N, K)
     "ap_moe_tc_takes": [_P, _P, _I, _I, _I, _I],
-    # int ap_moe_tc(a, w, out, out_dtype, first, pairs, E, N, K, gated, act, limit, alpha, shift, pair_scale, perm, stream)
-    "ap_moe_tc": [_P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _F, _F, _P, _P, _P],
+    # int ap_moe_tc(a, w, out, out_dtype, first, pairs, E, N, K, gated, act, limit, alpha, shift, pair_scale, perm,
+    #               x_a, x_w, x_out, x_rows, x_N, x_K, stream)
+    "ap_moe_tc": [_P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _F, _F, _P, _P, _P, _P, _P, _I, _I, _I, _P],
     "ap_moe_gather": [_P, _P, _P, _I, _I, _I, _P],
     # int ap_moe_gate_up(a, a_dtype, w, w_dtype, y, y_dtype, perm, top, tiles, pairs, E, F, K, gated, act, limit,
-    #                    alpha, shift, pair_scale, stream)
-    "ap_moe_gate_up": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _F, _F, _P, _P],
-    # int ap_moe_down(y, y_dtype, w, w_dtype, o, tiles, pairs, E, H, F, stream)
-    "ap_moe_down": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _P],
+    #                    alpha, shift, pair_scale, x_a, x_w, x_y, x_rows, x_N, x_K, stream)
+    "ap_moe_gate_up": [_P, _I, _P, _I, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _F, _F, _P, _P, _P, _P, _I, _I, _I, _P],
+    # int ap_moe_down(y, y_dtype, w, w_dtype, o, tiles, pairs, E, H, F, x_y, x_w, x_o, x_rows, x_N, x_K, stream)
+    "ap_moe_down": [_P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _P, _P, _P, _I, _I, _I, _P],
+    # int ap_moe_rows_takes(a, w, pairs, E, K)
+    "ap_moe_rows_takes": [_P, _P, _I, _I, _I],
     # int ap_moe_combine(o, place, weight, delta, T, H, top, chosen, real, rows, rows_dtype, base, stream)
     "ap_moe_combine": [_P, _P, _P, _P, _I, _I, _I, _P, _I, _P, _I, _P, _P],
     # int ap_add_dyt(x, delta, S, delta_stride, w, b, alpha, out, out_dtype, rows, R, H, stream)

@@ -132,12 +132,14 @@ def moe_gather(a: torch.Tensor, out: torch.Tensor, perm: torch.Tensor, top: int)
 
 def moe_gate_up(a: torch.Tensor, w: torch.Tensor, y: torch.Tensor, perm: torch.Tensor, top: int, tiles: torch.Tensor,
                 activation: str, limit: float = 0.0, alpha: float = 1.0, shift: float = 0.0,
-                experts: Optional[int] = None, pair_scale: Optional[torch.Tensor] = None, gated: bool = True) -> None:
+                experts: Optional[int] = None, pair_scale: Optional[torch.Tensor] = None, gated: bool = True,
+                shared=None) -> None:
     """For every row tile: ``y[p] = act(a[perm[p] // top] W_gate[e]^T, ... W_up[e]^T)`` with
     ``w [E, 2F, K]`` (gate rows, then up rows of each expert) and ``y [pairs, F]``.  ``experts``: the
     number the pairs were sorted by, where that is more than the experts that have weights.  ``pair_scale`` (32-bit
     ``[pairs]`` by pair ``t * top + k``): the pair's input row counts that many times, so both sums are multiplied
-    by it before the activation.  ``gated`` False: ``w [E, F, K]`` and ``y[p] = act(a[...] W[e]^T)``."""
+    by it before the activation.  ``gated`` False: ``w [E, F, K]`` and ``y[p] = act(a[...] W[e]^T)``.
+    ``shared`` (where :func:`moe_rows_taken`): as for :func:`moe_products`."""
     _check(a, "a", dims=2)
     _check(w, "w", dims=3)
     _check(y, "y", dims=2)
@@ -149,12 +151,13 @@ def moe_gate_up(a: torch.Tensor, w: torch.Tensor, y: torch.Tensor, perm: torch.T
          dtype_code(y.dtype), perm.data_ptr(), int(top), tiles.data_ptr(), pairs, int(experts or E), F, K,
          1 if gated else 0, activation_code(activation),
          float(limit), float(alpha), float(shift), pair_scale.data_ptr() if pair_scale is not None else 0,
-         stream_handle())
+         *_shared(shared, gated, y.dtype), stream_handle())
 
 
-def moe_down(y: torch.Tensor, w: torch.Tensor, o: torch.Tensor, tiles: torch.Tensor, experts: Optional[int] = None) -> None:
+def moe_down(y: torch.Tensor, w: torch.Tensor, o: torch.Tensor, tiles: torch.Tensor, experts: Optional[int] = None,
+             shared=None) -> None:
     """For every row tile: ``o[p] = y[p] W_down[e]^T`` with ``w [E, H, F]``; ``o [pairs, H]`` 32-bit.
-    ``experts``: as for :func:`moe_gate_up`."""
+    ``experts``, ``shared``: as for :func:`moe_gate_up`."""
     _check(y, "y", dims=2)
     _check(w, "w", dims=3)
     _check(o, "o", torch.float32, 2)
@@ -163,7 +166,7 @@ def moe_down(y: torch.Tensor, w: torch.Tensor, o: torch.Tensor, tiles: torch.Ten
     if F2 != F or tuple(o.shape) != (pairs, H):
         raise KernelError(f"moe_down: shapes disagree: y {tuple(y.shape)}, w {tuple(w.shape)}, o {tuple(o.shape)}")
     call(core(), "ap_moe_down", y.data_ptr(), dtype_code(y.dtype), w.data_ptr(), dtype_code(w.dtype), o.data_ptr(),
-         tiles.data_ptr(), pairs, int(experts or E), H, F, stream_handle())
+         tiles.data_ptr(), pairs, int(experts or E), H, F, *_shared(shared, False, o.dtype), stream_handle())
 
 
 def moe_products_taken(a: torch.Tensor, w: torch.Tensor, pairs: int) -> bool:
@@ -174,14 +177,37 @@ def moe_products_taken(a: torch.Tensor, w: torch.Tensor, pairs: int) -> bool:
     return bool(core().ap_moe_tc_takes(a.data_ptr(), w.data_ptr(), int(pairs), E, N, K))
 
 
+def moe_rows_taken(a: torch.Tensor, w: torch.Tensor, pairs: int, experts: int) -> bool:
+    """Whether :func:`moe_gate_up` and :func:`moe_down` take ``pairs`` rows of ``a``'s width with the kernel for few rows
+    (``experts``: the number the pairs are sorted by), beside which a shared expert can ride."""
+    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or not w.is_cuda:
+        return False
+    return bool(core().ap_moe_rows_takes(a.data_ptr(), w.data_ptr(), int(pairs), int(experts), w.shape[2]))
+
+
+def _shared(shared, gated: bool, out_dtype) -> tuple:
+    """The arguments of a shared expert that rides along: ``(rows [T, K], w [N or 2N, K], out [T, N])`` or None."""
+    if shared is None:
+        return 0, 0, 0, 0, 0, 0
+    a, w, out = shared
+    _check(a, "shared rows", torch.bfloat16, 2)
+    _check(w, "shared w", torch.bfloat16, 2)
+    _check(out, "shared out", out_dtype, 2)
+    rows, N = out.shape
+    if tuple(a.shape) != (rows, w.shape[1]) or w.shape[0] != (2 * N if gated else N):
+        raise KernelError(f"a shared expert's shapes disagree: rows {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    return a.data_ptr(), w.data_ptr(), out.data_ptr(), rows, N, w.shape[1]
+
+
 def moe_products(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, first: torch.Tensor, gated: bool = False,
                  activation: Optional[str] = None, limit: float = 0.0, alpha: float = 1.0, shift: float = 0.0,
-                 pair_scale: Optional[torch.Tensor] = None, perm: Optional[torch.Tensor] = None) -> None:
+                 pair_scale: Optional[torch.Tensor] = None, perm: Optional[torch.Tensor] = None, shared=None) -> None:
     """``out[p] = a[p] W[e]^T`` for the rows ``first[e] <= p < first[e + 1]`` of every expert, on the tensor cores:
     bfloat16 ``a [pairs, K]`` in grouped order, ``w [E, N, K]``, ``first`` int32 of at least ``E + 1``; rows from
     ``first[E]`` on are left alone.  ``activation``: of the 32-bit sums (:func:`gated_act`); with ``gated`` ``w`` is
     ``[E, 2N, K]`` (gate rows, then up rows of each expert) and ``out[p] = act(gate, up)``.  ``pair_scale`` (32-bit, by
-    ``perm[p]``): multiplies the sums before the activation."""
+    ``perm[p]``): multiplies the sums before the activation.  ``shared`` ``(rows, w, out)``: one more expert, of its own
+    sizes, for all those rows, under the same activation and unscaled."""
     _check(a, "a", torch.bfloat16, 2)
     _check(w, "w", torch.bfloat16, 3)
     _check(out, "out", dims=2)
@@ -200,7 +226,7 @@ def moe_products(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, first: tor
     call(core(), "ap_moe_tc", a.data_ptr(), w.data_ptr(), out.data_ptr(), dtype_code(out.dtype), first.data_ptr(), pairs, E,
          N, K, 1 if gated else 0, -1 if activation is None else activation_code(activation), float(limit), float(alpha),
          float(shift), pair_scale.data_ptr() if pair_scale is not None else 0, perm.data_ptr() if perm is not None else 0,
-         stream_handle())
+         *_shared(shared, gated, out.dtype), stream_handle())
 
 
 def moe_combine(o: torch.Tensor, place: torch.Tensor, weight: torch.Tensor, delta: torch.Tensor,

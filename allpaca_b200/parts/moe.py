@@ -93,7 +93,8 @@ class RoutedExperts(FeedForward):
                             f"not a routing")
         self.share_scale = float(p.get("share_scale", 1.0))
         self.first_rows = (2 if self.gated else 1) * self.inter       # rows of an expert's first matrix
-        self.shared = self.shared_gate = None
+        self.shared = self.shared_gate = self.shared_first = self.shared_down = None
+        self.shared_rides = False
         if p.get("shared"):
             sh = dict(p["shared"])
             one = {"hidden_size": self.hidden, "intermediate_size": int(sh["size"]),
@@ -104,6 +105,10 @@ class RoutedExperts(FeedForward):
                 one.update(names=("shared.up", "shared.down"), bias=False)
             self.shared = build("feed_forward", PartSpec("swiglu" if self.gated else "dense_act", one), env)
             self.shared_gated = bool(sh.get("gate", False))
+            # with the experts' activation it can ride in their launches, as one more expert of its own size
+            self.shared_size = int(sh["size"])
+            self.shared_rides = (env.dtype == torch.bfloat16 and one["activation"] == self.activation != "clamped_sigmoid"
+                                 and self.hidden % 8 == 0 and self.shared_size % 8 == 0)
 
     def parts(self):
         yield self
@@ -130,6 +135,10 @@ class RoutedExperts(FeedForward):
         if self.shared is not None:
             self.shared.load({n: tensors[n] for n in self.shared.weights()})
             self.shared_gate = tensors["shared.sg"].reshape(-1).contiguous() if self.shared_gated else None
+            if self.shared_rides and tensors["shared.up"].dtype == tensors["shared.down"].dtype == torch.bfloat16:
+                self.shared_first = torch.cat([tensors["shared.gate"], tensors["shared.up"]]).contiguous() if self.gated \
+                    else tensors["shared.up"].contiguous()
+                self.shared_down = tensors["shared.down"].contiguous()
         self.router_b = tensors[self.router_bias_name].float().contiguous() if self.router_bias else None
         # [experts, 2 F, hidden]: an expert's gate rows, then its up rows (without gates [experts, F, hidden]);
         # [experts, hidden, F]
@@ -159,22 +168,32 @@ class RoutedExperts(FeedForward):
         tiles = ws.get("moe.tiles", (ops.moe_max_tiles(pairs, self.outputs) + 1, 3), torch.int32)
         y = ws.get("moe.act", (pairs, self.inter), self.env.dtype)
         o = ws.get("moe.out", (pairs, self.hidden), torch.float32)
-        if self._on_tensor_cores(h, pairs):
+        tensor_cores = self._on_tensor_cores(h, pairs)
+        other = first_shared = second_shared = None
+        ys = ws.get("moe.shared_act", (T, self.shared_size), self.env.dtype) if self.shared_first is not None else None
+        if ys is not None and (tensor_cores or (self.experts > 0 and all(
+                ops.moe_rows_taken(t, m, pairs, self.outputs)
+                for t, m in ((h, self.gate_up), (y, self.down), (ys, self.shared_down[None]))))):
+            other = ws.get("moe.shared_out", (1, T, self.hidden), torch.float32)
+            first_shared, second_shared = (h, self.shared_first, ys), (ys, self.shared_down, other[0])
+        if tensor_cores:
             first = ws.get("moe.offsets", (self.outputs + 1,), torch.int32)
             ops.moe_sort(chosen, perm, place, tiles, self.outputs, first, real=self.experts)
             rows = ws.get("moe.rows", (pairs, self.hidden), torch.bfloat16)
             ops.moe_gather(h, rows, perm, self.top)
             ops.moe_products(rows, self.gate_up, y, first, gated=self.gated, activation=self.activation, limit=self.limit,
-                             alpha=self.alpha, shift=self.shift, pair_scale=weight.view(-1) if on_input else None, perm=perm)
-            ops.moe_products(y, self.down, o, first)
+                             alpha=self.alpha, shift=self.shift, pair_scale=weight.view(-1) if on_input else None, perm=perm,
+                             shared=first_shared)
+            ops.moe_products(y, self.down, o, first, shared=second_shared)
         else:
             ops.moe_sort(chosen, perm, place, tiles, self.outputs, real=self.experts)
             ops.moe_gate_up(h, self.gate_up, y, perm, self.top, tiles, self.activation, self.limit, self.alpha,
                             self.shift, experts=self.outputs, pair_scale=weight.view(-1) if on_input else None,
-                            gated=self.gated)
-            ops.moe_down(y, self.down, o, tiles, experts=self.outputs)
+                            gated=self.gated, shared=first_shared)
+            ops.moe_down(y, self.down, o, tiles, experts=self.outputs, shared=second_shared)
         delta = ws.get("moe.delta", (1, T, self.hidden), torch.float32)
-        other = self.shared.forward(h, step) if self.shared is not None else None
+        if self.shared is not None and other is None:
+            other = self.shared.forward(h, step)
         base = other[0] if other is not None and self.shared_gate is None else None
         if self.identity > 0:
             ops.moe_combine(o, place, weight, delta[0], chosen=chosen, real=self.experts, rows=h, base=base)
