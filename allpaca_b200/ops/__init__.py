@@ -512,11 +512,15 @@ def _decode_attention(lib, q, out, cache_layer, block_table, positions, rows, nu
         pm = scratch("attn.part_ml", (nsplit, rows, num_heads, 2), torch.float32).data_ptr()
     if tma:
         # fed by TMA: a ring of tiles in flight, two CTAs per SM; 2, 4, 8 or 16 slices are combined
-        # inside a thread-block cluster and need no scratch
+        # inside a thread-block cluster and need no scratch.  More CTAs than fit at once, of sequences that differ in
+        # length: the longest first
+        chunks = -(-(num_heads // num_kv_heads) // min(num_heads // num_kv_heads, 16))
+        keys = min(max_context, window) if window else max_context
+        by_length = 1 if (rows * num_kv_heads * chunks * nsplit > slots and 0 < mean_context * 4 < keys * 3) else 0
         call(lib, "ap_attention_decode_tma", q.data_ptr(), out.data_ptr(), cache_layer.data_ptr(),
              cache_layer.shape[0], block_table.data_ptr(), block_table.shape[1], positions.data_ptr(), rows,
              num_heads, num_kv_heads, head_dim, P, cache_layer.stride(0), float(scale), int(window or 0),
-             nsplit, po, pm, stream_handle())
+             nsplit, po, pm, by_length, stream_handle())
         return
     call(lib, "ap_attention_tc", q.data_ptr(), out.data_ptr(), cache_layer.data_ptr(),
          block_table.data_ptr(), block_table.shape[1], 0, positions.data_ptr(),
