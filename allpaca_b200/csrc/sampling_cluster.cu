@@ -14,7 +14,8 @@
 //     A pass counts (or sums the weights exp(l - max) of) the logits above each of fifteen
 //     thresholds that divide the current interval evenly, the cluster adds the partial
 //     results through distributed shared memory, and the interval shrinks to the sixteenth
-//     that holds the cut.  Two or three passes leave at most 2048 candidates;
+//     that holds the cut.  Two or three passes leave at most 2048 candidates (with a top_k of up to 2048 the first passes look
+//     at the largest logit of each thread only, which mostly leaves no other pass to do);
 //   * the candidates go to the first CTA, which sorts them (by logit descending, token id
 //     ascending) and reads the cut off the sorted list;
 //   * with a top_k of up to 2048 the list holds every survivor: top_p and the draw are then
@@ -36,6 +37,7 @@ namespace cg = cooperative_groups;
 #define SC_CAP 2048            // candidates the first CTA sorts
 #define SC_WORDS 24            // 32-bit words a CTA publishes per exchange
 #define SC_MAX_PASSES 64
+#define SC_AHEAD_PASSES 6      // over the threads' largest logits
 #define SC_REACH 120.0f        // exp(-120) is zero in 32-bit: logits further below the maximum weigh nothing
 
 __device__ __forceinline__ unsigned sc_key(float f) {
@@ -209,7 +211,74 @@ __device__ ScCut sc_search(cg::cluster_group& cl, ScShared& sh, int& parity, con
     int n_list = 0;
     bool degenerate = false, found = true;
     float n_cand = 0.f, equal_value = 0.f;
-    for (int pass = 0; pass < SC_MAX_PASSES; ++pass) {
+    bool counted = false;                // at, n_list: as below, for everything above lo
+    int at = 0;
+    if (gather_above && !weighted && !c0.active && count <= (float)SC_CAP) {
+        // Few of many are wanted, and as many of the threads' largest logits lie above some logit as are wanted in all: the
+        // list may end there.  One logit a thread to a pass instead of E; what the list then holds beyond the wanted ones
+        // are those that share a thread with a larger one, and what the last slice holds.
+        float tm = -INFINITY;
+#pragma unroll
+        for (int e = 0; e < E; ++e) tm = fmaxf(tm, row.l[e]);
+        float p_lo = lo, p_hi = hi, over = 0.f;
+        bool enough = false;
+        for (int pass = 0; pass < SC_AHEAD_PASSES; ++pass) {
+            const float step = (p_hi - p_lo) * (1.f / (SC_PROBES + 1));
+            unsigned mine = 0;                               // lane j: what the warp has above threshold j; the last: above p_lo
+#pragma unroll
+            for (int j = 0; j <= SC_PROBES; ++j) {
+                const float t = j < SC_PROBES ? p_hi - step * (float)(j + 1) : p_lo;
+                const unsigned b = __ballot_sync(0xffffffffu, tm > t && tm <= p_hi);
+                if (lane == j) mine = __popc(b);
+            }
+            __syncthreads();
+            if (lane <= SC_PROBES) sh.wred[warp][lane] = mine;
+            __syncthreads();
+            if (threadIdx.x <= SC_PROBES) {
+                unsigned v = 0;
+                for (int w = 0; w < SC_WARPS; ++w) v += sh.wred[w][threadIdx.x];
+                sh.pub[parity][threadIdx.x] = v;
+            }
+            sc_exchange(cl, sh, parity);
+            if (threadIdx.x <= SC_PROBES) {
+                unsigned v = 0;
+                for (int r = 0; r < SC_CLUSTER; ++r) v += sh.all[r][threadIdx.x];
+                sh.sum[threadIdx.x] = (float)v;
+            }
+            __syncthreads();
+            if (over + sh.sum[SC_PROBES] < target) break;    // (in the first pass only)
+            enough = true;
+            int j = 0;
+            while (j < SC_PROBES && over + sh.sum[j] < target) ++j;
+            const float next_hi = j == 0 ? p_hi : p_hi - step * (float)j;
+            const float next_lo = j == SC_PROBES ? p_lo : p_hi - step * (float)(j + 1);
+            const float holds = over + sh.sum[j];            // sum[SC_PROBES]: all of the interval
+            if (j > 0) over += sh.sum[j - 1];
+            const bool divides = next_hi > next_lo && !(next_hi == p_hi && next_lo == p_lo);
+            p_lo = next_lo;
+            if (!divides || holds <= 2.f * target + 256.f) break;
+            p_hi = next_hi;
+        }
+        if (enough) {
+            lo = p_lo;
+            counted = true;
+            int mine = 0, block_total;
+#pragma unroll
+            for (int e = 0; e < E; ++e) mine += row.l[e] > lo ? 1 : 0;
+            at = sc_scan_int(mine, sh, &block_total);
+            if (threadIdx.x == 0) sh.pub[parity][0] = (unsigned)block_total;
+            sc_exchange(cl, sh, parity);
+            for (int r = 0; r < SC_CLUSTER; ++r) {
+                if (r < rank) at += (int)sh.all[r][0];
+                n_list += (int)sh.all[r][0];
+            }
+            if (n_list > SC_CAP) {                           // the passes below go on from here
+                counted = false;
+                n_list = 0;
+            }
+        }
+    }
+    for (int pass = 0; pass < SC_MAX_PASSES && !counted; ++pass) {
         const float step = (hi - lo) * (1.f / (SC_PROBES + 1));
         float acc[SC_PROBES];
 #pragma unroll
@@ -350,19 +419,21 @@ __device__ ScCut sc_search(cg::cluster_group& cl, ScShared& sh, int& parity, con
         return cut;
     }
     // the candidates (with gather_above: everything above lo) into the first CTA's list
-    int mine = 0;
+    if (!counted) {
+        int mine = 0;
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const float x = row.l[e];
-        mine += (x > lo && (gather_above || x <= hi) && sc_passes(c0, sc_key(x), row.id0 + e)) ? 1 : 0;
-    }
-    int block_total;
-    int at = sc_scan_int(mine, sh, &block_total);
-    if (threadIdx.x == 0) sh.pub[parity][0] = (unsigned)block_total;
-    sc_exchange(cl, sh, parity);
-    for (int r = 0; r < SC_CLUSTER; ++r) {
-        if (r < rank) at += (int)sh.all[r][0];
-        n_list += (int)sh.all[r][0];
+        for (int e = 0; e < E; ++e) {
+            const float x = row.l[e];
+            mine += (x > lo && (gather_above || x <= hi) && sc_passes(c0, sc_key(x), row.id0 + e)) ? 1 : 0;
+        }
+        int block_total;
+        at = sc_scan_int(mine, sh, &block_total);
+        if (threadIdx.x == 0) sh.pub[parity][0] = (unsigned)block_total;
+        sc_exchange(cl, sh, parity);
+        for (int r = 0; r < SC_CLUSTER; ++r) {
+            if (r < rank) at += (int)sh.all[r][0];
+            n_list += (int)sh.all[r][0];
+        }
     }
     unsigned long long* first_list = cl.map_shared_rank(&sh.list[0], 0);
 #pragma unroll
@@ -414,8 +485,9 @@ __device__ ScCut sc_search(cg::cluster_group& cl, ScShared& sh, int& parity, con
 
 // PER_SM 2: two CTAs to an SM, for more rows than find room for their clusters at one (some 14: a cluster stays within a GPC); a
 // row is a chain of cluster barriers, and two rows hide each other's, though the registers are then tight.  Measured (one B200, top-k 40,
-// top-p 0.95, us, one and two to an SM): 8 rows of 32000 logits 32 and 35, 16 rows 49 and 35, 32 rows 69 and 37; of 128256 logits 8 rows 45
-// and 60, 16 rows 78 and 63, 24 rows 79 and 63, 64 rows 161 and 113.
+// top-p 0.95, us, one and two to an SM, with passes over all logits): 8 rows of 32000 logits 32 and 35, 16 rows 49 and 35, 32 rows 69
+// and 37; of 128256 logits 8 rows 45 and 60, 16 rows 78 and 63, 24 rows 79 and 63, 64 rows 161 and 113.  With the threads' largest
+// logits first: 8 rows 29, 16 rows 29, 64 rows 49; of 128256 logits 8 rows 38, 16 rows 46, 24 rows 45, 64 rows 81.
 template <int E, int PER_SM>
 __global__ void __launch_bounds__(SC_THREADS, PER_SM)
 sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, int V,
