@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(128) la_scan_kernel(const LaScanArgs A) {
 }
 
 // ---- one row per sequence, many states ----------------------------------------------------------
-// A step of single rows that has a state for every SM and more (decoding many requests): what bounds it is reading and
+// A step of single rows that has about a state for every SM and more (decoding many requests): what bounds it is reading and
 // writing the states.  One CTA per (sequence, head) asks for the whole state at once, 16 bytes to a copy, and keeps it in
 // shared memory, where the lanes lie across a row's columns and the warps across the rows; the new state goes straight
 // back, a row's columns side by side.  The sums over the rows are formed per warp and added in the order of the warps.
@@ -1035,11 +1035,12 @@ AP_EXPORT int ap_linear_scan(float* q, long long ld_q, float* k, long long ld_k,
         AP_CHECK_PDL_LAUNCH("linear_scan (rows made ready)",
                             ap_launch_pdl(la_prepare_kernel, dim3((unsigned)blocks), dim3(128), 0, stream, A));
     }
-    // Single rows with two states or more to an SM, states in whole 16-byte runs that fit three to an SM: see la_step_kernel.
-    // Fewer states leave SMs idle there, where la_scan_kernel cuts a state into blocks of columns.
+    // Single rows with about a state and more to an SM, states in whole 16-byte runs that fit three to an SM: see la_step_kernel.
+    // Fewer leave SMs idle there, where la_scan_kernel cuts a state into blocks of columns (heads of 128 x 128, cold, us, la_scan_kernel
+    // and la_step_kernel: 64 states 5.2 and 5.5, 128 8.7 and 7.5, 192 12.4 and 8.4, 256 15.8 and 9.6).
     const int J = V <= 128 ? 4 : V <= 160 ? 5 : 8;
     const size_t step_smem = ((size_t)D * V + 3 * D + (LS_WARPS + 1) * 32 * J) * sizeof(float);
-    if (T == nseq && (long long)nseq * heads >= 2 * 148 && V >= 64 && V <= 256 && (D * V) % 4 == 0 &&
+    if (T == nseq && (long long)nseq * heads >= 128 && V >= 64 && V <= 256 && (D * V) % 4 == 0 &&
         step_smem <= 74 * 1024 && aligned(state, state_stride)) {
         void (*step)(const LaScanArgs) = J == 4 ? la_step_kernel<4> : J == 5 ? la_step_kernel<5> : la_step_kernel<8>;
         cudaError_t e = cudaFuncSetAttribute(step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem);

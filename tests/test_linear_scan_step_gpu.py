@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("kind", ["head", "channel_delta", "gated_unit"])
 @pytest.mark.parametrize("seqs,heads,D,V,lens", [
-    (37, 8, 128, 128, None), (36, 8, 128, 128, None), (40, 16, 64, 65, None), (40, 8, 100, 161, None), (300, 1, 36, 256, None),
+    (16, 8, 128, 128, None), (15, 8, 128, 128, None), (40, 16, 64, 65, None), (40, 8, 100, 161, None), (300, 1, 36, 256, None),
     (40, 8, 128, 129, (0, 2)),                               # as many rows as sequences, yet not one to each
 ])
 def test_many_single_rows(kind, seqs, heads, D, V, lens):
