@@ -9,6 +9,11 @@
 // One block per row, the row kept in shared memory between the two passes.
 #include "common.cuh"
 
+#define EMBED_THREADS 256
+
+// The sum under the norm has one order for every number of rows, so that a row has the same bits in any step: it is formed as by
+// 256 threads, a pair of entries (an entry, where there are no positions) after another to each.  A CTA of 1024 leaves it to its
+// first 256, which take the row from shared memory.
 template <typename TW, typename TN>
 __global__ void __launch_bounds__(1024)
 embed_sinusoid_norm_kernel(const int* __restrict__ tokens, const int* __restrict__ positions,
@@ -41,6 +46,22 @@ embed_sinusoid_norm_kernel(const int* __restrict__ tokens, const int* __restrict
             ss = fmaf(v, v, ss);
         }
     }
+    if (blockDim.x > EMBED_THREADS && norm_w != nullptr) {
+        __syncthreads();
+        ss = 0.f;
+        if (threadIdx.x < EMBED_THREADS) {
+            if (inv_freq != nullptr) {
+#pragma unroll 4
+                for (int p = threadIdx.x; p < H / 2; p += EMBED_THREADS) {
+                    const float2 v = *reinterpret_cast<const float2*>(row_buf + 2 * p);
+                    ss = fmaf(v.y, v.y, fmaf(v.x, v.x, ss));
+                }
+            } else {
+#pragma unroll 4
+                for (int i = threadIdx.x; i < H; i += EMBED_THREADS) ss = fmaf(row_buf[i], row_buf[i], ss);
+            }
+        }
+    }
     float inv = 1.f;
     if (norm_w != nullptr) {
         ss = ap_block_sum(ss, red);
@@ -62,8 +83,11 @@ AP_EXPORT int ap_embed_sinusoid_norm(const int* tokens, const int* positions, co
     AP_REQUIRE((size_t)H * 4 <= 200 * 1024, "embed_sinusoid_norm: width %d does not fit the row buffer", H);
     if (T == 0) return AP_OK;
     const size_t smem = (size_t)H * sizeof(float);
-    // few rows: a pair of entries to a thread (8 rows of 2048 4.8 us; 256 threads with two angles to a pair 8.9 to 10.9)
-    const int threads = T <= 148 && H >= 1024 ? 1024 : 256;
+    // A CTA of 1024, with a pair of entries to a thread, for up to a row to an SM; beyond, such CTAs wait for one another.  With 1024
+    // threads and with 256, us: 1024 entries, 149 rows 3.5 and 3.5, 300 rows 4.9 and 3.7; 2048 entries, 149 rows 4.1 and 5.1, 300 rows
+    // 5.7 and 5.2, 2048 rows 21 and 11; 4096 entries, 149 rows 5.0 and 8.1, 512 rows 9.0 and 8.5.  (8 rows of 2048 3.5; with two angles
+    // to a pair 5.1.)
+    const int threads = T <= 148 && H >= 1024 ? 1024 : EMBED_THREADS;
     // The first kernel of a step is launched in plain stream order (see ap_embed_gather).
 #define LAUNCH(TW, TN)                                                                                       \
     do {                                                                                                     \

@@ -45,6 +45,22 @@ def test_embedding_with_position_vector_and_norm(table_dtype):
     close(x, want, 3e-3, "embedding at far positions")
 
 
+@pytest.mark.parametrize("W", [1000, 1024, 2048, 4100])
+def test_an_embedded_row_has_the_same_bits_in_any_step(W):
+    """The sum under the norm is formed in one order, whatever the number of rows: alone, and in steps of 148 and 149."""
+    from allpaca_b200 import ops
+    g = torch.Generator().manual_seed(W)
+    table, gain = torch.randn(60, W, generator=g).to(DEV), (1.0 + 0.1 * torch.randn(W, generator=g)).to(DEV)
+    tokens = torch.randint(0, 60, (149,), generator=g).to(torch.int32).to(DEV)
+    positions = torch.randint(0, 4000, (149,), generator=g).to(torch.int32).to(DEV)
+    inv_freq = torch.pow(torch.tensor(10000.0, dtype=torch.float64), -2.0 * torch.arange(W // 2) / W).float().to(DEV)
+    got = {}
+    for rows in (1, 148, 149):
+        x = got[rows] = torch.empty(rows, W, device=DEV)
+        ops.embed_sinusoid_norm(tokens[:rows], positions[:rows], table, inv_freq, gain, 1e-5, x)
+    assert torch.equal(got[148], got[149][:148]) and torch.equal(got[1], got[149][:1])
+
+
 def paged(kv, P, order):
     """kv [T, G, D+E] of one sequence -> (pages [n, G, P, D+E], block-table row) with the
     sequence's pages at the places ``order`` names."""
