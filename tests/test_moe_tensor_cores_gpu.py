@@ -49,3 +49,23 @@ def test_products_of_all_experts(counts, gated, name, N, K):
         # a sum of K products of unit size is off by about K^0.5 units of 2^-24 of its terms; bfloat16 stores seven bits
         tol = 2e-5 + (0.0 if name is None else 2.0 ** -8 * want.abs())
         assert bool(((got[rows] - want).abs() <= tol).all()), (e, float((got[rows] - want).abs().max()))
+
+
+@pytest.mark.parametrize("rows", [1, 40, 300])
+@pytest.mark.parametrize("name", ["silu", "clamped_sigmoid"])
+def test_gates_far_below_zero_keep_their_small_results(name, rows):
+    """1 + exp(88) is a 32-bit number, so a gate of -88 is no zero: times a large second factor it shows."""
+    from allpaca_b200 import ops
+    N, K = 64, 64
+    gates = torch.tensor([-87.0, -87.5, -88.0, -88.5, -80.0, -40.0, -5.0, 3.0]).repeat(N // 8)
+    a, w = torch.zeros(rows, K), torch.zeros(1, 2 * N, K)
+    a[:, 0] = 1.0
+    w[0, :N, 0], w[0, N:, 0] = gates, 2.0 ** 100
+    out = torch.empty(rows, N, dtype=torch.bfloat16, device=DEV)
+    ops.moe_products(a.to(torch.bfloat16).to(DEV), w.to(torch.bfloat16).to(DEV), out,
+                     torch.tensor([0, rows], dtype=torch.int32, device=DEV), gated=True, activation=name, limit=2.0 ** 101, alpha=1.0)
+    ops.check_kernel_status()
+    z = gates.double()
+    want = (z / (1.0 + torch.exp(-z)) * 2.0 ** 100).expand(rows, N)
+    # the exponential is off by some units of 2^-24, bfloat16 stores seven bits
+    assert bool(((out.double().cpu() - want).abs() <= (2.0 ** -8 + 1e-5) * want.abs()).all()), (out[0, :8].cpu(), want[0, :8])
