@@ -691,8 +691,8 @@ AP_EXPORT int ap_moe_gate_up(const void* a, int a_dtype, const void* w, int w_dt
                              void* x_y, int x_rows, int x_N, int x_K, cudaStream_t stream) {
     AP_REQUIRE(pairs >= 0 && E > 0 && F > 0 && K > 0 && top > 0 && act >= 0 && act <= ACT_RELU2, "moe_gate_up: bad sizes");
     AP_REQUIRE(gated || act != ACT_CLAMPED, "moe_gate_up: activation %d needs a gate", act);
-    if (pairs == 0) return AP_OK;
-    const int max_tiles = ap_moe_max_tiles(pairs, E);
+    if (pairs == 0 && x_rows == 0) return AP_OK;
+    const int max_tiles = pairs > 0 ? ap_moe_max_tiles(pairs, E) : 0;       // no pair: the shared expert alone
     const dim3 grid((unsigned)((F + MOE_BN - 1) / MOE_BN), (unsigned)max_tiles);
     AP_REQUIRE(max_tiles <= 65535, "moe_gate_up: %d row tiles exceed the grid", max_tiles);
     const long long expert_stride = (long long)(gated ? 2 : 1) * F * K;
@@ -733,8 +733,8 @@ AP_EXPORT int ap_moe_down(const void* y, int y_dtype, const void* w, int w_dtype
                           int E, int H, int F, const void* x_y, const void* x_w, float* x_o, int x_rows, int x_N, int x_K,
                           cudaStream_t stream) {
     AP_REQUIRE(pairs >= 0 && E > 0 && F > 0 && H > 0, "moe_down: bad sizes");
-    if (pairs == 0) return AP_OK;
-    const int max_tiles = ap_moe_max_tiles(pairs, E);
+    if (pairs == 0 && x_rows == 0) return AP_OK;
+    const int max_tiles = pairs > 0 ? ap_moe_max_tiles(pairs, E) : 0;       // no pair: the shared expert alone
     const dim3 grid((unsigned)((H + MOE_BN - 1) / MOE_BN), (unsigned)max_tiles);
     AP_REQUIRE(max_tiles <= 65535, "moe_down: %d row tiles exceed the grid", max_tiles);
 #define LAUNCH(TA, TW)                                                                                               \

@@ -207,7 +207,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant_
     }
     if (warp == 1) tc::tmem_alloc(tmem_slot, Cfg::kTmem);
     ap_pdl_wait();
-    for (int e = threadIdx.x; e <= g.experts; e += MT_THREADS) first[e] = g.first[e];
+    if (g.experts > 0)
+        for (int e = threadIdx.x; e <= g.experts; e += MT_THREADS) first[e] = g.first[e];
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -418,14 +419,15 @@ static int moe_launch(const void* a, const void* w, void* out, const MoeTcArgs& 
                       const void* x_w, void* x_out, cudaStream_t stream) {
     using Cfg = MoeTile<BN, SUB>;
     CUtensorMap tw, ta, txw, txa;
-    AP_REQUIRE(moe_map(&tw, w, (long long)args.experts * (GATED ? 2 : 1) * args.N, args.K, 64) &&
-                   moe_map(&ta, a, pairs, args.K, Cfg::kABox),
+    AP_REQUIRE(args.experts == 0 || (moe_map(&tw, w, (long long)args.experts * (GATED ? 2 : 1) * args.N, args.K, 64) &&
+                                     moe_map(&ta, a, pairs, args.K, Cfg::kABox)),
                "moe_tc: cannot encode the tensor maps");
-    txw = tw;
-    txa = ta;
     AP_REQUIRE(args.x_rows == 0 || (moe_map(&txw, x_w, (long long)(GATED ? 2 : 1) * args.x_N, args.x_K, 64) &&
                                     moe_map(&txa, x_a, args.x_rows, args.x_K, Cfg::kABox)),
                "moe_tc: cannot encode the shared expert's tensor maps");
+    // what is not there is not loaded from
+    if (args.experts == 0) { tw = txw; ta = txa; }
+    if (args.x_rows == 0) { txw = tw; txa = ta; }
     auto kern = moe_tc_kernel<BN, SUB, GATED, TO>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
     AP_REQUIRE(e == cudaSuccess, "moe_tc: cannot reserve %d bytes of shared memory: %s", Cfg::kSmem, cudaGetErrorString(e));
@@ -471,9 +473,10 @@ AP_EXPORT int ap_moe_tc(const void* a, const void* w, void* out, int out_dtype, 
     AP_REQUIRE((((uintptr_t)a | (uintptr_t)w) & 15) == 0, "moe_tc: operands must be 16-byte aligned");
     AP_REQUIRE(pair_scale == nullptr || perm != nullptr, "moe_tc: scales go by the permutation");
     AP_REQUIRE((long long)E * (gated ? 2 : 1) * N < 0x7fffffffLL, "moe_tc: too many weight rows");
-    if (pairs == 0) return AP_OK;
+    if (pairs == 0 && x_rows == 0) return AP_OK;
+    if (pairs == 0) E = 0;                     // the shared expert alone: first[] is not looked at
     const MoeTcArgs g{first, pair_scale, perm, E, 0, N, K, act, (long long)N, limit, alpha, shift, x_rows, 0, x_N, x_K};
-    const int mean = (pairs + E - 1) / E;
+    const int mean = E > 0 ? (pairs + E - 1) / E : x_rows;
 #define LAUNCH(BN, SUB)                                                                                                \
     do {                                                                                                               \
         if (gated && out_dtype == AP_BF16) return moe_launch<BN, SUB, true, bf16>(a, w, out, g, pairs, x_a, x_w, x_out, stream);        \

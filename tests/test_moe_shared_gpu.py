@@ -73,3 +73,28 @@ def test_beside_the_products_of_few_rows(T, top, E, gated, name, F, K, XF):
         e = int(chosen.view(-1)[pair])
         near(y[p:p + 1], act(name, h[pair // top][None].double() @ w[e].double().T, gated), True)
         near(o[p:p + 1], y[p:p + 1].double().cpu() @ down[e].double().T, False)
+
+
+@pytest.mark.parametrize("T", [1, 70])
+@pytest.mark.parametrize("gated,name", [(True, "silu"), (False, "relu2")])
+def test_a_shared_expert_without_any_pair(T, gated, name):
+    """No row goes to a routed expert: the shared one's results are there all the same, in each of the three calls."""
+    from allpaca_b200 import ops
+    g = torch.Generator().manual_seed(T)
+    E, N, K, XN, XK = 3, 40, 64, 72, 128
+    xa, xw, xdown = torch.randn(T, XK, generator=g).to(torch.bfloat16), matrix(g, 2 * XN if gated else XN, XK), matrix(g, 48, XN)
+    w, down = matrix(g, E, 2 * N if gated else N, K).to(DEV), matrix(g, E, N, K).to(DEV)
+    a, none = torch.empty(0, K, dtype=torch.bfloat16, device=DEV), torch.empty(0, dtype=torch.int32, device=DEV)
+    y = torch.empty(0, N, dtype=torch.bfloat16, device=DEV)
+    first = torch.full((E + 1,), 5, dtype=torch.int32, device=DEV)          # not looked at
+    tiles = torch.full((ops.moe_max_tiles(0, E) + 1, 3), 5, dtype=torch.int32, device=DEV)
+    want = act(name, xa.double() @ xw.double().T, gated)
+    outs = [torch.zeros(T, XN, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    ops.moe_products(a, w, y, first, gated=gated, activation=name, shared=(xa.to(DEV), xw.to(DEV), outs[0]))
+    ops.moe_gate_up(a, w, y, none, 1, tiles, name, gated=gated, shared=(xa.to(DEV), xw.to(DEV), outs[1]))
+    sums = torch.zeros(T, 48, device=DEV)
+    ops.moe_down(a, down, torch.empty(0, N, device=DEV), tiles, shared=(outs[1], xdown.to(DEV), sums))
+    ops.check_kernel_status()
+    for out in outs:
+        near(out, want, True)
+    near(sums, outs[1].double().cpu() @ xdown.double().T, False)
