@@ -206,6 +206,15 @@ class ModelRunner:
         G = len(self.cache.groups)
         T = sum(len(en.tokens) for en in entries)
         R = sum(len(en.want) for en in entries)
+        indexed = device_tokens is not None and any(en.device_row is not None for en in entries)
+        if device_tokens is not None:
+            if device_tokens.dtype != torch.int32 or not device_tokens.is_cuda or \
+                    (not indexed and device_tokens.numel() < T):
+                raise ValueError("device_tokens must be int32 on the device, one per row of the step")
+            device_tokens = device_tokens.reshape(-1).contiguous()
+            for en in entries if indexed else ():
+                if en.device_row is not None and (len(en.tokens) != 1 or not 0 <= en.device_row < device_tokens.numel()):
+                    raise ValueError(f"device_row {en.device_row} is not a token on the device for a single row")
         widest = -(-self.max_model_len // min(g.page_size for g in self.cache.groups)) if G else 0
         total_cap = 4 * T + 3 * nseq + 1 + R + nseq * widest * G
         if staging is None:
@@ -220,19 +229,11 @@ class ModelRunner:
             built.query_lens, built.seq_start
         total = int(layout.total)
         off = int(layout.off_tokens)
-        indexed = device_tokens is not None and any(en.device_row is not None for en in entries)
-        if device_tokens is not None:
-            if device_tokens.dtype != torch.int32 or not device_tokens.is_cuda or \
-                    (not indexed and device_tokens.numel() < T):
-                raise ValueError("device_tokens must be int32 on the device, one per row of the step")
-            device_tokens = device_tokens.reshape(-1).contiguous()
         if indexed:
             index = host[total:total + T]                  # the block has room for them behind the step's numbers
             index[:] = -1
             for en, at in zip(entries, tok_off):
                 if en.device_row is not None:
-                    if len(en.tokens) != 1 or not 0 <= en.device_row < device_tokens.numel():
-                        raise ValueError(f"device_row {en.device_row} is not a token on the device for a single row")
                     index[at] = en.device_row
         if total <= self.STAGE_BY_KERNEL:
             ops.stage_step(host_tensor, dev, 0, total, device_tokens, off, T, total if indexed else -1)

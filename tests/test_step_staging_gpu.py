@@ -90,3 +90,32 @@ def test_decoding_beside_portions_takes_tokens_from_the_device(tmp_path, budget,
             pass
         assert llm.runner.cache.num_running() == 0
         llm.runner.cache.check()
+
+
+def test_a_refused_step_changes_nothing(tmp_path):
+    """A place among the device's tokens that is not there, or one for several rows, or too few tokens: refused before pages are
+    taken and before a request has advanced, so that the same step without the fault gives what it would have given."""
+    from allpaca_b200.config import EngineConfig
+    from allpaca_b200.config.presets import preset_config
+    from allpaca_b200.engine.batch import BatchEntry
+    from allpaca_b200.engine.runner import ModelRunner
+    from allpaca_b200.weights.random_model import write_random_model
+    write_random_model(str(tmp_path), preset_config("tiny-a"), seed=0, dtype="float32", norm_std=0.02)
+    runner = ModelRunner(str(tmp_path), EngineConfig(dtype="float32", page_size=8, num_pages=32, max_num_seqs=4,
+                                                     max_num_batched_tokens=64))
+    prompt, tokens = list(range(3, 19)), torch.tensor([5, 9], dtype=torch.int32, device=DEV)
+    runner.step([BatchEntry("a", prompt, [])])
+    want = runner.step([BatchEntry("b", prompt, []), BatchEntry("a", [9], [0])]).clone()
+    runner.finish("a"), runner.finish("b")
+    runner.step([BatchEntry("a", prompt, [])])
+    state = lambda: (runner.cache.num_tokens("a"), runner.cache.has("b"), runner.cache.num_running(), runner.cache.num_free_pages(0))
+    before = state()
+    for wrong in (BatchEntry("a", [0], [0], 2), BatchEntry("a", [0], [0], -1), BatchEntry("a", [0, 0], [1], 1)):
+        with pytest.raises(ValueError):
+            runner.step([BatchEntry("b", prompt, []), wrong], device_tokens=tokens)
+        assert state() == before
+    for bad in (tokens[:1], tokens.long(), tokens.cpu()):
+        with pytest.raises(ValueError):
+            runner.step([BatchEntry("b", prompt, []), BatchEntry("a", [0], [0])], device_tokens=bad)
+        assert state() == before
+    assert torch.equal(runner.step([BatchEntry("b", prompt, []), BatchEntry("a", [0], [0], 1)], device_tokens=tokens), want)
