@@ -63,6 +63,11 @@ class ModelRunner:
         self._host_control = model.host_control()
         self.graph_replays = 0
 
+    def __del__(self):
+        copied = getattr(self, "_copied", None)
+        if copied is not None:
+            copied.synchronize()                         # a kernel in flight reads the pinned block
+
     # ---- caches ---------------------------------------------------------
     def _setup_caches(self) -> None:
         e = self.engine
@@ -305,3 +310,8 @@ class _DecodeGraph:
         self.generation = -1
         self.num_kernels = 0
         self.uses = 0                 # steps of this size so far that found no valid graph
+
+    def __del__(self):
+        copied = getattr(self, "copied", None)
+        if copied is not None:
+            copied.synchronize()                         # as in ModelRunner

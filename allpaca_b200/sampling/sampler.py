@@ -38,6 +38,10 @@ class Sampler:
         self._events = [torch.cuda.Event() for _ in range(2)]
         self._turn = 0
 
+    def __del__(self):
+        for event in getattr(self, "_events", ()):       # a kernel in flight reads the options and writes the host's tokens
+            event.synchronize()
+
     def launch(self, logits: torch.Tensor, params: Sequence[SamplingParams],
                uniforms: Sequence[float]) -> Pending:
         """Choose one token per row of ``logits [R, V]`` on the GPU, for the device and the host;

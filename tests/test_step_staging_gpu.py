@@ -119,3 +119,14 @@ def test_a_refused_step_changes_nothing(tmp_path):
             runner.step([BatchEntry("b", prompt, []), BatchEntry("a", [0], [0])], device_tokens=bad)
         assert state() == before
     assert torch.equal(runner.step([BatchEntry("b", prompt, []), BatchEntry("a", [0], [0], 1)], device_tokens=tokens), want)
+
+
+def test_a_sampler_goes_away_after_its_launches():
+    from allpaca_b200.sampling import SamplingParams
+    from allpaca_b200.sampling.sampler import Sampler
+    sampler, logits = Sampler(torch.device(DEV), 4), torch.randn(4, 300, device=DEV)
+    torch.cuda._sleep(100_000_000)                       # some 50 ms
+    done = sampler.launch(logits, [SamplingParams(max_tokens=1, seed=i) for i in range(4)], [0.1, 0.4, 0.6, 0.9]).event
+    assert not done.query()
+    del sampler
+    assert done.query()
