@@ -212,15 +212,21 @@ __device__ __forceinline__ void hm_mma(float (&c)[4], uint32_t a0, uint32_t a1, 
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ uint32_t hm_word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
-// four numbers as pairs of bfloat16: the terms they are the sum of
+// four numbers as pairs of bfloat16: the terms they are the sum of.  All terms but the last are kept within bfloat16's range, so
+// that numbers beyond it (up to 2^128 in 32 bits) count as what they are, and infinities and NaN, which the last term takes over, as well
 template <int TERMS> __device__ __forceinline__ void hm_split(float4 v, uint32_t (&lo)[TERMS], uint32_t (&hi)[TERMS]) {
+    constexpr float most = 0x1.fep127f;
+    auto in = [](float x) { return fminf(fmaxf(x, -most), most); };
 #pragma unroll
     for (int i = 0; i < TERMS; ++i) {
-        const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+        const float4 t = i + 1 < TERMS ? make_float4(in(v.x), in(v.y), in(v.z), in(v.w)) : v;
+        const __nv_bfloat162 a = __floats2bfloat162_rn(t.x, t.y), b = __floats2bfloat162_rn(t.z, t.w);
         lo[i] = *reinterpret_cast<const uint32_t*>(&a);
         hi[i] = *reinterpret_cast<const uint32_t*>(&b);
-        const float2 fa = __bfloat1622float2(a), fb = __bfloat1622float2(b);
-        v.x -= fa.x; v.y -= fa.y; v.z -= fb.x; v.w -= fb.y;
+        if (i + 1 < TERMS) {
+            const float2 fa = __bfloat1622float2(a), fb = __bfloat1622float2(b);
+            v.x -= fa.x; v.y -= fa.y; v.z -= fb.x; v.w -= fb.y;
+        }
     }
 }
 

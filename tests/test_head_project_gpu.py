@@ -52,3 +52,20 @@ def test_rotation_alone(out_dtype, T, H, K, tail, dims):
     ops.head_project(x.to(DEV), None, out, H, tail=tail, tail_dims=dims, cos_sin=cs.to(DEV) if dims else None)
     tol = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -23
     assert bool(((out.double().cpu().view(T, H, -1) - want).abs() <= tol * want.abs() + 1e-6).all())
+
+
+@pytest.mark.parametrize("K", [16, 272])
+def test_inputs_that_bfloat16_does_not_hold(K):
+    """32-bit inputs beyond the largest bfloat16 number count as what they are, infinite ones stay infinite, NaN stays NaN, and
+    each only in its own row."""
+    from allpaca_b200 import ops
+    most, inf, nan = torch.finfo(torch.float32).max, float("inf"), float("nan")
+    special = [most, -most, inf, -inf, nan, 1.0, 2.0 ** -140]
+    x = torch.zeros(len(special), K)
+    x[:, K - 3] = torch.tensor(special)
+    x[:, 1] = torch.tensor([0.0, 0.0, 1.0, 1.0, 1.0, 1.0, 0.0])
+    w = torch.full((1, K, 8), 0.0625).to(torch.bfloat16)
+    out = torch.empty(len(special), 8, dtype=torch.bfloat16, device=DEV)
+    ops.head_project(x.to(DEV), w.to(DEV), out, 1)
+    want = (x.double().sum(1) * 0.0625).to(torch.bfloat16)[:, None].expand(-1, 8)
+    assert torch.equal(torch.nan_to_num(out.cpu(), nan=7.0), torch.nan_to_num(want, nan=7.0)), (out[:, 0], want[:, 0])
