@@ -150,7 +150,7 @@ def bench_attention(args) -> dict:
         cache, table = caches[i % copies]
         ops.attention(q, out, cache, table, seq, pos, nh, nkv, hd, 1.0 / math.sqrt(hd), 0, seq_start=start,
                       query_lens=[1] * B, max_context=C, scratch=scratch, use_tma=not args.cp_async,
-                      mean_context=0 if args.plan_by_longest else mean)
+                      mean_context=0 if args.plan_by_longest else mean, settled=True)
     us = _time(fn, args.iters, args.warmup, not args.no_graph)
     return {"kernel": "attention_split+merge" if args.cp_async else "attention_split_tma+merge", "batch": B, "context": C, "heads": nh, "kv_heads": nkv,
             "head_dim": hd, "mean_context": mean,
@@ -203,7 +203,7 @@ def bench_latent_decode(args) -> dict:
 
     def fn(i):
         ops.latent_decode(q, out, caches[i % copies], table, start, pos, B, nh, D, R, 1.0 / math.sqrt(D), gate, C, ws,
-                          window=args.window, sink=sink)
+                          window=args.window, sink=sink, settled=True)
     us = _time(fn, args.iters, args.warmup, not args.no_graph)
     seen = min(C, args.window) if args.window > 0 else C              # keys a row reads
     per = B * seen * D * 2
@@ -357,7 +357,7 @@ def bench_versus_reference(args) -> dict:
         qq = torch.randn(M, NH * HD, device="cuda").to(dtype)
         oo = torch.empty_like(qq)
         return lambda i: ops.attention(qq, oo, cache, tbl, seq, last, NH, NKV, HD, HD ** -0.5, 0, seq_start=start,
-                                       query_lens=[1] * M, max_context=KEYS, scratch=scratch)
+                                       query_lens=[1] * M, max_context=KEYS, scratch=scratch, settled=True)
     rows.append((f"decode attention, {M} sequences x {KEYS} keys", timed(their_decode),
                  timed(our_decode(torch.float32)), timed(our_decode(torch.bfloat16))))
     # prompt attention of 512 tokens

@@ -234,7 +234,7 @@ template <typename TI>
 __global__ void __launch_bounds__(HM_WARPS * 32)
 head_project_mma_kernel(const TI* __restrict__ in, long long in_ld, int in_hs, const bf16* __restrict__ w, bf16* __restrict__ out,
                         long long out_ld, int out_hs, int T, int K, int N, int tail, int half, const float2* __restrict__ cos_sin,
-                        const int* __restrict__ seq_start, int nseq) {
+                        const int* __restrict__ seq_start, int nseq, int settled) {
     constexpr int TERMS = sizeof(TI) == 4 ? 3 : 1;
     __shared__ __align__(16) float part[HM_WARPS][HM_ROWS][HM_COLS];
     __shared__ int row_s[HM_ROWS];
@@ -249,6 +249,7 @@ head_project_mma_kernel(const TI* __restrict__ in, long long in_ld, int in_hs, c
             wv[j] = n0 + 8 * g < N ? *reinterpret_cast<const uint4*>(src + (size_t)j * N) : make_uint4(0, 0, 0, 0);
     };
     if (warp < steps) load_w(warp);
+    if (!settled) ap_pdl_wait();
     if (threadIdx.x < HM_ROWS) {
         const int i = blockIdx.x * HM_ROWS + threadIdx.x;
         int r = -1;
@@ -358,10 +359,11 @@ head_copy_kernel(const float* __restrict__ in, long long in_ld, int in_hs, TO* _
     }
 }
 
-// seq_start (or null): only the rows of the sequences that bring one row are needed, and others may be left as they are
+// seq_start (or null): only the rows of the sequences that bring one row are needed, and others may be left as they are; it is
+// read ahead of the kernels before this one where it is `settled` (common.cuh)
 AP_EXPORT int ap_head_project(const void* in, int in_dtype, long long in_ld, int in_hs, const void* w, int w_dtype,
                               void* out, int out_dtype, long long out_ld, int out_hs, int T, int H, int K, int N,
-                              int tail, int tail_dims, const float* cos_sin, const int* seq_start, int nseq, cudaStream_t stream) {
+                              int tail, int tail_dims, const float* cos_sin, const int* seq_start, int nseq, int settled, cudaStream_t stream) {
     AP_REQUIRE(T >= 0 && H > 0 && K > 0 && N > 0 && tail >= 0, "head_project: bad sizes T=%d H=%d K=%d N=%d", T, H, K, N);
     AP_REQUIRE(w != nullptr || N == K, "head_project: without a matrix the numbers are copied, N must equal K");
     AP_REQUIRE(H <= 65535, "head_project: %d heads exceed the grid", H);
@@ -382,7 +384,7 @@ AP_EXPORT int ap_head_project(const void* in, int in_dtype, long long in_ld, int
     AP_CHECK_PDL_LAUNCH("head_project", ap_launch_pdl(head_project_mma_kernel<TI>, grid, dim3(HM_WARPS * 32), 0, stream, \
                                                       (const TI*)in, in_ld, in_hs, (const bf16*)w, (bf16*)out, out_ld, \
                                                       out_hs, T, K, N, tail, tail_dims / 2, (const float2*)cos_sin,    \
-                                                      seq_start, nseq))
+                                                      seq_start, nseq, settled || seq_start == nullptr))
         if (in_dtype == AP_F32) LAUNCH_M(float);
         else LAUNCH_M(bf16);
 #undef LAUNCH_M

@@ -68,11 +68,12 @@ latent_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ cache,
                      int max_blocks, const int* __restrict__ seq_start, const int* __restrict__ positions, int nh, int D,
                      int R, int P, size_t page_stride, float scale, int window, int nsplit, float* __restrict__ part_o,
                      float* __restrict__ part_ml, bf16* __restrict__ out, const float* __restrict__ gate, long long gate_ld,
-                     const float* __restrict__ sink) {
+                     const float* __restrict__ sink, int settled) {
     extern __shared__ __align__(16) unsigned char ld_smem[];
     const int seq = blockIdx.x, h0 = blockIdx.y * LD_M, split = blockIdx.z;
     ap_pdl_trigger();
-    // the step's metadata and, but for the newest token, its pages are older than any kernel of the step
+    // where the caller says so, the step's metadata and, but for the newest token, its pages are older than the kernel ahead
+    if (!settled) ap_pdl_wait();
     const int row = seq_start[seq];
     if (seq_start[seq + 1] - row != 1) {
         ap_pdl_wait();
@@ -404,7 +405,7 @@ AP_EXPORT int ap_latent_decode(const void* q, void* out, const void* cache, cons
                                const int* seq_start, const int* positions, int nseq, int nh, int D, int R, int P,
                                long long page_stride, float scale, const float* gate, long long gate_ld, int nsplit,
                                float* scratch, long long scratch_floats, int window, const float* sink,
-                               cudaStream_t stream) {
+                               int settled, cudaStream_t stream) {
     AP_REQUIRE(nseq >= 0 && nh > 0 && P > 0 && max_blocks > 0 && nsplit >= 1 && nsplit <= LD_MAX_SPLITS,
                "latent_decode: bad sizes (at most %d key slices)", LD_MAX_SPLITS);
     AP_REQUIRE(ap_latent_decode_takes(D, R), "latent_decode: a record of %d with a value of %d is not one the kernel takes", D, R);
@@ -451,7 +452,7 @@ AP_EXPORT int ap_latent_decode(const void* q, void* out, const void* cache, cons
     AP_CHECK_PDL_LAUNCH("latent_decode",
                         cudaLaunchKernelEx(&cfg, kern, (const bf16*)q, (const bf16*)cache, block_table, max_blocks, seq_start,
                                            positions, nh, D, R, P, (size_t)page_stride, scale, window, nsplit, part_o, part_ml,
-                                           (bf16*)out, gate, gate_ld, sink));
+                                           (bf16*)out, gate, gate_ld, sink, settled));
     if (merge) return AP_OK;
     AP_CHECK_PDL_LAUNCH("latent_decode_merge",
                         ap_launch_pdl(latent_decode_merge_kernel, dim3((unsigned)nseq, (unsigned)nh), dim3(128), 0, stream,

@@ -53,6 +53,7 @@ struct AttnTcParams {
     int max_blocks, nseq, T, nh, nkv, P, window;
     int tokens_per_tile, heads_per_chunk, n_chunks, nsplit;
     float scale_log2;    // softmax scale * log2(e)
+    int settled;         // TMA-fed decode kernel: the metadata and all keys but the newest are older than the kernel ahead
     int by_length;       // TMA-fed decode kernel: the longest sequences' CTAs first (at most 64 sequences)
 };
 
@@ -648,11 +649,12 @@ attention_split_tma_kernel(const __grid_constant__ CUtensorMap tmap_kv, const __
     tc::fence_proxy_async();
     __syncthreads();
     ap_pdl_trigger();
-    // The step's positions and block tables were uploaded before any kernel of the step ran,
-    // and of the cache only the newest key of each row is written by the kernel before this
-    // one: the producer starts loading older keys at once and waits for the kernels before
+    // Where the caller says so, the step's positions and block tables were uploaded before any kernel
+    // of the step ran, and of the cache only the newest key of each row is written by the kernel before
+    // this one: the producer starts loading older keys at once and waits for the kernels before
     // this one only where it comes to the tile that holds the newest key; the consumers wait
     // before they read the queries.
+    if (!p.settled) ap_pdl_wait();
 
     // Row == sequence index.  Where the CTAs are more than fit at once and the sequences differ in length, the
     // CTAs (which start in the order of their index) take all heads of the longest sequence first: a long one
@@ -932,7 +934,8 @@ AP_EXPORT int ap_attention_decode_tma_in_cluster(int nh, int nkv, int nsplit) {
 AP_EXPORT int ap_attention_decode_tma(const void* q, void* out, const void* cache, long long num_pages,
                                       const int* block_table, int max_blocks, const int* positions, int T,
                                       int nh, int nkv, int hd, int P, long long page_stride, float scale,
-                                      int window, int nsplit, float* part_o, float* part_ml, int by_length, cudaStream_t stream) {
+                                      int window, int nsplit, float* part_o, float* part_ml, int settled, int by_length,
+                                      cudaStream_t stream) {
     AP_REQUIRE(ap_attention_decode_tma_supports(nh, nkv, hd, P), "attention (decode, TMA): shape not supported: "
                "heads=%d kv_heads=%d head_dim=%d page=%d", nh, nkv, hd, P);
     AP_REQUIRE(page_stride == 2LL * nkv * P * HD, "attention (decode, TMA): pages must be contiguous");
@@ -985,6 +988,7 @@ AP_EXPORT int ap_attention_decode_tma(const void* q, void* out, const void* cach
     p.n_chunks = (reps + p.heads_per_chunk - 1) / p.heads_per_chunk;
     p.tokens_per_tile = 1;
     p.nsplit = nsplit;
+    p.settled = settled;
     p.by_length = by_length && T <= 64 ? 1 : 0;
     AP_REQUIRE(nkv * p.n_chunks <= 65535, "attention: too many KV heads for the grid");
     dim3 grid(T, nkv * p.n_chunks, nsplit);

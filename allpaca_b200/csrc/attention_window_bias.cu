@@ -44,7 +44,7 @@ int attention_window_decode(const void* q, void* out, const void* cache, const i
                             const int* seq_start, const int* positions, int nseq, int nh, int nkv, int D, int VD, int P,
                             long long page_stride, float scale, float softcap, int window, const float* r1, const float* r2,
                             int RS, int voff, int bias_kind, int keep_first, const float* gate, long long gate_ld,
-                            const float* sink, int max_context, cudaStream_t stream);
+                            const float* sink, int max_context, int settled, cudaStream_t stream);
 
 // Key tiles a row tile walks: the tiles that hold kept first tokens (0 .. tiles_kept-1), then the
 // tiles from the window's first (tile_win) on; where the two meet or overlap, all tiles from 0.
@@ -851,7 +851,7 @@ AP_EXPORT int ap_attention_window_bias(const void* q, void* out, const void* cac
                                        int nh, int nkv, int D, int VD, int P, long long page_stride, float scale,
                                        float softcap, int window, const float* r1, const float* r2, int single_rows, int other_rows,
                                        int RS, int voff, int bias_kind, int keep_first, const float* gate,
-                                       long long gate_ld, const float* sink, int max_context, cudaStream_t stream) {
+                                       long long gate_ld, const float* sink, int max_context, int settled, cudaStream_t stream) {
     AP_REQUIRE(T >= 0 && nseq >= 0 && nh > 0 && nkv > 0 && nh % nkv == 0 && P > 0 && max_blocks > 0,
                "attention_window_bias: bad sizes T=%d heads=%d kv_heads=%d page=%d", T, nh, nkv, P);
     AP_REQUIRE(D > 0 && VD > 0 && D <= MAX_WIDE_HEAD && VD <= MAX_WIDE_HEAD,
@@ -878,7 +878,7 @@ AP_EXPORT int ap_attention_window_bias(const void* q, void* out, const void* cac
     if (single_rows == 1 && dtype == AP_BF16 && attention_window_decode_takes(q, cache, D, VD, page_stride, RS, voff)) {
         const int rc = attention_window_decode(q, out, cache, block_table, max_blocks, seq_start, positions, nseq, nh, nkv, D, VD,
                                                P, page_stride, scale, softcap, window, r1, r2, RS, voff, bias_kind, keep_first,
-                                               gate, gate_ld, sink, max_context, stream);
+                                               gate, gate_ld, sink, max_context, settled, stream);
         if (rc != AP_OK || !other_rows) return rc;
     } else if (single_rows == 1) {
         const int rep = nh / nkv;

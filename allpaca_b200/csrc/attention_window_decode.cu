@@ -56,10 +56,11 @@ attention_window_decode_kernel(const bf16* __restrict__ q, bf16* __restrict__ ou
                                size_t page_stride, float scale, float softcap, int window, const float* __restrict__ r1,
                                const float* __restrict__ r2, int RS, int voff, int bias_kind, int keep_first,
                                const float* __restrict__ gate, long long gate_ld, const float* __restrict__ sink,
-                               int nslice) {
+                               int nslice, int settled) {
     extern __shared__ __align__(16) float part[];            // [warps][heads here][VD], then maxima and sums of weights
     ap_pdl_trigger();
-    // the step's metadata and, but for the newest token, its pages are older than any kernel of the step
+    // where the caller says so, the step's metadata and, but for the newest token, its pages are older than the kernel ahead
+    if (!settled) ap_pdl_wait();
     const int seq = blockIdx.x / nslice, slice = blockIdx.x % nslice, kvh = blockIdx.y;
     const int row = seq_start[seq];
     if (seq_start[seq + 1] - row != 1) {
@@ -295,7 +296,7 @@ int attention_window_decode(const void* q, void* out, const void* cache, const i
                             const int* seq_start, const int* positions, int nseq, int nh, int nkv, int D, int VD, int P,
                             long long page_stride, float scale, float softcap, int window, const float* r1, const float* r2,
                             int RS, int voff, int bias_kind, int keep_first, const float* gate, long long gate_ld,
-                            const float* sink, int max_context, cudaStream_t stream) {
+                            const float* sink, int max_context, int settled, cudaStream_t stream) {
     const int rep = nh / nkv, nz = (rep + AWD_HEADS - 1) / AWD_HEADS;
     AP_REQUIRE(nkv <= 65535 && nz <= 65535, "attention_window_bias: %d key/value heads exceed the grid", nkv);
     // a CTA walks 64 keys at a time: shared by more CTAs while that shortens the walk and two of them fit every SM
@@ -337,6 +338,6 @@ int attention_window_decode(const void* q, void* out, const void* cache, const i
     AP_CHECK_PDL_LAUNCH("attention_window_decode",
                         cudaLaunchKernelEx(&cfg, kern, (const bf16*)q, (bf16*)out, (const bf16*)cache, block_table, max_blocks,
                                            seq_start, positions, nh, nkv, D, VD, P, (size_t)page_stride, scale, softcap, window,
-                                           r1, r2, RS, voff, bias_kind, keep_first, gate, gate_ld, sink, nslice));
+                                           r1, r2, RS, voff, bias_kind, keep_first, gate, gate_ld, sink, nslice, settled));
     return AP_OK;
 }

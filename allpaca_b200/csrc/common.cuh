@@ -45,8 +45,12 @@ typedef __nv_bfloat16 bf16;
 // ---- programmatic dependent launch ---------------------------------------------------
 // Kernels of the decode path are launched so that a kernel may start while the one before
 // it on the stream is still running.  Such a kernel does only work that depends on nothing
-// the earlier kernels write (set-up, prefetch of weights) until ap_pdl_wait() returns,
-// which is when every earlier kernel has finished and its writes are visible; and it calls
+// the earlier kernels write (set-up, prefetch of weights, options in pinned host memory) until
+// ap_pdl_wait() returns, which is when every earlier kernel has finished and its writes are
+// visible.  Decode attention, and the per-head products of single rows, also read a step's block
+// tables, positions and first rows and all keys but each row's newest ahead of it, but only where the
+// caller says that those are `settled`: written before the kernel ahead could begin.  An
+// engine's are, as its steps begin with a kernel in plain stream order.  And a kernel calls
 // ap_pdl_trigger() once the kernel after it may start the same way.  Launched without the
 // attribute both are no-ops.
 __device__ __forceinline__ void ap_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

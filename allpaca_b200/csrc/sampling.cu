@@ -392,10 +392,11 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
     }
 }
 
-// The kernel above: one CTA per row, any vocabulary.
+// The kernel above: one CTA per row, any vocabulary, in plain stream order.  early (here and below): the options lie in pinned host
+// memory, so a kernel may read them before those ahead of it have ended.
 AP_EXPORT int ap_sample_rows(const float* logits, long long row_stride, int R, int V, const float* temperature,
                              const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out,
-                             cudaStream_t stream) {
+                             int early, cudaStream_t stream) {
     AP_REQUIRE(R >= 0 && V > 0 && row_stride >= V, "sample: bad sizes R=%d V=%d", R, V);
     if (R == 0) return AP_OK;
     sample_kernel<<<R, SAMP_THREADS, 0, stream>>>(logits, row_stride, V, temperature, top_k, top_p, uniform, out, host_out);
@@ -407,14 +408,14 @@ AP_EXPORT int ap_sample_rows(const float* logits, long long row_stride, int R, i
 extern "C" int ap_sample_cluster_max_vocab(void);
 extern "C" int ap_sample_cluster(const float* logits, long long row_stride, int R, int V, const float* temperature,
                                  const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out,
-                                 cudaStream_t stream);
+                                 int early, cudaStream_t stream);
 
 // One token per row: the cluster kernel where the vocabulary fits its registers (up to 262144
 // entries), else one CTA per row.
 AP_EXPORT int ap_sample(const float* logits, long long row_stride, int R, int V, const float* temperature,
                         const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out,
-                        cudaStream_t stream) {
+                        int early, cudaStream_t stream) {
     if (V > 0 && V <= ap_sample_cluster_max_vocab() && R <= 65535)
-        return ap_sample_cluster(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
-    return ap_sample_rows(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
+        return ap_sample_cluster(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, early, stream);
+    return ap_sample_rows(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, early, stream);
 }

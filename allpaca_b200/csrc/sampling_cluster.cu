@@ -493,16 +493,17 @@ __global__ void __launch_bounds__(SC_THREADS, PER_SM)
 sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, int V,
                       const float* __restrict__ temperature, const int* __restrict__ top_k,
                       const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out,
-                      int* __restrict__ host_out) {
+                      int* __restrict__ host_out, int early) {
     cg::cluster_group cl = cg::this_cluster();
     __shared__ ScShared sh;
     const int rank = (int)cl.block_rank();
     const int r = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float* src = logits + (size_t)r * row_stride;
-    // the row's options may lie in pinned host memory: each is asked for once, while the logits are still being formed
+    // the row's options may lie in pinned host memory (early): each is asked for once, while the logits are still being formed
     __shared__ float option_s[4];
     ap_pdl_trigger();
+    if (!early) ap_pdl_wait();
     if (threadIdx.x < 4)
         option_s[threadIdx.x] = threadIdx.x == 0 ? temperature[r] : threadIdx.x == 1 ? __int_as_float(top_k[r])
                                 : threadIdx.x == 2 ? top_p[r] : uniform[r];
@@ -714,7 +715,7 @@ sample_cluster_kernel(const float* __restrict__ logits, long long row_stride, in
 
 template <int E>
 static int sc_launch(const float* logits, long long row_stride, int R, int V, const float* temperature,
-                     const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out, cudaStream_t stream) {
+                     const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out, int early, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(SC_CLUSTER, R);
     cfg.blockDim = dim3(SC_THREADS);
@@ -731,7 +732,7 @@ static int sc_launch(const float* logits, long long row_stride, int R, int V, co
     cfg.numAttrs = ap_pdl_enabled() ? 2 : 1;
     const bool many = E <= 32 && R > 12;
     cudaError_t e = cudaLaunchKernelEx(&cfg, many ? sample_cluster_kernel<E, E <= 32 ? 2 : 1> : sample_cluster_kernel<E, 1>, logits,
-                                       row_stride, V, temperature, top_k, top_p, uniform, out, host_out);
+                                       row_stride, V, temperature, top_k, top_p, uniform, out, host_out, early);
     AP_REQUIRE(e == cudaSuccess, "sample (cluster): launch failed: %s", cudaGetErrorString(e));
     return AP_OK;
 }
@@ -741,16 +742,16 @@ AP_EXPORT int ap_sample_cluster_max_vocab(void) { return SC_CLUSTER * SC_THREADS
 
 AP_EXPORT int ap_sample_cluster(const float* logits, long long row_stride, int R, int V, const float* temperature,
                                 const int* top_k, const float* top_p, const float* uniform, int* out, int* host_out,
-                                cudaStream_t stream) {
+                                int early, cudaStream_t stream) {
     AP_REQUIRE(R >= 0 && V > 0 && row_stride >= V, "sample: bad sizes R=%d V=%d", R, V);
     AP_REQUIRE(V <= ap_sample_cluster_max_vocab(), "sample (cluster): a vocabulary of %d exceeds %d", V,
                ap_sample_cluster_max_vocab());
     AP_REQUIRE(R <= 65535, "sample (cluster): %d rows exceed the grid", R);
     if (R == 0) return AP_OK;
     const int per = (V + SC_CLUSTER * SC_THREADS - 1) / (SC_CLUSTER * SC_THREADS);
-    if (per <= 4) return sc_launch<4>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
-    if (per <= 8) return sc_launch<8>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
-    if (per <= 16) return sc_launch<16>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
-    if (per <= 32) return sc_launch<32>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
-    return sc_launch<64>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, stream);
+    if (per <= 4) return sc_launch<4>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, early, stream);
+    if (per <= 8) return sc_launch<8>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, early, stream);
+    if (per <= 16) return sc_launch<16>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, early, stream);
+    if (per <= 32) return sc_launch<32>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, early, stream);
+    return sc_launch<64>(logits, row_stride, R, V, temperature, top_k, top_p, uniform, out, host_out, early, stream);
 }

@@ -488,7 +488,7 @@ def gemm_tc_persistent(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, pair
 
 
 def _decode_attention(lib, q, out, cache_layer, block_table, positions, rows, num_heads, num_kv_heads, head_dim, P,
-                      scale, window, max_context, scratch, use_tma, mean_context=0) -> None:
+                      scale, window, max_context, scratch, use_tma, mean_context=0, settled=False) -> None:
     """The first ``rows`` rows of the batch, one per sequence: the split kernels."""
     tma = (use_tma and hasattr(lib, "ap_attention_decode_tma")
            and bool(lib.ap_attention_decode_tma_supports(num_heads, num_kv_heads, head_dim, P))
@@ -520,7 +520,7 @@ def _decode_attention(lib, q, out, cache_layer, block_table, positions, rows, nu
         call(lib, "ap_attention_decode_tma", q.data_ptr(), out.data_ptr(), cache_layer.data_ptr(),
              cache_layer.shape[0], block_table.data_ptr(), block_table.shape[1], positions.data_ptr(), rows,
              num_heads, num_kv_heads, head_dim, P, cache_layer.stride(0), float(scale), int(window or 0),
-             nsplit, po, pm, by_length, stream_handle())
+             nsplit, po, pm, 1 if settled else 0, by_length, stream_handle())
         return
     call(lib, "ap_attention_tc", q.data_ptr(), out.data_ptr(), cache_layer.data_ptr(),
          block_table.data_ptr(), block_table.shape[1], 0, positions.data_ptr(),
@@ -578,7 +578,7 @@ def attention(q: torch.Tensor, out: torch.Tensor, cache_layer: torch.Tensor,
               window: int = 0, seq_start: Optional[torch.Tensor] = None,
               query_lens: Optional[Sequence[int]] = None, max_context: int = 0,
               scratch=None, use_tcgen05: bool = True, use_tma: bool = True,
-              wide: Optional[bool] = None, mean_context: int = 0) -> None:
+              wide: Optional[bool] = None, mean_context: int = 0, settled: bool = False) -> None:
     """Causal attention of every row of ``q [T, nh*hd]`` over its sequence's cached keys.
 
     float32 runs the general CUDA-core kernel (the true 32-bit path).  bfloat16 runs on the
@@ -589,7 +589,11 @@ def attention(q: torch.Tensor, out: torch.Tensor, cache_layer: torch.Tensor,
     ``scratch(name, shape, dtype)`` supplies the partial-result buffers of the split kernel
     where its key slices are not combined inside a thread-block cluster.  ``max_context`` and
     ``mean_context`` (0: all alike) are bounds on the longest and the average number of keys of
-    the one-row sequences, from which the number of key slices is planned.
+    the one-row sequences, from which the number of key slices is planned.  ``settled``: the caller's
+    word that the block tables, the positions and all keys but each one-row sequence's newest were
+    written before the kernel launched ahead of this call could begin; the kernels for one-row
+    sequences then ask for them while that kernel still runs.  An engine's step may say so where it
+    begins with a kernel in plain stream order.
     """
     _check(q, "q", dims=2)
     _check(out, "out", q.dtype, 2)
@@ -619,7 +623,7 @@ def attention(q: torch.Tensor, out: torch.Tensor, cache_layer: torch.Tensor,
             nd += 1
         if nd > 0:
             _decode_attention(lib, q, out, cache_layer, block_table, positions, nd, num_heads, num_kv_heads,
-                              head_dim, P, scale, window, max_context, scratch, use_tma, mean_context)
+                              head_dim, P, scale, window, max_context, scratch, use_tma, mean_context, settled)
         if nd < nseq:
             _prompt_attention(lib, q, out, cache_layer, block_table, seq_start, positions, nd, query_lens[nd:], T,
                               num_heads, num_kv_heads, head_dim, P, scale, window, use_tcgen05, wide)
@@ -735,6 +739,7 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
             _check(t, n, dt, 1)
         elif not t.is_pinned() or t.dtype != dt or t.dim() != 1 or not t.is_contiguous():
             raise KernelError(f"sample: {n} must be a contiguous vector of {dt} on the device or in pinned memory")
+    early = not any(t.is_cuda for t in (temperature, top_k, top_p, uniform))     # no kernel writes what lies on the host
     for t, n in ((temperature, "temperature"), (top_k, "top_k"), (top_p, "top_p"), (uniform, "uniform"), (out, "out")):
         if t.shape[0] < R:
             raise KernelError(f"sample: {n} has fewer than {R} entries")
@@ -742,7 +747,7 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
     if entry is None:
         raise KernelError(f"sample: unknown method {method!r}")
     call(core(), entry, logits.data_ptr(), V, R, V, temperature.data_ptr(), top_k.data_ptr(),
-         top_p.data_ptr(), uniform.data_ptr(), out.data_ptr(), _host_tokens(host, R), stream_handle())
+         top_p.data_ptr(), uniform.data_ptr(), out.data_ptr(), _host_tokens(host, R), 1 if early else 0, stream_handle())
 
 
 def stage_step(host: torch.Tensor, dev: torch.Tensor, first: int, n: int, device_tokens: Optional[torch.Tensor] = None,

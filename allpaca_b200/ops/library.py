@@ -37,9 +37,9 @@ _CORE_SIGNATURES = {
     # int ap_stage_step(host, dev, first, n, device_tokens, off_tokens, tokens, index, stream)
     "ap_stage_step": [_P, _P, _I, _I, _P, _I, _I, _P, _P],
     "ap_argmax": [_P, _L, _I, _I, _P, _P, _P],
-    "ap_sample": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P, _P],
-    "ap_sample_rows": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P, _P],
-    "ap_sample_cluster": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P, _P],
+    "ap_sample": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P, _I, _P],
+    "ap_sample_rows": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P, _I, _P],
+    "ap_sample_cluster": [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P, _I, _P],
     # int ap_embed_sinusoid_norm(tokens, positions, table, table_dtype, inv_freq, norm_w, norm_dtype, eps, scale,
     #                            x, T, H, V, stream)
     "ap_embed_sinusoid_norm": [_P, _P, _P, _I, _P, _P, _I, _F, _F, _P, _I, _I, _I, _P],
@@ -51,21 +51,21 @@ _CORE_SIGNATURES = {
     # int ap_attention_window_bias(q, out, cache, dtype, block_table, max_blocks, seq_start, positions, nseq, T,
     #                              nh, nkv, D, VD, P, page_stride, scale, softcap, window, r1, r2, single_rows,
     #                              other_rows, record, value_offset, bias_kind, keep_first, gate, gate_ld, sink,
-    #                              max_context, stream)
+    #                              max_context, settled, stream)
     "ap_attention_window_bias": [_P, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _L, _F, _F, _I, _P, _P, _I, _I,
-                                 _I, _I, _I, _I, _P, _L, _P, _I, _P],
+                                 _I, _I, _I, _I, _P, _L, _P, _I, _I, _P],
     # int ap_latent_prepare(in, ld, q0, Q, q_weight, cq, kv0, R, rot, rot_dims, kv_weight, cache, act_dtype, positions,
     #                       token_seq, block_table, max_blocks, P, page_stride, cos_sin, eps, T, stream)
     "ap_latent_prepare": [_P, _L, _I, _I, _P, _P, _I, _I, _I, _I, _P, _P, _I, _P, _P, _P, _I, _I, _L, _P, _F, _I, _P],
     # int ap_head_project(in, in_dtype, in_ld, in_hs, w, w_dtype, out, out_dtype, out_ld, out_hs, T, H, K, N, tail,
-    #                     tail_dims, cos_sin, seq_start, nseq, stream)
-    "ap_head_project": [_P, _I, _L, _I, _P, _I, _P, _I, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P],
+    #                     tail_dims, cos_sin, seq_start, nseq, settled, stream)
+    "ap_head_project": [_P, _I, _L, _I, _P, _I, _P, _I, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, _I, _P],
     # int ap_latent_gather(cache, dtype, page_stride, P, record, block_table, max_blocks, seq_start, context_lens,
     #                      nseq, out, where, width, total, window, stream)
     "ap_latent_gather": [_P, _I, _L, _I, _I, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _P],
     # int ap_latent_decode(q, out, cache, block_table, max_blocks, seq_start, positions, nseq, nh, record, value,
-    #                      P, page_stride, scale, gate, gate_ld, nsplit, scratch, scratch_floats, window, sink, stream)
-    "ap_latent_decode": [_P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _L, _F, _P, _L, _I, _P, _L, _I, _P, _P],
+    #                      P, page_stride, scale, gate, gate_ld, nsplit, scratch, scratch_floats, window, sink, settled, stream)
+    "ap_latent_decode": [_P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _L, _F, _P, _L, _I, _P, _L, _I, _P, _I, _P],
     "ap_latent_decode_splits": [_I, _I, _I],
     "ap_latent_decode_takes": [_I, _I],
     # int ap_latent_prefill(q, out, kv, where, width, seq_start, positions, nseq, T, nh, key, value, scale, gate,
@@ -236,8 +236,8 @@ _OPTIONAL_ATTN_SIGNATURES: Dict[str, list] = {
     "ap_attention_tcgen05_wide_tokens_per_cta": [_I, _I],
     "ap_attention_tcgen05_wide_status": [],
     # int ap_attention_decode_tma(q, out, cache, num_pages, block_table, max_blocks, positions, T, nh, nkv, hd, P,
-    #                             page_stride, scale, window, nsplit, part_o, part_ml, by_length, stream)
-    "ap_attention_decode_tma": [_P, _P, _P, _L, _P, _I, _P, _I, _I, _I, _I, _I, _L, _F, _I, _I, _P, _P, _I, _P],
+    #                             page_stride, scale, window, nsplit, part_o, part_ml, settled, by_length, stream)
+    "ap_attention_decode_tma": [_P, _P, _P, _L, _P, _I, _P, _I, _I, _I, _I, _I, _L, _F, _I, _I, _P, _P, _I, _I, _P],
     "ap_attention_decode_tma_supports": [_I, _I, _I, _I],
     "ap_attention_decode_tma_in_cluster": [_I, _I, _I],
     "ap_attention_decode_tma_status": [],

@@ -120,7 +120,8 @@ def attention_window_bias(q: torch.Tensor, out: torch.Tensor, cache_layer: torch
                           single_rows: bool = False, other_rows: bool = True, bias: Optional[str] = "log",
                           keep_first: int = 0, gate: Optional[torch.Tensor] = None,
                           record: Optional[int] = None, value_offset: Optional[int] = None,
-                          sink: Optional[torch.Tensor] = None, softcap: float = 0.0, max_context: int = 0) -> None:
+                          sink: Optional[torch.Tensor] = None, softcap: float = 0.0, max_context: int = 0,
+                          settled: bool = False) -> None:
     """Causal attention of ``q [T, nh*D]`` over pages ``[pages, nkv, P, record]`` into
     ``out [T, nh*VD]``: ``score = cap(q.k * scale) - bias_h(distance)`` (``cap(s) = softcap * tanh(s / softcap)``
     where ``softcap`` is positive, else ``s``), over the last ``window`` keys (0: all)
@@ -139,7 +140,7 @@ def attention_window_bias(q: torch.Tensor, out: torch.Tensor, cache_layer: torch
     whether the step has sequences of another length as well (they run on the general kernel,
     which serves everything when ``single_rows`` is False).  ``max_context`` (0: not known): the longest context
     among the sequences that bring one row; from a thousand visible keys on, the decode kernel shares a
-    sequence's key tiles between the CTAs of a cluster."""
+    sequence's key tiles between the CTAs of a cluster.  ``settled``: as for :func:`ops.attention`."""
     _check(q, "q", dims=2)
     _check(out, "out", q.dtype, 2)
     T = q.shape[0]
@@ -176,7 +177,7 @@ def attention_window_bias(q: torch.Tensor, out: torch.Tensor, cache_layer: torch
          int(window or 0),
          r1.data_ptr() if r1 is not None else 0, r2.data_ptr() if r2 is not None else 0,
          2 if single_rows == "skip" else (1 if single_rows else 0), 1 if other_rows else 0, record, value_offset, BIAS_KINDS[bias], int(keep_first or 0),
-         gptr, gld, sink.data_ptr() if sink is not None else 0, int(max_context or 0), stream_handle())
+         gptr, gld, sink.data_ptr() if sink is not None else 0, int(max_context or 0), 1 if settled else 0, stream_handle())
 
 
 def latent_prepare(proj: torch.Tensor, q_col: int, q_rank: int, q_weight: Optional[torch.Tensor],
@@ -227,14 +228,14 @@ def latent_prepare(proj: torch.Tensor, q_col: int, q_rank: int, q_weight: Option
 
 def head_project(inp: torch.Tensor, weight: Optional[torch.Tensor], out: torch.Tensor, heads: int, tail: int = 0,
                  tail_dims: int = 0, cos_sin: Optional[torch.Tensor] = None,
-                 singles: Optional[torch.Tensor] = None, num_seqs: int = 0) -> None:
+                 singles: Optional[torch.Tensor] = None, num_seqs: int = 0, settled: bool = False) -> None:
     """``out[t, h, :N] = inp[t, h, :K] @ weight[h]`` for ``weight [heads, K, N]``, every sum 32-bit in a
     fixed order.  ``inp [T, heads*(K + tail)]`` and ``out [T, heads*(N + tail)]``: the ``tail``
     numbers behind a head's ``K`` inputs go behind its ``N`` outputs, the first ``tail_dims`` of them
     rotated by ``cos_sin [T, tail_dims/2, 2]`` (entry ``i`` paired with ``i + tail_dims/2``).  With
     ``weight`` None the ``K`` numbers are copied (``out`` has ``inp``'s shape): a rotation alone.  ``singles`` (the
     step's ``seq_start``, of ``num_seqs`` sequences): only the rows of sequences that bring one row are needed; what
-    becomes of the others is not said."""
+    becomes of the others is not said; ``settled``, of ``singles``: as for :func:`ops.attention`."""
     if inp.dim() != 2 or not inp.is_cuda or inp.stride(1) != 1:
         raise KernelError("head_project: inp must be a CUDA matrix with contiguous rows (it may be a view of wider rows)")
     _check(out, "out", dims=2)
@@ -266,7 +267,7 @@ def head_project(inp: torch.Tensor, weight: Optional[torch.Tensor], out: torch.T
         ssptr = singles.data_ptr()
     call(core(), "ap_head_project", inp.data_ptr(), dtype_code(inp.dtype), inp.stride(0), K + tail, weight_ptr,
          weight_code, out.data_ptr(), dtype_code(out.dtype), out.stride(0), N + tail, T, H, K, N,
-         int(tail), int(tail_dims), csptr, ssptr, int(num_seqs), stream_handle())
+         int(tail), int(tail_dims), csptr, ssptr, int(num_seqs), 1 if settled else 0, stream_handle())
 
 
 CONV_ACTIVATIONS = {None: 0, "silu": 1}
@@ -394,14 +395,15 @@ def latent_decode_takes(record: int, value_dim: int) -> bool:
 def latent_decode(q: torch.Tensor, out: torch.Tensor, cache_layer: torch.Tensor, block_table: torch.Tensor,
                   seq_start: torch.Tensor, positions: torch.Tensor, num_seqs: int, num_heads: int, record: int,
                   value_dim: int, scale: float, gate: Optional[torch.Tensor], max_context: int, workspace,
-                  window: int = 0, sink: Optional[torch.Tensor] = None) -> None:
+                  window: int = 0, sink: Optional[torch.Tensor] = None, settled: bool = False) -> None:
     """bfloat16 attention of the sequences that bring ONE row over pages ``[pages, P, record]`` whose
     records are every head's key and, in their first ``value_dim`` numbers, every head's value:
     ``q [T, heads*record]`` -> ``out [T, heads*value_dim]`` times ``sigmoid(gate[t, h])`` (rows of other
     sequences are left alone).  All heads of a sequence share the key tiles on the tensor cores; the
     keys are cut into slices by ``max_context`` (the longest context the step may hold), whose partial
     results wait in a buffer taken from ``workspace``.  ``window`` (0: none): a row sees its last ``window``
-    keys; ``sink`` (32-bit ``[heads]``): the denominator also holds ``exp(sink[h])``."""
+    keys; ``sink`` (32-bit ``[heads]``): the denominator also holds ``exp(sink[h])``.  ``settled``: as for
+    :func:`ops.attention`."""
     _check(q, "q", torch.bfloat16, 2)
     _check(out, "out", torch.bfloat16, 2)
     T = q.shape[0]
@@ -433,7 +435,7 @@ def latent_decode(q: torch.Tensor, out: torch.Tensor, cache_layer: torch.Tensor,
     call(lib, "ap_latent_decode", q.data_ptr(), out.data_ptr(), cache_layer.data_ptr(), block_table.data_ptr(),
          block_table.shape[1], seq_start.data_ptr(), positions.data_ptr(), int(num_seqs), int(num_heads), int(record),
          int(value_dim), P, page_stride, float(scale), gptr, gld, nsplit, scratch.data_ptr(), need, window,
-         sink.data_ptr() if sink is not None else 0, stream_handle())
+         sink.data_ptr() if sink is not None else 0, 1 if settled else 0, stream_handle())
 
 
 def latent_prefill_takes(key_dim: int, value_dim: int) -> bool:

@@ -175,7 +175,7 @@ class GroupedQueryAttention(Mixer):
                       step.positions, self.nh, self.nkv, self.hd, self.scale,
                       self.window or 0, seq_start=step.seq_start, query_lens=step.host_query_lens,
                       max_context=step.max_decode_context_len or step.max_context_len, scratch=ws.get,
-                      mean_context=step.mean_context_len)
+                      mean_context=step.mean_context_len, settled=True)
         return attn
 
     def _materialise(self, qkv: torch.Tensor, T: int) -> torch.Tensor:

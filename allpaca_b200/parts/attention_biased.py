@@ -231,7 +231,7 @@ class DistanceBiasedAttention(Mixer):
                                   self.nh, self.nkv, self.hd, self.vd, self.scale, self.window or 0, self.r1, self.r2,
                                   single_rows=single, other_rows=step.max_query_len != 1, bias=self.bias_kind,
                                   keep_first=self.keep_first, gate=gate, softcap=self.softcap, sink=self.sink,
-                                  max_context=step.max_decode_context_len or step.max_context_len)
+                                  max_context=step.max_decode_context_len or step.max_context_len, settled=True)
         delta = self.o.forward(out, "battn.o", "delta", into=into)
         if self.output_bias is not None and add_bias:
             ops.bias_add(delta if into is not None else delta[0], self.output_bias)
