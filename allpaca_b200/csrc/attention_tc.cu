@@ -656,9 +656,9 @@ attention_split_tma_kernel(const __grid_constant__ CUtensorMap tmap_kv, const __
     // before they read the queries.
     if (!p.settled) ap_pdl_wait();
 
-    // Row == sequence index.  Where the CTAs are more than fit at once and the sequences differ in length, the
-    // CTAs (which start in the order of their index) take all heads of the longest sequence first: a long one
-    // that starts last is waited for by everybody (24 rows of 16 to 4096 keys, 8 KV heads, in a step: 18.0 us, 21.5 in the order of the rows).
+    // Row == sequence index.  Where the caller asks for it (`longest_first` of the ops says when, with both sides measured), the
+    // CTAs, which start in the order of their index, take all heads of the longest sequence first: a long one that starts
+    // last is waited for by everybody.
     int row = blockIdx.x, by = blockIdx.y;
     if (p.by_length) {
         const int at = blockIdx.y * p.T + blockIdx.x, want = at / gridDim.y;
