@@ -92,7 +92,7 @@ argmax_cluster_kernel(const float* __restrict__ logits, long long row_stride, in
     }
     if (rank == 0 && (int)threadIdx.x < V - 4 * runs) {
         const int i = 4 * runs + threadIdx.x;
-        argmax_better(bv, bi, row[i], i);
+        if (row[i] > bv) { bv = row[i]; bi = i; }            // (the highest ids; a row without a finite value keeps none)
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll

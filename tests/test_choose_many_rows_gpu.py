@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.mark.parametrize("R,V", [(1, 8188), (1, 8192), (3, 8195), (37, 9000), (38, 9000), (2, 128256), (4, 40001)])
+@pytest.mark.parametrize("R,V", [(1, 8188), (1, 16384), (1, 16385), (3, 16387), (37, 20000), (38, 20000), (2, 128256), (4, 40001),
+                                 (3, 40002)])
 def test_first_maximum(R, V):
     from allpaca_b200 import ops
     g = torch.Generator().manual_seed(V + R)
@@ -25,6 +26,12 @@ def test_first_maximum(R, V):
     want = torch.nan_to_num(l, nan=-torch.inf).argmax(1)
     assert out[0] == 5 and torch.equal(out.cpu().long(), want) or (R > 2 and out[2] == 0)
     want[2 if R > 2 else 0] = 0 if R > 2 else 5
+    assert torch.equal(out.cpu().long(), want)
+    # rows that begin on 16-byte boundaries whatever their length, with larger numbers behind their ends
+    wide = torch.full((R, (V + 3) // 4 * 4), 99.0)
+    wide[:, :V] = l
+    wide, out = wide.to(DEV), torch.full_like(out, -1)
+    ops.call(ops.core(), "ap_argmax", wide.data_ptr(), wide.shape[1], R, V, out.data_ptr(), 0, ops.stream_handle())
     assert torch.equal(out.cpu().long(), want)
 
 
