@@ -126,8 +126,11 @@ AP_EXPORT int ap_argmax(const float* logits, long long row_stride, int R, int V,
                         cudaStream_t stream) {
     AP_REQUIRE(R >= 0 && V > 0 && row_stride >= V, "argmax: bad sizes R=%d V=%d", R, V);
     if (R == 0) return AP_OK;
-    // rows that fill the GPU by themselves, short ones and rows off a 16-byte boundary take a CTA each
-    if (R <= 2 * 148 / ARGMAX_CLUSTER && V >= 4 * ARGMAX_CLUSTER * ARGMAX_THREADS / 2 && row_stride % 4 == 0 && ((uintptr_t)logits & 15) == 0) {
+    // A cluster to a row from 16385 logits on and for as many rows as find room at two CTAs to an SM; and rows on 16-byte boundaries.
+    // With a CTA and with a cluster to a row, us, logits in L2: 8192 logits, 1 row 2.0 and 2.2, 37 rows 2.1 and 3.0; 16384, 1 row 2.3 and
+    // 2.2, 37 rows 2.4 and 3.0; 20480, 1 row 2.6 and 2.4, 37 rows 3.1 and 3.1; 128256, 1 row 5.8 and 3.1, 37 rows 6.6 and 4.5.  Beyond 37 rows:
+    // 48 of 32000 4.2 and 3.3, 64 of 32000 4.8 and 5.4, 128 of 32000 5.1 and 8.7, of 128256 11.5 and 12.2.
+    if (R <= 2 * 148 / ARGMAX_CLUSTER && V > 4 * ARGMAX_CLUSTER * ARGMAX_THREADS && row_stride % 4 == 0 && ((uintptr_t)logits & 15) == 0) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(R * ARGMAX_CLUSTER));
         cfg.blockDim = dim3(ARGMAX_THREADS);
