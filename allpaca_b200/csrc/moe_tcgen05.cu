@@ -484,6 +484,11 @@ AP_EXPORT int ap_moe_tc(const void* a, const void* w, void* out, int out_dtype, 
         if (!gated && out_dtype == AP_F32) return moe_launch<BN, SUB, false, float>(a, w, out, g, pairs, x_a, x_w, x_out, stream);      \
         AP_REQUIRE(false, "moe_tc: unsupported out dtype %d", out_dtype);                                              \
     } while (0)
+    // Tiles of about twice the average, so that a second tile of an expert is rare; 256 weight rows by 128 where a weight tile's
+    // bytes are no longer the cost.  Both products, us, tiles of 16, 32, 64 and 2 x 128 rows, pairs dealt at random.  16 experts of
+    // 2048 x 1024 with gates: 8 pairs to an expert 41, 41, 41, 43; 16 54, 42, 42, 44; 32 62, 52, 44, 46; 48 76, 49, 46, 47; 64 77, 65, 58, 49; 256
+    // 262, 148, 99, 102.  32 of 4096 x 2048 without: 8 176, 176, 176, 182; 16 181, 180, 179, 184; 32 240, 195, 188, 198; 49 312, 215, 186, 194; 64 360, 239,
+    // 208, 206; 256 1248, 705, 465, 411.
     if (2 * mean <= 16) LAUNCH(16, 1);
     if (2 * mean <= 32) LAUNCH(32, 1);
     if (mean <= 48) LAUNCH(64, 1);

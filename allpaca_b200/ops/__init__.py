@@ -642,8 +642,8 @@ def longest_first(ctas: int, nsplit: int, slots: int, keys: int, mean_context: i
     up to 700 to 8192 keys, five mixtures of lengths, head sizes 64 and 128 on 2 to 8 key/value heads: 573 workloads, keys
     rotating over more than L2): the 86 that the rule takes are 1 to 23 % faster than in the order of the sequences (64 of up
     to 4096 keys, mean 2000, head size 128: 101 -> 78 us; 24 of up to 2881, mean 625, head size 64: 20 -> 16).  The others would
-    be 2 % slower on average: shorter slices up to 30 %, eight slices or more than two rounds of CTAs up to 27 %; 149 of them
-    would gain 2 % and more, 248 would lose that."""
+    be 2 % slower on average: shorter slices up to 21 %, eight slices or more rounds of CTAs up to 30 %; 149 of them would gain
+    2 % and more, 248 would lose that."""
     tiles = keys // (64 * nsplit)
     return (slots < ctas * nsplit and ctas * nsplit * 10 < slots * 19 and nsplit <= 4
             and tiles >= (8 if nsplit == 4 else 24) and 0 < mean_context * 4 < keys * 3)
