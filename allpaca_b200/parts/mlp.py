@@ -24,7 +24,9 @@ class SwiGLU(FeedForward):
     Llama path), ``activation`` of the gate (``"silu"`` and ``"gelu_tanh"`` are applied in the
     product's epilogue on the tensor cores; others, like ``"relu"``, by a kernel of its own after the
     product; only with ``"silu"`` is the norm before folded in), ``names`` (the
-    local tensor names of gate, up and down; default ``gate_proj.weight`` and so on)."""
+    local tensor names of gate, up and down; default ``gate_proj.weight`` and so on), ``halves`` (True: the
+    matrix is held as the gate's rows, then the up rows, for a caller that takes it in that order; the activation is then a
+    kernel of its own on 32-bit sums; without biases)."""
 
     def __init__(self, params, env: BuildEnv):
         super().__init__(params, env)
@@ -38,6 +40,9 @@ class SwiGLU(FeedForward):
         self.gate_name, self.up_name, self.down_name = names
         if self.bias and params.get("names"):
             raise ValueError("a gated feed-forward with biases keeps the default tensor names")
+        self.halves = bool(params.get("halves", False))
+        if self.bias and self.halves:
+            raise ValueError("a gated feed-forward in halves takes no biases")
         self.gate_up = Linear(env, 2 * self.inter, self.hidden)
         self.down = Linear(env, self.hidden, self.inter)
 
@@ -53,13 +58,17 @@ class SwiGLU(FeedForward):
 
     def load(self, tensors: Mapping[str, torch.Tensor]) -> None:
         gate, up = tensors[self.gate_name], tensors[self.up_name]
+        if self.halves:
+            self.gate_up.load(torch.cat([gate, up]))
+            self.down.load(tensors[self.down_name])
+            return
         gu_bias = torch.stack([tensors["gate_proj.bias"], tensors["up_proj.bias"]], dim=1).reshape(-1) \
             if self.bias else None
         self.gate_up.load(torch.stack([gate, up], dim=1).reshape(2 * self.inter, self.hidden), gu_bias)
         self.down.load(tensors[self.down_name], tensors["down_proj.bias"] if self.bias else None)
 
     def can_fold_input_norm(self) -> bool:
-        return self.activation == "silu" and self.gate_up.fusable() and self.down.fusable()
+        return self.activation == "silu" and not self.halves and self.gate_up.fusable() and self.down.fusable()
 
     def fold_input_norm(self, weight: torch.Tensor) -> None:
         """Multiply the weight of the norm before this feed-forward into its first product."""
@@ -77,7 +86,10 @@ class SwiGLU(FeedForward):
     def forward(self, h: torch.Tensor, step) -> torch.Tensor:
         T = h.shape[0]
         act = None
-        if self.activation in ("silu", "gelu_tanh"):
+        if self.halves:
+            act = self.env.workspace.get("ffn.act", (T, self.inter), self.env.dtype)
+            ops.gated_act(self.gate_up.forward(h, "ffn.sums", "float32"), act, self.activation)
+        elif self.activation in ("silu", "gelu_tanh"):
             act = self.gate_up.forward_gated(h, "ffn.act", activation=self.activation)   # the product's epilogue
         if act is None:
             gu = self.gate_up.forward(h, "ffn.gate_up", "either")

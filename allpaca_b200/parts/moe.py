@@ -28,7 +28,8 @@ activations of ``ops.gated_act`` (``clamped_sigmoid``: ``g' = min(g, limit)``,
 On the device the (row, choice) pairs are grouped by expert, every expert's rows run through
 its two products in tiles, and a last pass adds each row's weighted results in the order of
 its choices.  Counts and tiles never leave the device, so a step can be replayed from a CUDA
-graph, and a row's result does not depend on what else is in the batch.
+graph.  In 32 bits a row's result does not depend on what else is in the batch; in bfloat16 the number of pairs in
+the step chooses between the kernels below, whose sums have different orders.
 
 In bfloat16 the rows are gathered in grouped order and both products of all experts run on the tensor cores, a launch
 each; a step of very few pairs, other types and sizes that TMA cannot address take kernels on the CUDA cores.
@@ -99,16 +100,16 @@ class RoutedExperts(FeedForward):
             sh = dict(p["shared"])
             one = {"hidden_size": self.hidden, "intermediate_size": int(sh["size"]),
                    "activation": sh.get("activation", self.activation)}
-            if self.gated:
-                one["names"] = ("shared.gate", "shared.up", "shared.down")
-            else:
-                one.update(names=("shared.up", "shared.down"), bias=False)
-            self.shared = build("feed_forward", PartSpec("swiglu" if self.gated else "dense_act", one), env)
-            self.shared_gated = bool(sh.get("gate", False))
             # with the experts' activation it can ride in their launches, as one more expert of its own size
             self.shared_size = int(sh["size"])
             self.shared_rides = (env.dtype == torch.bfloat16 and one["activation"] == self.activation != "clamped_sigmoid"
                                  and self.hidden % 8 == 0 and self.shared_size % 8 == 0)
+            if self.gated:
+                one.update(names=("shared.gate", "shared.up", "shared.down"), halves=self.shared_rides)
+            else:
+                one.update(names=("shared.up", "shared.down"), bias=False)
+            self.shared = build("feed_forward", PartSpec("swiglu" if self.gated else "dense_act", one), env)
+            self.shared_gated = bool(sh.get("gate", False))
 
     def parts(self):
         yield self
@@ -136,9 +137,9 @@ class RoutedExperts(FeedForward):
             self.shared.load({n: tensors[n] for n in self.shared.weights()})
             self.shared_gate = tensors["shared.sg"].reshape(-1).contiguous() if self.shared_gated else None
             if self.shared_rides and tensors["shared.up"].dtype == tensors["shared.down"].dtype == torch.bfloat16:
-                self.shared_first = torch.cat([tensors["shared.gate"], tensors["shared.up"]]).contiguous() if self.gated \
-                    else tensors["shared.up"].contiguous()
-                self.shared_down = tensors["shared.down"].contiguous()
+                # the shared part's own matrices, in the order that the routed products take
+                self.shared_first = self.shared.gate_up.weight if self.gated else self.shared.up.weight
+                self.shared_down = self.shared.down.weight
         self.router_b = tensors[self.router_bias_name].float().contiguous() if self.router_bias else None
         # [experts, 2 F, hidden]: an expert's gate rows, then its up rows (without gates [experts, F, hidden]);
         # [experts, hidden, F]

@@ -98,3 +98,26 @@ def test_a_shared_expert_without_any_pair(T, gated, name):
     for out in outs:
         near(out, want, True)
     near(sums, outs[1].double().cpu() @ xdown.double().T, False)
+
+
+@pytest.mark.parametrize("T", [1, 40, 300])
+@pytest.mark.parametrize("activation", ["silu", "relu"])
+def test_a_gated_feed_forward_held_in_halves(T, activation):
+    """What a shared expert runs as where it cannot ride, against 64 bits: the sums stay in 32 bits up to the activation."""
+    from allpaca_b200.parts import BuildEnv, Workspace
+    from allpaca_b200.parts.base import PartSpec, build
+    H, S = 72, 136
+    g = torch.Generator().manual_seed(T)
+    h = torch.randn(T, H, generator=g).to(torch.bfloat16)
+    tensors = {"gate_proj.weight": matrix(g, S, H), "up_proj.weight": matrix(g, S, H), "down_proj.weight": matrix(g, H, S)}
+    z, u = (h.double() @ tensors[n].double().T for n in ("gate_proj.weight", "up_proj.weight"))
+    mid = (torch.nn.functional.silu(z) if activation == "silu" else torch.relu(z)) * u
+    want = mid @ tensors["down_proj.weight"].double().T
+    env = BuildEnv(dtype=torch.bfloat16, device=torch.device(DEV), workspace=Workspace(torch.device(DEV)), page_size=16, max_seqs=1)
+    part = build("feed_forward", PartSpec("swiglu", {"hidden_size": H, "intermediate_size": S, "activation": activation,
+                                                     "halves": True}), env)
+    part.load({n: t.to(DEV) for n, t in tensors.items()})
+    got = part.forward(h.to(DEV), None)[0].double().cpu()
+    # the activation is stored in bfloat16: half a unit in the last place of each of the S terms, whose squares add up
+    tol = 6 * 2.0 ** -9 * torch.sqrt((mid ** 2) @ (tensors["down_proj.weight"].double() ** 2).T) + 2e-5
+    assert bool(((got - want).abs() <= tol).all()), float(((got - want).abs() / tol).max())
