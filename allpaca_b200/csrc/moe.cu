@@ -27,8 +27,7 @@
 // ---- the activation alone ------------------------------------------------------------
 template <typename TI, typename TO>
 __global__ void gated_act_kernel(const TI* __restrict__ in, TO* __restrict__ out, int T, int I, int pairs, int act,
-                                 float limit, float alpha, float shift, const float* __restrict__ row_scale,
-                                 const int* __restrict__ scale_index) {
+                                 float limit, float alpha, float shift) {
     ap_pdl_trigger();
     ap_pdl_wait();
     const size_t n = (size_t)T * I;
@@ -37,23 +36,19 @@ __global__ void gated_act_kernel(const TI* __restrict__ in, TO* __restrict__ out
         const size_t base = t * 2 * (size_t)I;
         const float g = ap_to_float(in[pairs ? base + 2 * j : base + j]);
         const float u = ap_to_float(in[pairs ? base + 2 * j + 1 : base + I + j]);
-        // a scale of the row's INPUT: both products are linear in it, so it multiplies both sums
-        const float sc = row_scale ? row_scale[scale_index ? scale_index[t] : t] : 1.0f;
-        out[e] = ap_from_float<TO>(gated_activation(g * sc, u * sc, act, limit, alpha, shift));
+        out[e] = ap_from_float<TO>(gated_activation(g, u, act, limit, alpha, shift));
     }
 }
 
 AP_EXPORT int ap_gated_act(const void* in, int in_dtype, void* out, int out_dtype, int T, int I, int pairs, int act,
-                           float limit, float alpha, float shift, const float* row_scale, const int* scale_index,
-                           cudaStream_t stream) {
+                           float limit, float alpha, float shift, cudaStream_t stream) {
     AP_REQUIRE(T >= 0 && I > 0 && act >= 0 && act <= ACT_RELU2, "gated_act: bad sizes T=%d I=%d or activation %d", T, I, act);
     if (T == 0) return AP_OK;
     long long blocks = ((long long)T * I + 255) / 256;
     if (blocks > 148 * 32) blocks = 148 * 32;
 #define LAUNCH(TI, TO)                                                                                              \
     AP_CHECK_PDL_LAUNCH("gated_act", ap_launch_pdl(gated_act_kernel<TI, TO>, dim3((unsigned)blocks), dim3(256), 0, stream, \
-                                                   (const TI*)in, (TO*)out, T, I, pairs, act, limit, alpha, shift, row_scale, \
-                                                   scale_index))
+                                                   (const TI*)in, (TO*)out, T, I, pairs, act, limit, alpha, shift))
     if (in_dtype == AP_F32 && out_dtype == AP_F32) LAUNCH(float, float);
     else if (in_dtype == AP_F32 && out_dtype == AP_BF16) LAUNCH(float, bf16);
     else if (in_dtype == AP_BF16 && out_dtype == AP_BF16) LAUNCH(bf16, bf16);

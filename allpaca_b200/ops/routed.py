@@ -19,23 +19,18 @@ def activation_code(name: str) -> int:
 
 
 def gated_act(gate_up: torch.Tensor, out: torch.Tensor, activation: str = "silu", pairs: bool = False,
-              limit: float = 0.0, alpha: float = 1.0, shift: float = 0.0,
-              row_scale: Optional[torch.Tensor] = None, scale_index: Optional[torch.Tensor] = None) -> None:
+              limit: float = 0.0, alpha: float = 1.0, shift: float = 0.0) -> None:
     """``out[t, j] = act(gate, up)`` for ``gate_up [T, 2I]`` holding ``[gate | up]`` (or, with
     ``pairs``, gate and up columns alternating).  ``silu``: ``silu(g) u``; ``relu``: ``max(g, 0) u``;
     ``clamped_sigmoid``: ``g' sigmoid(alpha g') (u' + shift)`` with ``g' = min(g, limit)`` and
-    ``u' = clamp(u, -limit, limit)``; ``gelu_tanh``: ``0.5 g (1 + tanh(sqrt(2/pi) (g + 0.044715 g^3))) u``; ``relu2``: ``max(g, 0)^2 u``.
-    ``row_scale`` (32-bit): gate and up of row ``t`` are first multiplied by ``row_scale[scale_index[t]]``
-    (``scale_index`` int32 or None: ``row_scale[t]``), which is what a scale of the row's input does to both."""
+    ``u' = clamp(u, -limit, limit)``; ``gelu_tanh``: ``0.5 g (1 + tanh(sqrt(2/pi) (g + 0.044715 g^3))) u``; ``relu2``: ``max(g, 0)^2 u``."""
     _check(gate_up, "gate_up", dims=2)
     _check(out, "out", dims=2)
     T, inter = out.shape
     if tuple(gate_up.shape) != (T, 2 * inter):
         raise KernelError("gated_act: out must be [T, I] for gate_up [T, 2I]")
     call(core(), "ap_gated_act", gate_up.data_ptr(), dtype_code(gate_up.dtype), out.data_ptr(), dtype_code(out.dtype),
-         T, inter, 1 if pairs else 0, activation_code(activation), float(limit), float(alpha), float(shift),
-         row_scale.data_ptr() if row_scale is not None else 0,
-         scale_index.data_ptr() if scale_index is not None else 0, stream_handle())
+         T, inter, 1 if pairs else 0, activation_code(activation), float(limit), float(alpha), float(shift), stream_handle())
 
 
 def moe_route(logits: torch.Tensor, bias: Optional[torch.Tensor], chosen: torch.Tensor, weight: torch.Tensor) -> None:
