@@ -32,7 +32,8 @@ AP_EXPORT int ap_attention_head_dim(void) { return HD; }
 
 // A CTA takes one row and one head, 128 keys at a time.  Latency bounds it (a decode step's keys are few): a key's page is looked up
 // once, by the thread that forms its score with 16-byte loads of the key; the weighted sum of the values deals a chunk's keys to
-// eight or more groups of threads, 16 bytes of the head to a thread, and adds the groups up in their order.
+// groups of threads, 16 bytes of the head to a thread (head size 64 eight groups, 128 four, 256 two), and adds the groups up in
+// their order.
 // Measured (one B200, 32-bit, head size 64, 32 heads on 8, in a step): 4 rows of some 100 keys 7.9 us, 173 rows of 20 to 90 20.8;
 // a thread per column walking all keys, with a page lookup each, took 18.4 and 53.
 #define VEC (HD % 4 == 0 ? 4 : 1)

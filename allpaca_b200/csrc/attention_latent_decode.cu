@@ -10,10 +10,9 @@
 //   O [16 x R] += P [16 x 64] V [64 x R]          warp w: its eighth of the R columns; V is the same
 //                                                 tile, read transposed (ldmatrix.trans)
 //
-// Key tiles come by cp.async.  With one tile buffer (LD_STAGES 1, the default) two CTAs share an SM and
-// one computes while the other loads; with two buffers a CTA loads its next tile while it uses this
-// one and has the SM alone (measured: 74 against 110 us for 64 sequences of 2048 keys, 32 against 34
-// for 8 of 4096, 39 against 34 for one of 8192).  The slices of a sequence's keys leave unnormalised sums with their maximum
+// Key tiles come by cp.async into one buffer, so that two CTAs share an SM and one computes while the other
+// loads (two buffers, a CTA alone on the SM loading its next tile while it uses this one, were slower: 64 sequences
+// of 2048 keys 74 us with one, 110 with two; 8 of 4096 32 and 34; one of 8192 39 and 34).  The slices of a sequence's keys leave unnormalised sums with their maximum
 // and weight sum: up to eight slices are the CTAs of a cluster, which merge them through distributed shared memory, apply the
 // output gate and round; more (few sequences of long contexts) go through memory to a second kernel that does the same.
 // Scores, softmax and sums are 32-bit.

@@ -1,8 +1,8 @@
 """The 32-bit path gives a row the same bits whatever else is in the batch, however its
 prompt was cut into steps and whichever pages it lies in.
 
-The kernels are written for it: the CUDA-core product sums k in ascending order inside one
-thread per output, the norm reduces a row inside one block in a fixed order, and the 32-bit
+The kernels are written for it: the CUDA-core products cut k into runs that depend on its length
+alone, each one thread's sum in ascending order, added up in their order; the norm reduces a row inside one block in a fixed order, and the 32-bit
 attention walks a row's keys in chunks that start at the row's first visible position, not at
 a portion's edge.  The reference guards the same property of its kernels
 (crates/allpaca-cuda/src/lib.rs:5841-5903, crates/allpaca-core/src/model.rs:10851-10863).
