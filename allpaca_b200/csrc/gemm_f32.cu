@@ -9,8 +9,8 @@
 //   16-byte read serves 16 to 32 multiply-adds.  Where the 128-row tiles do not fill the GPU, the runs of a tile go to
 //   the eight CTAs of a cluster, which add up through distributed shared memory; else a CTA walks all of K and keeps
 //   the finished runs' sum beside the current one.
-// * beyond, tiles of 64, 96 or 128 rows x 128 columns, always a cluster of eight per tile: 8 x 16 outputs to a thread (a
-//   byte read from shared memory serves 5.3 multiply-adds; at 8 x 8 the reads take as long as the arithmetic).
+// * beyond, tiles of 64 to 176 rows x 96, 112 or 128 columns, always a cluster of eight per tile: up to 11 x 14 outputs to a thread (a
+//   byte read from shared memory serves 6.2 multiply-adds; at 8 x 8 the reads take as long as the arithmetic).
 //
 // Measured (one B200, weights rotating over more than L2; in brackets the 64 x 64 tiles of gemm_simt.cu, which load 4 bytes
 // at a time), us:
@@ -19,7 +19,8 @@
 //      1     7.5 (152)      6.5 (153)      31.4 (210)     18.1 (621)
 //      4     9.7 (152)      8.6 (153)      39.1 (211)     25.7 (625)     189 (1168): 5.6 TB/s
 //     32    20.8 (157)     19.8 (156)      83.7 (222)     69.0 (640)     549 (1261)
-//    173    98.5 (151)     54.7 (148)       396 (674)      187 (591)
+//    173    62.6 (151)     50.0 (148)       353 (674)      176 (591)
+//    300     113            99             615            350
 //    512     183 (303)      122 (208)       968 (1357)     434 (852): 40 TFLOP/s of the CUDA cores' 74
 //
 // The relative error against 64 bits is 2.9e-7 at K = 2048 and 5.7e-7 at 8192 (8.1e-7 and 1.6e-6 for one chain over K).
@@ -211,22 +212,23 @@ gemm_f32_few_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constan
     }
 }
 
-// Tiles of 16 RM rows x 128 columns.  Thread (ty, tx) owns rows ty + 16 i and columns tx + 8 j; the first thread also
+// Tiles of 16 RM rows x 8 CN columns.  Thread (ty, tx) owns rows ty + 16 i and columns tx + 8 j; the first thread also
 // loads (a fifth warp would leave 168 registers to a thread); the CTA's rank in its cluster is its run of K.
-template <int RM>
+template <int RM, int CN>
 __global__ void __launch_bounds__(128, 2)
 gemm_f32_tile_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUtensorMap ta, float* __restrict__ C,
                      int M, int N, int K, long long ldc) {
     constexpr int BM = 16 * RM;
-    constexpr uint32_t A_BYTES = BM * F32_BK * 4;
+    constexpr int BN = 8 * CN;
+    constexpr uint32_t A_BYTES = BM * F32_BK * 4, W_BYTES = BN * F32_BK * 4;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* w_ring = smem;
-    uint8_t* a_ring = smem + F32_TILE_STAGES * F32_W_BYTES;
+    uint8_t* a_ring = smem + F32_TILE_STAGES * W_BYTES;
     uint64_t* bars = (uint64_t*)(a_ring + F32_TILE_STAGES * A_BYTES);
     F32Ring ring{bars, bars + F32_TILE_STAGES, (volatile int*)(bars + 2 * F32_TILE_STAGES)};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = (int)(blockIdx.x / F32_SEGS) * F32_BN, m0 = (int)blockIdx.y * BM;
+    const int n0 = (int)(blockIdx.x / F32_SEGS) * BN, m0 = (int)blockIdx.y * BM;
     const int rank = (int)tc::cluster_ctarank();
     const int nkb = (K + F32_BK - 1) / F32_BK, run = (nkb + F32_SEGS - 1) / F32_SEGS;
     const int kb0 = min(nkb, rank * run), blocks = min(nkb, kb0 + run) - kb0;
@@ -241,8 +243,8 @@ gemm_f32_tile_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
     }
     __syncthreads();
     auto ask_w = [&](int b) {
-        tc::mbar_expect_tx(&ring.full[b % F32_TILE_STAGES], F32_W_BYTES + A_BYTES);
-        tc::tma_load_2d(w_ring + (b % F32_TILE_STAGES) * F32_W_BYTES, &tw, (kb0 + b) * F32_BK, n0, &ring.full[b % F32_TILE_STAGES]);
+        tc::mbar_expect_tx(&ring.full[b % F32_TILE_STAGES], W_BYTES + A_BYTES);
+        tc::tma_load_2d(w_ring + (b % F32_TILE_STAGES) * W_BYTES, &tw, (kb0 + b) * F32_BK, n0, &ring.full[b % F32_TILE_STAGES]);
     };
     auto ask_a = [&](int b) {
         tc::tma_load_2d(a_ring + (b % F32_TILE_STAGES) * A_BYTES, &ta, (kb0 + b) * F32_BK, m0, &ring.full[b % F32_TILE_STAGES]);
@@ -254,14 +256,14 @@ gemm_f32_tile_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
     for (int b = 0; b < asked; ++b) ask_a(b);
 
     const int tx = lane & 7, ty = warp * 4 + (lane >> 3);
-    float acc[RM][16];
+    float acc[RM][CN];
 #pragma unroll
     for (int i = 0; i < RM; ++i)
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < CN; ++j) acc[i][j] = 0.f;
     for (int b = 0; b < blocks; ++b) {
         if (!f32_landed<F32_TILE_STAGES>(ring, b)) break;
-        const uint8_t* wb = w_ring + (b % F32_TILE_STAGES) * F32_W_BYTES;
+        const uint8_t* wb = w_ring + (b % F32_TILE_STAGES) * W_BYTES;
         const uint8_t* ab = a_ring + (b % F32_TILE_STAGES) * A_BYTES;
 #pragma unroll 1
         for (int c = 0; c < F32_BK / 4; ++c) {
@@ -269,7 +271,7 @@ gemm_f32_tile_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
 #pragma unroll
             for (int i = 0; i < RM; ++i) a[i] = f32_block_read(ab, ty + 16 * i, c);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < CN; ++j) {
                 const float4 w = f32_block_read(wb, tx + 8 * j, c);
 #pragma unroll
                 for (int i = 0; i < RM; ++i) {
@@ -299,19 +301,19 @@ gemm_f32_tile_kernel(const __grid_constant__ CUtensorMap tw, const __grid_consta
     // nothing is left in flight when the ring takes the sums
     for (int b = max(0, asked - F32_TILE_STAGES); b < asked; ++b)
         tc::mbar_wait(&ring.full[b % F32_TILE_STAGES], (uint32_t)((b / F32_TILE_STAGES) & 1));
-    float* part = reinterpret_cast<float*>(smem);                // [row][128]: the ring is idle now
-    static_assert(BM * F32_BN * 4 <= F32_TILE_STAGES * (F32_W_BYTES + (int)A_BYTES), "the ring holds a tile of sums");
+    float* part = reinterpret_cast<float*>(smem);                // [row][BN]: the ring is idle now
+    static_assert(BM * BN * 4 <= F32_TILE_STAGES * ((int)W_BYTES + (int)A_BYTES), "the ring holds a tile of sums");
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < RM; ++i)
 #pragma unroll
-        for (int j = 0; j < 16; ++j) part[(ty + 16 * i) * F32_BN + tx + 8 * j] = acc[i][j];
+        for (int j = 0; j < CN; ++j) part[(ty + 16 * i) * BN + tx + 8 * j] = acc[i][j];
     tc::cluster_sync();
     // each CTA finishes BM / 8 of the tile's rows
     constexpr int ROWS = BM / F32_SEGS;
-    for (int e = threadIdx.x; e < ROWS * F32_BN; e += blockDim.x) {
-        const int m = rank * ROWS + e / F32_BN, c = e % F32_BN;
-        const uint32_t at = tc::smem_addr(part + m * F32_BN + c);
+    for (int e = threadIdx.x; e < ROWS * BN; e += blockDim.x) {
+        const int m = rank * ROWS + e / BN, c = e % BN;
+        const uint32_t at = tc::smem_addr(part + m * BN + c);
         float p[F32_SEGS], v = 0.f;
 #pragma unroll
         for (int s = 0; s < F32_SEGS; ++s) p[s] = tc::ld_cluster_f32(tc::map_to_rank(at, (uint32_t)s));
@@ -412,17 +414,40 @@ int gemm_f32(const float* a, const float* w, float* out, int M, int N, int K, lo
         FEW(8);
 #undef FEW
     }
-    // the row tile that leaves the fewest rows empty, the larger one of two equals
-    int rm = 8, best = (M + 127) / 128 * 128;
-    if ((M + 95) / 96 * 96 < best) { rm = 6; best = (M + 95) / 96 * 96; }
-    if ((M + 63) / 64 * 64 < best) { rm = 4; best = (M + 63) / 64 * 64; }
-    const dim3 grid((unsigned)tiles_n * F32_SEGS, (unsigned)(best / (16 * rm)));
+    // A round of clusters takes about 28 + outputs to a thread, whatever K (us at K = 2048, one round: 4 x 16 outputs 38, 6 x 16 50, 8 x 16 61,
+    // 8 x 12 48, 10 x 12 57, 11 x 12 62, 11 x 14 71), and 34 clusters of 8 run at once (more than 272 CTAs of two to an SM make a second
+    // round), so the tile with the least of rounds x (28 + outputs) is taken, one of 128 columns unless another has 6 % less (512 rows x 16384:
+    // 968 us in 8 x 16, 985 in 11 x 14, which the rule alone would prefer by 5 %): 173 rows x 3072 one round of 11 x 12 instead of two of
+    // 6 x 16 (62 against 98 us), x 16384 five of 11 x 14 instead of eight (353 against 396).  Every tile gives the same bits.
+    static const int shapes[][2] = {{8, 16}, {6, 16}, {4, 16}, {8, 12}, {10, 12}, {11, 12}, {11, 14}};
+    int rm = 8, cn = 16;
+    long long least = -1;
+    for (const auto& s : shapes) {
+        const long long clusters = (long long)((M + 16 * s[0] - 1) / (16 * s[0])) * ((N + 8 * s[1] - 1) / (8 * s[1]));
+        const long long cost = (clusters + 33) / 34 * (28 + s[0] * s[1]) * (s[1] == 16 ? 94 : 100);
+        if (least < 0 || cost < least) {
+            least = cost;
+            rm = s[0];
+            cn = s[1];
+        }
+    }
+    const dim3 grid((unsigned)((N + 8 * cn - 1) / (8 * cn)) * F32_SEGS, (unsigned)((M + 16 * rm - 1) / (16 * rm)));
     AP_REQUIRE(grid.y <= 65535, "gemm: %d rows exceed the grid of the CUDA-core kernel", M);
+    AP_REQUIRE(f32_make_map(&tw, w, N, K, ldw, 8 * cn), "gemm_f32: cannot encode the weight's tensor map");
     AP_REQUIRE(f32_make_map(&ta, a, M, K, lda, 16 * rm), "gemm_f32: cannot encode the rows' tensor map");
-    const size_t smem = F32_TILE_STAGES * (size_t)(F32_W_BYTES + 16 * rm * F32_BK * 4) + 2 * F32_TILE_STAGES * 8 + 16 + 1024;
-    if (rm == 8) return f32_launch(gemm_f32_tile_kernel<8>, grid, 128, smem, true, stream, tw, ta, out, M, N, K, ldc, 0);
-    if (rm == 6) return f32_launch(gemm_f32_tile_kernel<6>, grid, 128, smem, true, stream, tw, ta, out, M, N, K, ldc, 0);
-    return f32_launch(gemm_f32_tile_kernel<4>, grid, 128, smem, true, stream, tw, ta, out, M, N, K, ldc, 0);
+    const size_t smem = F32_TILE_STAGES * (size_t)((8 * cn + 16 * rm) * F32_BK * 4) + 2 * F32_TILE_STAGES * 8 + 16 + 1024;
+#define TILE(RM, CN) \
+    if (rm == RM && cn == CN) return f32_launch(gemm_f32_tile_kernel<RM, CN>, grid, 128, smem, true, stream, tw, ta, out, M, N, K, ldc, 0)
+    TILE(8, 16);
+    TILE(6, 16);
+    TILE(4, 16);
+    TILE(8, 12);
+    TILE(10, 12);
+    TILE(11, 12);
+    TILE(11, 14);
+#undef TILE
+    ap_set_error("gemm_f32: no kernel of %d x %d outputs", rm, cn);
+    return AP_ERR_UNSUPPORTED;
 }
 
 // 0 when every product here so far ran to its end; else the wait that expired (1 a free stage, 2 operands)
