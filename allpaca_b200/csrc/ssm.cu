@@ -349,6 +349,76 @@ AP_EXPORT int ap_ssm_scan(const float* xbc, long long ld_xbc, const float* dt_ra
     return AP_OK;
 }
 
+// ---- what surrounds the recurrence of a prompt's portions --------------------------------
+// A portion of many rows runs eight tokens at a time as linear attention (linear_attention.cu: queries C, keys B, values x,
+// written under dt, decayed by a number per head and token).  These two kernels are what that leaves: the numbers per head and token
+// ahead of it, the part of the input that bypasses the state behind it.  Both move a few MB (2048 rows of 32 heads of 64, with the two
+// kernels of linear_attention.cu 217 us; the chain above, token after token, 853).
+__global__ void __launch_bounds__(256)
+ssm_gates_kernel(const float* __restrict__ dt_raw, long long ld_dt, const float* __restrict__ dt_bias,
+                 const float* __restrict__ a_log, float* __restrict__ dt, float* __restrict__ decay, int T, int heads) {
+    ap_pdl_trigger();
+    ap_pdl_wait();
+    const size_t e = blockIdx.x * (size_t)256 + threadIdx.x;
+    if (e >= (size_t)T * heads) return;
+    const size_t t = e / heads;
+    const int h = (int)(e - t * heads);
+    const float v = ssm_softplus(dt_raw[t * ld_dt + h] + (dt_bias ? dt_bias[h] : 0.f));
+    dt[e] = v;
+    decay[e] = expf(-expf(a_log[h]) * v);
+}
+
+AP_EXPORT int ap_ssm_gates(const float* dt_raw, long long ld_dt, const float* dt_bias, const float* a_log, float* dt,
+                           float* decay, int T, int heads, cudaStream_t stream) {
+    AP_REQUIRE(T >= 0 && heads > 0 && ld_dt >= heads, "ssm_gates: bad sizes");
+    if (T == 0) return AP_OK;
+    const unsigned blocks = (unsigned)(((long long)T * heads + 255) / 256);
+    AP_CHECK_PDL_LAUNCH("ssm_gates", ap_launch_pdl(ssm_gates_kernel, dim3(blocks), dim3(256), 0, stream, dt_raw, ld_dt, dt_bias,
+                                                   a_log, dt, decay, T, heads));
+    return AP_OK;
+}
+
+// y[t, h, :] += d_skip[h] x[t, h, :]; VEC columns to a thread
+template <int VEC>
+__global__ void __launch_bounds__(256)
+ssm_skip_kernel(float* __restrict__ y, const float* __restrict__ x, long long ld_x, const float* __restrict__ d_skip, size_t n,
+                int inner, int vdim) {
+    ap_pdl_trigger();
+    ap_pdl_wait();
+    const size_t e = (blockIdx.x * (size_t)256 + threadIdx.x) * VEC;
+    if (e >= n) return;
+    const size_t t = e / inner;
+    const int c = (int)(e - t * inner);
+    const float d = d_skip[c / vdim];
+    const float* px = x + t * ld_x + c;
+    if constexpr (VEC == 4) {
+        float4 v = *reinterpret_cast<const float4*>(y + e);
+        const float4 u = *reinterpret_cast<const float4*>(px);
+        v.x = fmaf(d, u.x, v.x);
+        v.y = fmaf(d, u.y, v.y);
+        v.z = fmaf(d, u.z, v.z);
+        v.w = fmaf(d, u.w, v.w);
+        *reinterpret_cast<float4*>(y + e) = v;
+    } else {
+        y[e] = fmaf(d, *px, y[e]);
+    }
+}
+
+AP_EXPORT int ap_ssm_skip(float* y, const float* x, long long ld_x, const float* d_skip, int T, int heads, int vdim,
+                          cudaStream_t stream) {
+    AP_REQUIRE(T >= 0 && heads > 0 && vdim > 0 && ld_x >= (long long)heads * vdim, "ssm_skip: bad sizes");
+    if (T == 0) return AP_OK;
+    const int inner = heads * vdim;
+    const size_t n = (size_t)T * inner;
+    const bool vec = vdim % 4 == 0 && ld_x % 4 == 0 && ((((uintptr_t)y) | ((uintptr_t)x)) & 15) == 0;
+    const unsigned blocks = (unsigned)((n / (vec ? 4 : 1) + 255) / 256);
+    if (vec)
+        AP_CHECK_PDL_LAUNCH("ssm_skip", ap_launch_pdl(ssm_skip_kernel<4>, dim3(blocks), dim3(256), 0, stream, y, x, ld_x, d_skip, n, inner, vdim));
+    else
+        AP_CHECK_PDL_LAUNCH("ssm_skip", ap_launch_pdl(ssm_skip_kernel<1>, dim3(blocks), dim3(256), 0, stream, y, x, ld_x, d_skip, n, inner, vdim));
+    return AP_OK;
+}
+
 // ---- gate, then RMS norm per slice of the row -------------------------------------------
 // y: [T, inner] 32-bit; z: [T, ld_z] 32-bit gate (column 0 of the view); one warp per (row, part).
 template <typename TW, typename TO>

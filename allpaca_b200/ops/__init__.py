@@ -851,7 +851,7 @@ def check_kernel_status() -> None:
 
 from .mixers import (attention_window_bias, causal_conv, embed_sinusoid_norm, gated_group_rmsnorm,  # noqa: E402
                      head_project, latent_decode, latent_decode_takes, latent_gather, latent_prefill,
-                     latent_prefill_takes, latent_prepare, qk_norm_store, ssm_scan)
+                     latent_prefill_takes, latent_prepare, qk_norm_store, ssm_in_blocks, ssm_scan)
 from . import routed  # noqa: E402,F401
 from .routed import (gated_act, moe_combine, moe_down, moe_gate_up, moe_gather, moe_max_tiles, moe_products, moe_products_taken,  # noqa: E402
                      moe_rows_taken,

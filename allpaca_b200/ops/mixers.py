@@ -6,7 +6,7 @@ from typing import Optional
 
 import torch
 
-from . import AP_F32, KernelError, _check, call, core, dtype_code, stream_handle
+from . import AP_F32, KernelError, _check, call, core, dtype_code, recurrent, stream_handle
 
 
 def embed_sinusoid_norm(tokens: torch.Tensor, positions: torch.Tensor, table: torch.Tensor,
@@ -309,15 +309,28 @@ def causal_conv(inp: torch.Tensor, col0: int, weight: torch.Tensor, bias: Option
          positions.data_ptr(), state_slots.data_ptr(), out.data_ptr(), T, int(num_seqs), C, taps, stream_handle())
 
 
+def ssm_in_blocks(rows: int, num_seqs: int, heads: int) -> bool:
+    """Whether a step's state-space recurrence runs eight tokens at a time (four launches and a pass over its scratch, some 10 us)
+    and not token after token (0.4 to 0.7 us a row of the longest chain, more where the states fill the SMs).
+
+    Measured (one B200, us, token after token and eight at a time; states of 128 x 64 on 32 heads): 8 sequences of 4 rows 15
+    and 23, of 8 rows 23 and 24, of 12 32 and 27, of 32 76 and 37, of 256 569 and 207; one sequence of 16 rows 15 and 13, of 64 47 and 17, of 512
+    347 and 71; states of 64 x 64 on 16 heads: one sequence of 16 rows 8.5 and 10.9, of 64 26 and 14, 8 of 16 18 and 14."""
+    return rows > 24 * num_seqs or (rows > 8 * num_seqs and rows * heads >= 2048)
+
+
 def ssm_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torch.Tensor], a_log: torch.Tensor,
              d_skip: Optional[torch.Tensor], state: torch.Tensor, seq_start: torch.Tensor, positions: torch.Tensor,
              state_slots: torch.Tensor, y: torch.Tensor, num_seqs: int, heads: int, groups: int, state_size: int,
-             value_dim: int) -> None:
+             value_dim: int, workspace=None) -> None:
     """The recurrence of a selective state-space layer with one decay per head, all 32-bit:
     ``dt = softplus(dt_raw + dt_bias)``, ``S = exp(-exp(a_log) dt) S + dt B x^T``,
     ``y = S^T C + d_skip x``.  ``xbc [T, heads*vdim + 2*groups*N]`` holds x, B and C side by side;
     ``dt_raw [T, heads]`` may be a strided view; ``state [slots, heads, N, vdim]`` may be a strided
-    view of the slots' rows.  A sequence whose first row has position 0 starts from zero."""
+    view of the slots' rows.  A sequence whose first row has position 0 starts from zero.
+
+    With ``workspace`` (where the buffers between its kernels come from) a step whose sequences bring several rows on
+    average runs eight tokens at a time (:func:`linear_scan`); without it, token after token."""
     _check(xbc, "xbc", torch.float32, 2)
     _check(y, "y", torch.float32, 2)
     T = y.shape[0]
@@ -337,6 +350,17 @@ def ssm_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torch.Te
                 raise KernelError(f"ssm_scan: {n} must have one entry per head")
     for t, n in ((seq_start, "seq_start"), (positions, "positions"), (state_slots, "state_slots")):
         _check(t, n, torch.int32, 1)
+    if workspace is not None and ssm_in_blocks(T, num_seqs, heads):
+        gates = workspace.get("ssm_scan.gates", (2, T, heads), torch.float32)
+        call(core(), "ap_ssm_gates", dt_raw.data_ptr(), dt_raw.stride(0), dt_bias.data_ptr() if dt_bias is not None else 0,
+             a_log.data_ptr(), gates[0].data_ptr(), gates[1].data_ptr(), T, heads, stream_handle())
+        keys, queries = xbc[:, inner:inner + groups * state_size], xbc[:, inner + groups * state_size:]
+        recurrent.linear_scan(queries, keys, xbc[:, :inner], y, state, seq_start, positions, state_slots, num_seqs, heads, groups,
+                              state_size, value_dim, "head_ready", decay_head=gates[1], write_gate=gates[0], workspace=workspace)
+        if d_skip is not None:
+            call(core(), "ap_ssm_skip", y.data_ptr(), xbc.data_ptr(), xbc.stride(0), d_skip.data_ptr(), T, heads, value_dim,
+                 stream_handle())
+        return
     call(core(), "ap_ssm_scan", xbc.data_ptr(), xbc.stride(0), dt_raw.data_ptr(), dt_raw.stride(0),
          dt_bias.data_ptr() if dt_bias is not None else 0, a_log.data_ptr(),
          d_skip.data_ptr() if d_skip is not None else 0, state.data_ptr(), state.stride(0), seq_start.data_ptr(),

@@ -93,7 +93,7 @@ class Mamba2(Mixer):
         y = ws.get("mamba.y", (T, self.inner), torch.float32)
         ops.ssm_scan(xbc, proj[:, self.inner + self.conv_channels:], self.dt_bias, self.a_log, self.d_skip,
                      ssm_state, step.seq_start, step.positions, step.state_slots, y, S, self.heads, self.groups,
-                     self.N, self.vd)
+                     self.N, self.vd, workspace=ws if self.env.dtype == torch.bfloat16 else None)
         gated = ws.get("mamba.gated", (T, self.inner), self.env.dtype)
         ops.gated_group_rmsnorm(y, proj[:, :self.inner], self.norm_w, self.eps, gated, self.norm_groups)
         return self.out_proj.forward(gated, "mamba.o", "delta")
