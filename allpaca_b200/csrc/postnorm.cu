@@ -122,6 +122,81 @@ gated_postnorm_kernel(float* __restrict__ x, const int* __restrict__ rows, const
     }
 }
 
+// The same where a warp has one run of at most PN_RUNS 16-byte loads of a row (up to 4096 columns in up to eight groups) and the result
+// is one slice.  A step of few rows is a chain of latencies: here the weight and the gate's bias, which no kernel writes, are
+// asked for ahead of the kernel before, everything else at once, and the row waits in registers.  The sums are those of the kernel
+// above, in its order.  Measured (one B200): four requests on four layers of 2048 columns in four groups, nine such norms a step, prompts of 300 to
+// 1500 tokens and 24 new ones: 17.96 -> 17.63 ms.
+#define PN_RUNS 4
+template <typename TW, typename TO>
+__global__ void __launch_bounds__(PN_THREADS)
+gated_postnorm_rows_kernel(float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ delta,
+                           const float* __restrict__ gate, long long ld_gate, const float* __restrict__ gate_bias, float alpha,
+                           const TW* __restrict__ w, int groups, float eps, int update, TO* __restrict__ out, int H, int split,
+                           int chunk) {
+    __shared__ float ss_s[PN_WARPS];
+    ap_pdl_trigger();
+    const int r = blockIdx.x, u = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gw = H / groups, g = u / split, part = u - g * split;
+    const int c0 = g * gw + part * chunk + lane * 4, c1 = u < groups * split ? min(g * gw + (part + 1) * chunk, (g + 1) * gw) : 0;
+    float ww[PN_RUNS][4], b[PN_RUNS][4];
+#pragma unroll
+    for (int k = 0; k < PN_RUNS; ++k) {
+        const int c = c0 + 128 * k;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ww[k][i] = b[k][i] = 0.f;
+        if (c < c1) {
+            pn_load<4>(w + c, ww[k]);
+            if (gate && gate_bias) pn_load<4>(gate_bias + c, b[k]);
+        }
+    }
+    ap_pdl_wait();
+    const size_t t = rows ? (size_t)rows[r] : (size_t)r;
+    float* xr = x + t * H;
+    float v[PN_RUNS][4], d[PN_RUNS][4], e[PN_RUNS][4];
+#pragma unroll
+    for (int k = 0; k < PN_RUNS; ++k) {
+        const int c = c0 + 128 * k;
+        if (c < c1) {
+            pn_load<4>(xr + c, v[k]);
+            if (delta) pn_load<4>(delta + t * H + c, d[k]);
+            if (gate) pn_load<4>(gate + t * ld_gate + c, e[k]);
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < PN_RUNS; ++k) {
+        if (c0 + 128 * k < c1) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                v[k][i] *= alpha;
+                if (delta) {
+                    if (gate) d[k][i] *= 1.0f / (1.0f + expf(-(e[k][i] + b[k][i])));
+                    v[k][i] += d[k][i];
+                }
+                ss = fmaf(v[k][i], v[k][i], ss);
+            }
+        }
+    }
+    ss = ap_warp_sum(ss);
+    if (lane == 0) ss_s[u] = ss;
+    __syncthreads();
+    float total = 0.f;
+    if (c1 > 0)
+        for (int j = 0; j < split; ++j) total += ss_s[g * split + j];
+    const float inv = 1.0f / sqrtf(total / (float)gw + eps);
+#pragma unroll
+    for (int k = 0; k < PN_RUNS; ++k) {
+        const int c = c0 + 128 * k;
+        if (c < c1) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[k][i] = v[k][i] * inv * ww[k][i];
+            if (update) pn_store<4>(xr + c, v[k]);
+            if (out) pn_store<4>(out + (size_t)r * H + c, v[k]);
+        }
+    }
+}
+
 AP_EXPORT int ap_gated_postnorm(float* x, const int* rows, int R, const float* delta, int S, long long slice_stride,
                                 const float* gate, long long ld_gate, const float* gate_bias, float alpha,
                                 const void* w, int w_dtype, int groups, float eps, int update, void* out,
@@ -155,7 +230,16 @@ AP_EXPORT int ap_gated_postnorm(float* x, const int* rows, int R, const float* d
                                                             gate_bias, alpha, (const TW*)w, groups, eps, update,    \
                                                             (TO*)out, H, split, chunk));                            \
     } while (0)
-#define LAUNCH(TW, TO) do { if (vec) LAUNCH_V(TW, TO, 4); else LAUNCH_V(TW, TO, 1); } while (0)
+    const bool registers = vec && groups * split <= PN_WARPS && chunk <= 128 * PN_RUNS && (delta == nullptr || S == 1);
+#define LAUNCH(TW, TO)                                                                                              \
+    do {                                                                                                            \
+        if (registers)                                                                                              \
+            AP_CHECK_PDL_LAUNCH("gated_postnorm", ap_launch_pdl(gated_postnorm_rows_kernel<TW, TO>, dim3((unsigned)R), dim3(PN_THREADS), \
+                                                                0, stream, x, rows, delta, gate, ld_gate, gate_bias, alpha, \
+                                                                (const TW*)w, groups, eps, update, (TO*)out, H, split, chunk)); \
+        else if (vec) LAUNCH_V(TW, TO, 4);                                                                          \
+        else LAUNCH_V(TW, TO, 1);                                                                                   \
+    } while (0)
     const int od = out ? out_dtype : AP_F32;
     if (w_dtype == AP_F32 && od == AP_F32) LAUNCH(float, float);
     else if (w_dtype == AP_F32 && od == AP_BF16) LAUNCH(float, bf16);

@@ -1,0 +1,44 @@
+"""The norm after a gated sum where a row waits in registers: runs that fill a warp's loads and do not, groups of one to eight warps'
+parts and parts that are empty, one step over the widest row, with and without a result, a gate and its bias, chosen rows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def want(x, w, groups, eps, alpha, delta, gate, bias):
+    v = alpha * x.double()
+    if delta is not None:
+        d = delta.double()
+        if gate is not None:
+            d = d * torch.sigmoid(gate.double() + (bias.double() if bias is not None else 0.0))
+        v = v + d
+    v = v.reshape(v.shape[0], groups, -1)
+    return (v / torch.sqrt((v * v).mean(-1, keepdim=True) + eps)).flatten(1) * w.double()
+
+
+@pytest.mark.parametrize("W, groups", [(4, 1), (24, 3), (128, 8), (512, 1), (1000, 2), (1020, 5), (2048, 4), (4096, 1), (4096, 8), (4100, 1)])
+@pytest.mark.parametrize("form", ["gate", "no gate", "no result"])
+def test_rows_in_registers(W, groups, form):
+    from allpaca_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(W + groups)
+    T, eps, alpha = 5, 1e-6, 1.7
+    x, delta, gate = (torch.randn(T, W, generator=g, device="cuda") for _ in range(3))
+    wide = torch.zeros(T, W + 8, device="cuda")
+    wide[:, :W] = gate
+    w, bias = 1.0 + 0.2 * torch.randn(W, generator=g, device="cuda"), torch.randn(W, generator=g, device="cuda")
+    kw = {"alpha": alpha}
+    if form != "no result":
+        kw["delta"] = delta.unsqueeze(0)
+    if form == "gate":
+        kw.update(gate=wide[:, :W], gate_bias=bias)
+    ref = want(x, w, groups, eps, alpha, delta if form != "no result" else None, gate if form == "gate" else None, bias)
+    got, out = x.clone(), torch.empty(T, W, dtype=torch.bfloat16, device="cuda")
+    ops.gated_postnorm(got, w, groups, eps, copy=out, **kw)
+    assert float((got.double() - ref).abs().max()) <= 4e-6 * float(ref.abs().max())          # some 20 roundings of 2^-24
+    assert torch.equal(out, got.bfloat16())
+    if form == "no result":
+        picked, rows = torch.empty(2, W, device="cuda"), torch.tensor([3, 1], dtype=torch.int32, device="cuda")
+        before = x.clone()
+        ops.gated_postnorm(x, w, groups, eps, alpha=alpha, rows=rows, out=picked)
+        assert torch.equal(x, before) and torch.equal(picked, got[[3, 1]])
