@@ -18,7 +18,7 @@ def want(x, w, groups, eps, alpha, delta, gate, bias):
 
 
 @pytest.mark.parametrize("W, groups", [(4, 1), (24, 3), (128, 8), (512, 1), (1000, 2), (1020, 5), (2048, 4), (4096, 1), (4096, 8), (4100, 1)])
-@pytest.mark.parametrize("form", ["gate", "no gate", "no result"])
+@pytest.mark.parametrize("form", ["gate", "two slices", "no gate", "no result"])
 def test_rows_in_registers(W, groups, form):
     from allpaca_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(W + groups)
@@ -30,9 +30,13 @@ def test_rows_in_registers(W, groups, form):
     kw = {"alpha": alpha}
     if form != "no result":
         kw["delta"] = delta.unsqueeze(0)
-    if form == "gate":
+    if form == "two slices":
+        other = torch.randn(T, W, generator=g, device="cuda")
+        kw["delta"] = torch.stack([delta, other])
+        delta = delta + other
+    if form in ("gate", "two slices"):
         kw.update(gate=wide[:, :W], gate_bias=bias)
-    ref = want(x, w, groups, eps, alpha, delta if form != "no result" else None, gate if form == "gate" else None, bias)
+    ref = want(x, w, groups, eps, alpha, delta if form != "no result" else None, gate if form in ("gate", "two slices") else None, bias)
     got, out = x.clone(), torch.empty(T, W, dtype=torch.bfloat16, device="cuda")
     ops.gated_postnorm(got, w, groups, eps, copy=out, **kw)
     assert float((got.double() - ref).abs().max()) <= 4e-6 * float(ref.abs().max())          # some 20 roundings of 2^-24
