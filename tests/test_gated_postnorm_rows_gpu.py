@@ -46,3 +46,24 @@ def test_rows_in_registers(W, groups, form):
         before = x.clone()
         ops.gated_postnorm(x, w, groups, eps, alpha=alpha, rows=rows, out=picked)
         assert torch.equal(x, before) and torch.equal(picked, got[[3, 1]])
+
+
+@pytest.mark.parametrize("W, groups", [(4, 1), (1020, 5), (2048, 4), (4096, 8)])
+@pytest.mark.parametrize("slices", [1, 2])
+@pytest.mark.parametrize("gated", ["bias", "gate", None])
+def test_bits_of_the_general_kernel(W, groups, slices, gated):
+    """Slices of zeros behind the same sums change nothing but the kernel: more than two of them take the general one."""
+    from allpaca_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(W + slices)
+    T = 9
+    x, gate = (torch.randn(T, W, generator=g, device="cuda") for _ in range(2))
+    delta = torch.zeros(4, T, W, device="cuda")
+    delta[:slices] = torch.randn(slices, T, W, generator=g, device="cuda")
+    w, bias = 1.0 + 0.2 * torch.randn(W, generator=g, device="cuda"), torch.randn(W, generator=g, device="cuda")
+    results = []
+    for n in (slices, 4):
+        got = x.clone()
+        ops.gated_postnorm(got, w, groups, 1e-6, alpha=1.7, delta=delta[:n], gate=gate if gated else None,
+                           gate_bias=bias if gated == "bias" else None)
+        results.append(got)
+    assert torch.equal(*results)
