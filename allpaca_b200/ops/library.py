@@ -131,8 +131,8 @@ _CORE_SIGNATURES = {
     #                    in_w, w, eps, update, out, out_dtype, streams, H, stream)
     "ap_stream_norm": [_P, _P, _I, _P, _I, _L, _P, _P, _F, _F, _P, _P, _P, _P, _F, _I, _P, _I, _I, _I, _P],
     # int ap_gated_postnorm(x, rows, R, delta, S, slice_stride, gate, ld_gate, gate_bias, alpha, w, w_dtype, groups,
-    #                       eps, update, out, out_dtype, H, stream)
-    "ap_gated_postnorm": [_P, _P, _I, _P, _I, _L, _P, _L, _P, _F, _P, _I, _I, _F, _I, _P, _I, _I, _P],
+    #                       eps, update, out, out_dtype, H, settled, stream)
+    "ap_gated_postnorm": [_P, _P, _I, _P, _I, _L, _P, _L, _P, _F, _P, _I, _I, _F, _I, _P, _I, _I, _I, _P],
     # int ap_gated_row_add(delta, other, h, h_dtype, g, g_dtype, T, H, stream)
     "ap_gated_row_add": [_P, _P, _P, _I, _P, _I, _I, _I, _P],
     # int ap_bias_act(in, in_dtype, bias, out, out_dtype, T, N, act, stream)

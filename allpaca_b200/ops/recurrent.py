@@ -173,14 +173,16 @@ def head_norm_gate(y: torch.Tensor, gate: torch.Tensor, weight: Optional[torch.T
 def gated_postnorm(x: torch.Tensor, weight: torch.Tensor, groups: int, eps: float, alpha: float = 1.0,
                    delta: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
                    gate_bias: Optional[torch.Tensor] = None, copy: Optional[torch.Tensor] = None,
-                   rows: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> None:
+                   rows: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None, settled: bool = False) -> None:
     """The norm after a sum: ``v = alpha * x + sigmoid(gate + gate_bias) * sum(delta)``, then every one of the
     ``groups`` equal runs of ``v`` over its own ``sqrt(mean(run^2) + eps)``, times ``weight``; all 32-bit.
 
     Without ``rows``: ``x`` (32-bit ``[T, H]``) is overwritten with the result, and ``copy`` (optional, any type)
     receives it too.  With ``rows`` (int32 indices) or ``out`` alone: the chosen (or all) rows are normed into
     ``out`` and ``x`` stays.  ``delta``: 32-bit partial sums ``[S, T, H]`` or ``[T, H]``; ``gate``: 32-bit ``[T, H]``
-    raw (may be a run of columns of a wider matrix), ``gate_bias [H]``."""
+    raw (may be a run of columns of a wider matrix), ``gate_bias [H]``.  ``settled``: no kernel that may still be running
+    writes ``weight`` or ``gate_bias`` (a loaded model's are so); the kernel may then read them before the one ahead of it has
+    ended."""
     _check(x, "x", torch.float32, 2)
     _check(weight, "weight", dims=1)
     T, H = x.shape
@@ -215,7 +217,7 @@ def gated_postnorm(x: torch.Tensor, weight: torch.Tensor, groups: int, eps: floa
          gptr, gld, gate_bias.data_ptr() if gate_bias is not None else 0, float(alpha), weight.data_ptr(),
          dtype_code(weight.dtype), int(groups), float(eps), 1 if update else 0,
          target.data_ptr() if target is not None else 0, dtype_code(target.dtype) if target is not None else AP_F32,
-         H, stream_handle())
+         H, 1 if settled else 0, stream_handle())
 
 
 def gated_row_add(delta: torch.Tensor, other: torch.Tensor, h: torch.Tensor, g: torch.Tensor) -> None:

@@ -146,10 +146,10 @@ class GroupRMSNorm(Norm):
         if delta is not None and rows is None:
             ops.residual_add(x, delta)
             delta = None
-        ops.gated_postnorm(x, self.weight, self.groups, self.eps, delta=delta, rows=rows, out=out)
+        ops.gated_postnorm(x, self.weight, self.groups, self.eps, delta=delta, rows=rows, out=out, settled=True)
 
     def gated_sum(self, x, delta, gate, gate_bias, alpha: float, copy=None) -> None:
         """``x <- norm(alpha * x + sigmoid(gate + gate_bias) * sum(delta))`` in place on the 32-bit stream;
         ``copy`` (optional) receives the new rows in its own type."""
         ops.gated_postnorm(x, self.weight, self.groups, self.eps, alpha=alpha, delta=delta, gate=gate,
-                           gate_bias=gate_bias, copy=copy)
+                           gate_bias=gate_bias, copy=copy, settled=True)

@@ -67,3 +67,22 @@ def test_bits_of_the_general_kernel(W, groups, slices, gated):
                            gate_bias=bias if gated == "bias" else None)
         results.append(got)
     assert torch.equal(*results)
+
+
+def test_weight_and_bias_of_the_kernel_before():
+    """A weight and a gate's bias that the kernel right ahead writes, one that lets the next kernel start early, are read as that one
+    leaves them, unless the caller says that nothing in flight writes them."""
+    from allpaca_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(3)
+    T, W, rows = 4, 2048, 2048                               # a long kernel before: many rows, the vectors among its last
+    x, delta, gate = (torch.randn(T, W, generator=g, device="cuda") for _ in range(3))
+    source, ones = torch.randn(rows, W, generator=g, device="cuda"), torch.ones(W, device="cuda")
+    for _ in range(20):
+        made = torch.full((rows, W), float("nan"), device="cuda")
+        got, want = x.clone(), x.clone()
+        torch.cuda.synchronize()
+        ops.gated_postnorm(source, ones, 4, 1e-6, out=made)
+        ops.gated_postnorm(got, made[-1], 4, 1e-6, delta=delta, gate=gate, gate_bias=made[-2])
+        torch.cuda.synchronize()
+        ops.gated_postnorm(want, made[-1], 4, 1e-6, delta=delta, gate=gate, gate_bias=made[-2], settled=True)
+        assert torch.equal(got, want)
