@@ -243,7 +243,7 @@ AP_EXPORT int ap_gated_postnorm(float* x, const int* rows, int R, const float* d
         if (registers)                                                                                              \
             AP_CHECK_PDL_LAUNCH("gated_postnorm", ap_launch_pdl(gated_postnorm_rows_kernel<TW, TO>, dim3((unsigned)R), dim3(PN_THREADS), \
                                                                 0, stream, x, rows, delta, \
-                                                                S == 2 ? delta + slice_stride : (const float*)nullptr, gate, ld_gate, gate_bias, alpha, \
+                                                                delta != nullptr && S == 2 ? delta + slice_stride : (const float*)nullptr, gate, ld_gate, gate_bias, alpha, \
                                                                 (const TW*)w, groups, eps, update, (TO*)out, H, split, chunk, settled)); \
         else if (vec) LAUNCH_V(TW, TO, 4);                                                                          \
         else LAUNCH_V(TW, TO, 1);                                                                                   \

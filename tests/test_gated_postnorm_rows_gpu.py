@@ -86,3 +86,14 @@ def test_weight_and_bias_of_the_kernel_before():
         torch.cuda.synchronize()
         ops.gated_postnorm(want, made[-1], 4, 1e-6, delta=delta, gate=gate, gate_bias=made[-2], settled=True)
         assert torch.equal(got, want)
+
+
+def test_slices_of_no_sums():
+    """At the C entry: no sums to add, and a count of slices all the same."""
+    from allpaca_b200 import ops
+    x, w = torch.randn(3, 512, device="cuda"), torch.ones(512, device="cuda")
+    want = x.clone()
+    ops.gated_postnorm(want, w, 4, 1e-6, alpha=1.7)
+    ops.call(ops.core(), "ap_gated_postnorm", x.data_ptr(), 0, 3, 0, 2, x.numel(), 0, 0, 0, 1.7, w.data_ptr(),
+             ops.dtype_code(w.dtype), 4, 1e-6, 1, 0, ops.AP_F32, 512, 0, ops.stream_handle())
+    assert torch.equal(x, want)
