@@ -237,7 +237,12 @@ AP_EXPORT int ap_gated_postnorm(float* x, const int* rows, int R, const float* d
                                                             gate_bias, alpha, (const TW*)w, groups, eps, update,    \
                                                             (TO*)out, H, split, chunk));                            \
     } while (0)
-    const bool registers = vec && groups * split <= PN_WARPS && chunk <= 128 * PN_RUNS && (delta == nullptr || S <= 2);
+    // The row in registers takes 122 of them a thread, two CTAs to an SM: as long as all rows run at once it is the faster one (296 rows under a
+    // gate, us, general kernel and this one: 512 columns 2.8 and 2.3, 2048 5.2 and 4.3, 4096 8.1 and 6.7), beyond the general kernel, six CTAs to an SM, mostly
+    // (297 rows of 2048 5.5 and 6.1, 1024 10.6 and 12.9, 2048 16.7 and 22.3; 2048 rows of 512 9.6 and 16.5), but for two slices of the widest
+    // rows (1024 rows of 4096 23.5 and 20.7, 2048 39.2 and 36.0; 768 15.3 and 16.9).
+    const bool registers = vec && groups * split <= PN_WARPS && chunk <= 128 * PN_RUNS && (delta == nullptr || S <= 2) &&
+                           (R <= 2 * 148 || (R >= 1024 && chunk > 128 * (PN_RUNS - 1) && delta != nullptr && S == 2));
 #define LAUNCH(TW, TO)                                                                                              \
     do {                                                                                                            \
         if (registers)                                                                                              \

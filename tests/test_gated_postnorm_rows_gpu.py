@@ -97,3 +97,20 @@ def test_slices_of_no_sums():
     ops.call(ops.core(), "ap_gated_postnorm", x.data_ptr(), 0, 3, 0, 2, x.numel(), 0, 0, 0, 1.7, w.data_ptr(),
              ops.dtype_code(w.dtype), 4, 1e-6, 1, 0, ops.AP_F32, 512, 0, ops.stream_handle())
     assert torch.equal(x, want)
+
+
+@pytest.mark.parametrize("W, groups, slices", [(512, 1, 1), (2048, 4, 2), (4096, 8, 2)])
+@pytest.mark.parametrize("T", [296, 297, 1023, 1024])
+def test_rows_around_the_change_of_kernels(W, groups, slices, T):
+    """As many rows as run at once and one more, and as many as take two slices of wide rows back: each row has the bits it has alone."""
+    from allpaca_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(T + W)
+    x, gate = (torch.randn(T, W, generator=g, device="cuda") for _ in range(2))
+    delta = torch.randn(slices, T, W, generator=g, device="cuda")
+    w, bias = 1.0 + 0.2 * torch.randn(W, generator=g, device="cuda"), torch.randn(W, generator=g, device="cuda")
+    got = x.clone()
+    ops.gated_postnorm(got, w, groups, 1e-6, alpha=1.7, delta=delta, gate=gate, gate_bias=bias)
+    for r in (0, T // 2, T - 1):
+        one = x[r:r + 1].clone()
+        ops.gated_postnorm(one, w, groups, 1e-6, alpha=1.7, delta=delta[:, r:r + 1].contiguous(), gate=gate[r:r + 1], gate_bias=bias)
+        assert torch.equal(one, got[r:r + 1])
