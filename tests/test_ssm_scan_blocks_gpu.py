@@ -61,3 +61,36 @@ def test_portions_of_many_rows(Hh, E, N, G, bare):
                                     torch.zeros(Hh).double() if bare else d_skip.double()).reshape(-1, inner)
         # the tolerance of the recurrence token after token (test_viresun_kernels_gpu.py)
         assert float((torch.cat(got[i]).double() - want).abs().max()) <= 2e-5 * float(want.abs().max()), i
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["value", "key", "query", "step"])
+def test_rows_before_one_that_is_not_finite(where, value):
+    """A token whose numbers are not finite leaves every earlier row of its portion as it is, those of the same eight among them, and
+    the other sequences; the recurrence token after token says which rows those are."""
+    from allpaca_b200 import ops
+    g = torch.Generator().manual_seed(5)
+    Hh, E, N = 4, 32, 64
+    inner, lengths, bad = Hh * E, [61, 40], 29
+    xbc = torch.randn(sum(lengths), inner + 2 * N, generator=g)
+    dt = torch.randn(sum(lengths), Hh, generator=g)
+    if where == "step":
+        dt[bad, 1] = value
+    else:
+        xbc[bad, {"value": 3, "key": inner + 5, "query": inner + N + 5}[where]] = value
+    a_log, d_skip = torch.log(0.02 + 0.3 * torch.rand(Hh, generator=g)), torch.randn(Hh, generator=g)
+    pos = torch.cat([torch.arange(n) for n in lengths]).int().to(DEV)
+    assert ops.ssm_in_blocks(sum(lengths), 2, Hh)
+    results = []
+    for ws in (None, Workspace(torch.device(DEV))):
+        state = torch.zeros(2, Hh, N, E, device=DEV)
+        y = torch.empty(sum(lengths), inner, device=DEV)
+        ops.ssm_scan(xbc.to(DEV), dt.to(DEV), None, a_log.to(DEV), d_skip.to(DEV), state, i32([0, 61, 101]), pos, i32([0, 1]), y, 2,
+                     Hh, 1, N, E, workspace=ws)
+        results.append((y, state))
+    (chain, chain_state), (blocks, blocks_state) = results
+    for want, got in ((chain, blocks), (chain_state, blocks_state)):
+        finite = torch.isfinite(want)
+        assert torch.equal(torch.isfinite(got), finite)
+        assert float((got - want)[finite].abs().max()) <= 2e-5 * float(want[finite].abs().max())
+    assert bool(torch.isfinite(blocks[:bad]).all()) and not bool(torch.isfinite(blocks[bad]).all())
