@@ -378,16 +378,17 @@ AP_EXPORT int ap_ssm_gates(const float* dt_raw, long long ld_dt, const float* dt
     return AP_OK;
 }
 
-// y[t, h, :] += d_skip[h] x[t, h, :]; VEC columns to a thread
+// y[t, h, :] += d_skip[h] x[t, h, :] in the sequences' rows, the others are left as they are; VEC columns to a thread
 template <int VEC>
 __global__ void __launch_bounds__(256)
-ssm_skip_kernel(float* __restrict__ y, const float* __restrict__ x, long long ld_x, const float* __restrict__ d_skip, size_t n,
-                int inner, int vdim) {
+ssm_skip_kernel(float* __restrict__ y, const float* __restrict__ x, long long ld_x, const float* __restrict__ d_skip,
+                const int* __restrict__ seq_start, int nseq, size_t n, int inner, int vdim) {
     ap_pdl_trigger();
     ap_pdl_wait();
     const size_t e = (blockIdx.x * (size_t)256 + threadIdx.x) * VEC;
     if (e >= n) return;
     const size_t t = e / inner;
+    if ((long long)t < seq_start[0] || (long long)t >= seq_start[nseq]) return;
     const int c = (int)(e - t * inner);
     const float d = d_skip[c / vdim];
     const float* px = x + t * ld_x + c;
@@ -404,18 +405,20 @@ ssm_skip_kernel(float* __restrict__ y, const float* __restrict__ x, long long ld
     }
 }
 
-AP_EXPORT int ap_ssm_skip(float* y, const float* x, long long ld_x, const float* d_skip, int T, int heads, int vdim,
-                          cudaStream_t stream) {
-    AP_REQUIRE(T >= 0 && heads > 0 && vdim > 0 && ld_x >= (long long)heads * vdim, "ssm_skip: bad sizes");
-    if (T == 0) return AP_OK;
+AP_EXPORT int ap_ssm_skip(float* y, const float* x, long long ld_x, const float* d_skip, const int* seq_start, int T, int nseq,
+                          int heads, int vdim, cudaStream_t stream) {
+    AP_REQUIRE(T >= 0 && nseq >= 0 && heads > 0 && vdim > 0 && ld_x >= (long long)heads * vdim, "ssm_skip: bad sizes");
+    if (T == 0 || nseq == 0) return AP_OK;
     const int inner = heads * vdim;
     const size_t n = (size_t)T * inner;
     const bool vec = vdim % 4 == 0 && ld_x % 4 == 0 && ((((uintptr_t)y) | ((uintptr_t)x)) & 15) == 0;
     const unsigned blocks = (unsigned)((n / (vec ? 4 : 1) + 255) / 256);
     if (vec)
-        AP_CHECK_PDL_LAUNCH("ssm_skip", ap_launch_pdl(ssm_skip_kernel<4>, dim3(blocks), dim3(256), 0, stream, y, x, ld_x, d_skip, n, inner, vdim));
+        AP_CHECK_PDL_LAUNCH("ssm_skip", ap_launch_pdl(ssm_skip_kernel<4>, dim3(blocks), dim3(256), 0, stream, y, x, ld_x, d_skip,
+                                                     seq_start, nseq, n, inner, vdim));
     else
-        AP_CHECK_PDL_LAUNCH("ssm_skip", ap_launch_pdl(ssm_skip_kernel<1>, dim3(blocks), dim3(256), 0, stream, y, x, ld_x, d_skip, n, inner, vdim));
+        AP_CHECK_PDL_LAUNCH("ssm_skip", ap_launch_pdl(ssm_skip_kernel<1>, dim3(blocks), dim3(256), 0, stream, y, x, ld_x, d_skip,
+                                                     seq_start, nseq, n, inner, vdim));
     return AP_OK;
 }
 

@@ -75,9 +75,10 @@ _CORE_SIGNATURES = {
     # int ap_causal_conv(in, ld_in, col0, in_bias, w, bias, act, state, state_stride, seq_start, positions,
     #                    state_slots, out, T, nseq, C, taps, stream)
     "ap_causal_conv": [_P, _L, _I, _P, _P, _P, _I, _P, _L, _P, _P, _P, _P, _I, _I, _I, _I, _P],
-    # int ap_ssm_gates(dt_raw, ld_dt, dt_bias, a_log, dt, decay, T, heads, stream); ap_ssm_skip(y, x, ld_x, d_skip, T, heads, vdim, stream)
+    # int ap_ssm_gates(dt_raw, ld_dt, dt_bias, a_log, dt, decay, T, heads, stream); ap_ssm_skip(y, x, ld_x, d_skip, seq_start, T, nseq, heads,
+    #                                                                                                  vdim, stream)
     "ap_ssm_gates": [_P, _L, _P, _P, _P, _P, _I, _I, _P],
-    "ap_ssm_skip": [_P, _P, _L, _P, _I, _I, _I, _P],
+    "ap_ssm_skip": [_P, _P, _L, _P, _P, _I, _I, _I, _I, _P],
     # int ap_ssm_scan(xbc, ld_xbc, dt_raw, ld_dt, dt_bias, a_log, d_skip, state, state_stride, seq_start, positions,
     #                 state_slots, y, T, nseq, heads, groups, N, vdim, stream)
     "ap_ssm_scan": [_P, _L, _P, _L, _P, _P, _P, _P, _L, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _P],

@@ -358,8 +358,8 @@ def ssm_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torch.Te
         recurrent.linear_scan(queries, keys, xbc[:, :inner], y, state, seq_start, positions, state_slots, num_seqs, heads, groups,
                               state_size, value_dim, "head_ready", decay_head=gates[1], write_gate=gates[0], workspace=workspace)
         if d_skip is not None:
-            call(core(), "ap_ssm_skip", y.data_ptr(), xbc.data_ptr(), xbc.stride(0), d_skip.data_ptr(), T, heads, value_dim,
-                 stream_handle())
+            call(core(), "ap_ssm_skip", y.data_ptr(), xbc.data_ptr(), xbc.stride(0), d_skip.data_ptr(), seq_start.data_ptr(), T,
+                 int(num_seqs), heads, value_dim, stream_handle())
         return
     call(core(), "ap_ssm_scan", xbc.data_ptr(), xbc.stride(0), dt_raw.data_ptr(), dt_raw.stride(0),
          dt_bias.data_ptr() if dt_bias is not None else 0, a_log.data_ptr(),

@@ -94,3 +94,23 @@ def test_rows_before_one_that_is_not_finite(where, value):
         assert torch.equal(torch.isfinite(got), finite)
         assert float((got - want)[finite].abs().max()) <= 2e-5 * float(want[finite].abs().max())
     assert bool(torch.isfinite(blocks[:bad]).all()) and not bool(torch.isfinite(blocks[bad]).all())
+
+
+@pytest.mark.parametrize("E", [32, 5])
+def test_rows_of_no_sequence(E):
+    """Rows ahead of the first sequence's and behind the last one's stay as they are, in blocks as token after token."""
+    from allpaca_b200 import ops
+    g = torch.Generator().manual_seed(6)
+    Hh, N, T, first, last = 4, 16, 130, 3, 101
+    xbc, dt = torch.randn(T, Hh * E + 2 * N, generator=g).to(DEV), torch.randn(T, Hh, generator=g).to(DEV)
+    a_log, d_skip = torch.randn(Hh, generator=g).to(DEV), torch.randn(Hh, generator=g).to(DEV)
+    pos = (torch.arange(T) - first).int().to(DEV)
+    assert ops.ssm_in_blocks(T, 1, Hh)
+    results = []
+    for ws in (None, Workspace(torch.device(DEV))):
+        y = torch.full((T, Hh * E), 7.0, device=DEV)
+        ops.ssm_scan(xbc, dt, None, a_log, d_skip, torch.zeros(1, Hh, N, E, device=DEV), i32([first, last]), pos, i32([0]), y, 1, Hh, 1,
+                     N, E, workspace=ws)
+        results.append(y)
+    assert all(bool((y[:first] == 7.0).all()) and bool((y[last:] == 7.0).all()) for y in results)
+    assert float((results[0] - results[1]).abs().max()) <= 2e-5 * float(results[0].abs().max())
