@@ -309,28 +309,38 @@ def causal_conv(inp: torch.Tensor, col0: int, weight: torch.Tensor, bias: Option
          positions.data_ptr(), state_slots.data_ptr(), out.data_ptr(), T, int(num_seqs), C, taps, stream_handle())
 
 
-def ssm_in_blocks(rows: int, num_seqs: int, heads: int) -> bool:
-    """Whether a step's state-space recurrence runs eight tokens at a time (four launches and a pass over its scratch, some 10 us)
-    and not token after token (0.4 to 0.7 us a row of the longest chain, more where the states fill the SMs).
+def ssm_in_blocks(rows: int, num_seqs: int, heads: int, state_size: int = 128, value_dim: int = 64, longest: int = 0) -> bool:
+    """Whether a step's state-space recurrence runs eight tokens at a time (four launches and a pass over its scratch, some 10 us,
+    and a share for each block and each state) and not token after token (a chain as long as the ``longest`` sequence's rows, 0.2 to 0.7 us a
+    row, and a share for each row of each state).  ``longest`` 0: not known, the sequences are taken for equally long.
 
-    Measured (one B200, us, token after token and eight at a time; states of 128 x 64 on 32 heads): 8 sequences of 4 rows 15
-    and 23, of 8 rows 23 and 24, of 12 32 and 27, of 32 76 and 37, of 256 569 and 207; one sequence of 16 rows 15 and 13, of 64 47 and 17, of 512
-    347 and 71; states of 64 x 64 on 16 heads: one sequence of 16 rows 8.5 and 10.9, of 64 26 and 14, 8 of 16 18 and 14."""
-    return rows > 24 * num_seqs or (rows > 8 * num_seqs and rows * heads >= 2048)
+    Of 615 steps measured (up to 200 single rows beside one to eight portions of 2 to 512, 2 to 64 equal portions, 4 to 64 heads, states of 16 x 32 to
+    128 x 64) 581 take the faster way or one within 3 % of it, and none goes more than 7 % above token after token.  On one B200, us, token after token and eight at a time, states of 128 x 64 on 32
+    heads: one sequence of 12 rows 12.3 and 12.6, of 16 14.9 and 12.6, of 512 355 and 71; 8 of 4 rows 15 and 22, of 8 23.2 and 22.9, of 32 76 and 37;
+    a portion of 24 rows beside 16 single ones 41 and 48, of 32 49 and 49; of 256 beside 40 314 and 130, beside 63 335 and 179, beside 200 482
+    and 520."""
+    if num_seqs <= 0 or rows <= 2 * num_seqs:                # (linear_scan goes token after token there)
+        return False
+    longest = max(longest, -(-rows // num_seqs))
+    size = heads * state_size * value_dim / 2 ** 18
+    portions = (rows - num_seqs) / (longest - 1)             # as many of the longest as the rows allow, single rows beside them
+    blocks = num_seqs - portions + portions * -(-longest // 8)
+    return min(0.4, 0.2 + state_size / 320) * longest + 0.4 * rows * size > 10 + (blocks + 0.6 * num_seqs) * size
 
 
 def ssm_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torch.Tensor], a_log: torch.Tensor,
              d_skip: Optional[torch.Tensor], state: torch.Tensor, seq_start: torch.Tensor, positions: torch.Tensor,
              state_slots: torch.Tensor, y: torch.Tensor, num_seqs: int, heads: int, groups: int, state_size: int,
-             value_dim: int, workspace=None) -> None:
+             value_dim: int, workspace=None, longest: int = 0) -> None:
     """The recurrence of a selective state-space layer with one decay per head, all 32-bit:
     ``dt = softplus(dt_raw + dt_bias)``, ``S = exp(-exp(a_log) dt) S + dt B x^T``,
     ``y = S^T C + d_skip x``.  ``xbc [T, heads*vdim + 2*groups*N]`` holds x, B and C side by side;
     ``dt_raw [T, heads]`` may be a strided view; ``state [slots, heads, N, vdim]`` may be a strided
     view of the slots' rows.  A sequence whose first row has position 0 starts from zero.
 
-    With ``workspace`` (where the buffers between its kernels come from) a step whose sequences bring several rows on
-    average runs eight tokens at a time (:func:`linear_scan`); without it, token after token."""
+    With ``workspace`` (where the buffers between its kernels come from) a step in which a sequence brings many rows
+    (``longest``, the most that one brings; 0: not known) runs eight tokens at a time (:func:`linear_scan`) where
+    :func:`ssm_in_blocks` says so; without it, token after token."""
     _check(xbc, "xbc", torch.float32, 2)
     _check(y, "y", torch.float32, 2)
     T = y.shape[0]
@@ -350,7 +360,7 @@ def ssm_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torch.Te
                 raise KernelError(f"ssm_scan: {n} must have one entry per head")
     for t, n in ((seq_start, "seq_start"), (positions, "positions"), (state_slots, "state_slots")):
         _check(t, n, torch.int32, 1)
-    if workspace is not None and ssm_in_blocks(T, num_seqs, heads):
+    if workspace is not None and ssm_in_blocks(T, num_seqs, heads, state_size, value_dim, longest):
         gates = workspace.get("ssm_scan.gates", (2, T, heads), torch.float32)
         call(core(), "ap_ssm_gates", dt_raw.data_ptr(), dt_raw.stride(0), dt_bias.data_ptr() if dt_bias is not None else 0,
              a_log.data_ptr(), gates[0].data_ptr(), gates[1].data_ptr(), T, heads, stream_handle())

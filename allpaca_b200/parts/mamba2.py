@@ -90,10 +90,12 @@ class Mamba2(Mixer):
         xbc = ws.get("mamba.xbc", (T, self.conv_channels), torch.float32)
         ops.causal_conv(proj, self.inner, self.conv_w, self.conv_b, conv_state, step.seq_start, step.positions,
                         step.state_slots, xbc, S)
+        # in bfloat16 a portion's recurrence goes eight tokens at a time where the step's rows make that the faster way: its last bits
+        # depend on the step it shares, as the products' do; in 32 bits a row has the same bits in every step
         y = ws.get("mamba.y", (T, self.inner), torch.float32)
         ops.ssm_scan(xbc, proj[:, self.inner + self.conv_channels:], self.dt_bias, self.a_log, self.d_skip,
                      ssm_state, step.seq_start, step.positions, step.state_slots, y, S, self.heads, self.groups,
-                     self.N, self.vd, workspace=ws if self.env.dtype == torch.bfloat16 else None)
+                     self.N, self.vd, workspace=ws if self.env.dtype == torch.bfloat16 else None, longest=step.max_query_len)
         gated = ws.get("mamba.gated", (T, self.inner), self.env.dtype)
         ops.gated_group_rmsnorm(y, proj[:, :self.inner], self.norm_w, self.eps, gated, self.norm_groups)
         return self.out_proj.forward(gated, "mamba.o", "delta")
