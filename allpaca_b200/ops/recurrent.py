@@ -96,7 +96,9 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, y: torch.Tens
     if workspace is not None:
         block = int(lib.ap_linear_scan_block(T, int(num_seqs), int(heads), int(key_dim), int(value_dim), DECAY_MODES[decay]))
         if block > 0:
-            blocks = (T // 8 + int(num_seqs)) * int(heads)
+            # places for T // 8 + num_seqs blocks a head, the sequences counted in runs of 64: steps of as many rows whose sequences come
+            # and go ask for the same buffer (a larger one moves, and every recorded step that names scratch buffers is recorded again)
+            blocks = (T // 8 + (int(num_seqs) + 63) // 64 * 64) * int(heads)
             scratch = workspace.get("linear_scan.blocks", (blocks * block,), torch.float32).data_ptr()
     call(lib, "ap_linear_scan", qp, ldq, kp, ldk, vp, ldv, dcp, dcl, dhp, dhl,
          decay_const.data_ptr() if decay_const is not None else 0, dt_bias.data_ptr() if dt_bias is not None else 0,

@@ -115,3 +115,17 @@ def test_rows_of_no_sequence(E):
         results.append(y)
     assert all(bool((y[:first] == 7.0).all()) and bool((y[last:] == 7.0).all()) for y in results)
     assert float((results[0] - results[1]).abs().max()) <= 2e-5 * float(results[0].abs().max())
+
+
+def test_scratch_of_steps_of_as_many_rows():
+    """More sequences in a step of as many rows ask for no other buffers: a larger one would have the engine record its graphs again."""
+    from allpaca_b200 import ops
+    Hh, E, N, T = 4, 32, 64, 160
+    ws, seen = Workspace(torch.device(DEV)), []
+    for seqs in (1, 2, 5, 20, 40):
+        n = T // seqs
+        ops.ssm_scan(torch.randn(T, Hh * E + 2 * N, device=DEV), torch.randn(T, Hh, device=DEV), None, torch.zeros(Hh, device=DEV), None,
+                     torch.zeros(seqs, Hh, N, E, device=DEV), i32([n * i for i in range(seqs + 1)]), i32(list(range(n)) * seqs),
+                     i32(list(range(seqs))), torch.empty(T, Hh * E, device=DEV), seqs, Hh, 1, N, E, workspace=ws, longest=T)
+        seen.append(ws.generation)
+    assert len(set(seen)) == 1
