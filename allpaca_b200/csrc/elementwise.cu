@@ -624,8 +624,8 @@ rope_kv_store_bf16x8_kernel(const bf16* __restrict__ in, bf16* __restrict__ q_ou
     }
 }
 
-// The same for a step of many rows, a thread taking the same eight pairs of RUN neighbouring heads (or RUN runs of V side by side):
-// the row's cosines and sines, twice a pair's own bytes, are read once for them, and the heads' loads are in flight together.  Traffic
+// The same for a step of many rows, a thread taking the same eight pairs of RUN neighbouring heads (or RUN runs of V, as far apart as the
+// row has threads for V): the row's cosines and sines, twice a pair's own bytes, are read once for them, and the heads' loads are in flight together.  Traffic
 // bounds it then: 2048 rows of 32 + 8 + 8 heads of 128 15.6 -> 12.1 us (4.2 TB/s of 25 MB in, 25 MB out; the table comes from L2).
 #define ROPE_RUN 4
 __global__ void __launch_bounds__(ROPE_THREADS)
@@ -699,7 +699,7 @@ rope_kv_store_rows_kernel(const bf16* __restrict__ in, bf16* __restrict__ q_out,
             *reinterpret_cast<uint4*>(dst + i + half) = rb4;
         }
     } else {
-        // V: runs of eight elements, the thread's RUN of them a warp apart in the row
+        // V: runs of eight elements, the thread's RUN of them `per` apart in the row
         const int runs = nkv * (hd >> 3), per = threads - rot_threads, first = item - rot_threads;
         uint4 v[ROPE_RUN];
 #pragma unroll
@@ -737,7 +737,15 @@ AP_EXPORT int ap_rope_kv_store(const void* in, int in_dtype, int S, long long in
         // (heads without a place in the cache are rotated by nobody: then only the queries are taken)
         const int rot_threads = ((cache ? nh + nkv : nh) + ROPE_RUN - 1) / ROPE_RUN * (hd / 16);
         const int threads = rot_threads + (cache ? (nkv * (hd / 8) + ROPE_RUN - 1) / ROPE_RUN : 0);
-        if (T >= 256 && (long long)T * threads < (1LL << 31)) {
+        // Four heads to a thread leave a quarter of the threads, so the kernel pays where the step still fills the SMs with them and a thread's
+        // loads are long runs (heads of 112 and more), or where the other kernel's CTAs, one to a row, stay mostly empty.  Measured (us, eight pairs
+        // of one head to a thread and of four): 32 + 8 + 8 heads of 128: 512 rows 5.0 and 5.4, 768 6.0 and 5.6, 2048 12.4 and 11.0, 8192 48.7 and 38.3;
+        // 16 + 8 + 8: 640 rows 4.5 and 5.2, 1024 5.8 and 5.7, 2048 10.0 and 9.1; 4 + 2 + 2 heads of 64: 768 rows 2.7 and 3.6, 1024 3.9 and 3.6, 4096 8.8 and
+        // 5.8.  Shorter heads in steps up to some 4096 rows lose (32 + 8 + 8 of 64: 1024 rows 4.7 and 6.2, 4096 11.6 and 12.8, 8192 25.7 and 24.8).
+        const int all_items = (nh + nkv) * (hd / 16) + nkv * (hd / 8);
+        const long long all_threads = (nh + nkv + ROPE_RUN - 1) / ROPE_RUN * (hd / 16) + (nkv * (hd / 8) + ROPE_RUN - 1) / ROPE_RUN;
+        const bool rows = T >= 8192 || (T >= 1024 && all_items <= 40) || (hd >= 112 && all_threads >= 64 && T * all_threads >= 80000);
+        if (rows && (long long)T * threads < (1LL << 31)) {
             const unsigned ctas = (unsigned)(((long long)T * threads + ROPE_THREADS - 1) / ROPE_THREADS);
             AP_CHECK_PDL_LAUNCH("rope_kv_store", ap_launch_pdl(
                 rope_kv_store_rows_kernel, dim3(ctas), dim3(ROPE_THREADS), 0, stream, (const bf16*)in, (bf16*)q_out, (bf16*)cache,
