@@ -418,7 +418,8 @@ template <typename T>
 __global__ void clear_page_tails_kernel(T* __restrict__ pages, size_t run_stride, size_t page_stride, int runs,
                                         int outer, int P, int inner, const int* __restrict__ positions,
                                         const int* __restrict__ token_seq, const int* __restrict__ block_table,
-                                        int max_blocks, const int* __restrict__ context_lens) {
+                                        int max_blocks, const int* __restrict__ context_lens, unsigned step_runs,
+                                        unsigned step_outer) {
     const int t = blockIdx.x;
     const int pos = positions[t];
     if (pos % P != 0) return;
@@ -426,12 +427,18 @@ __global__ void clear_page_tails_kernel(T* __restrict__ pages, size_t run_stride
     const int page = block_table[(size_t)seq * max_blocks + pos / P];
     const int first = context_lens[seq] - pos;          // slots 0 .. first-1 are written by this step's rows
     if (page < 0 || first >= P) return;
-    // the cleared slots of one plane are contiguous: a warp takes a plane at a time
-    const int per_plane = (P - first) * inner, planes = runs * outer, lane = threadIdx.x & 31;
-    for (int plane = blockIdx.y * CLEAR_WARPS + (threadIdx.x >> 5); plane < planes; plane += gridDim.y * CLEAR_WARPS) {
-        const int run = plane / outer, o = plane - run * outer;
+    // the cleared slots of one plane are contiguous: a warp takes a plane at a time, and steps to its next by the row's warps as whole
+    // runs and planes (their product, which may be large, is formed nowhere)
+    const size_t per_plane = (size_t)(P - first) * inner;
+    const unsigned warp = blockIdx.y * CLEAR_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31, planes = (unsigned)outer;
+    unsigned run = warp / planes, o = warp - run * planes;
+    for (; run < (unsigned)runs; run += step_runs, o += step_outer) {
+        if (o >= planes) {
+            o -= planes;
+            if (++run >= (unsigned)runs) break;
+        }
         T* p = pages + run * run_stride + (size_t)page * page_stride + ((size_t)o * P + first) * inner;
-        for (int e = lane; e < per_plane; e += 32) p[e] = T{};
+        for (size_t e = lane; e < per_plane; e += 32) p[e] = T{};
     }
 }
 
@@ -449,14 +456,15 @@ AP_EXPORT int ap_clear_page_tails(void* pages, int elem_bytes, long long run_str
            (run_stride * elem_bytes) % (unit * 2) == 0 && (page_stride * elem_bytes) % (unit * 2) == 0)
         unit *= 2;
     const int scale = (int)(unit / elem_bytes);
-    AP_REQUIRE((long long)runs * outer < (1LL << 30) && (long long)P * inner < (1LL << 30), "clear_page_tails: a page of %d x %d x %d", runs, outer, P);
     // many CTAs to a row where few rows ask (a step of single rows), few where most rows are not the first of a page
     dim3 grid(T, T <= 64 ? 32 : 8);
+    const unsigned warps = grid.y * CLEAR_WARPS;
 #define LAUNCH(TT)                                                                                            \
     clear_page_tails_kernel<TT><<<grid, CLEAR_WARPS * 32, 0, stream>>>((TT*)pages, (size_t)(run_stride / scale),          \
                                                           (size_t)(page_stride / scale), runs, outer, P,     \
                                                           inner / scale, positions, token_seq, block_table,   \
-                                                          max_blocks, context_lens)
+                                                          max_blocks, context_lens, warps / (unsigned)outer,  \
+                                                          warps % (unsigned)outer)
     if (unit == 16) LAUNCH(uint4);
     else if (unit == 8) LAUNCH(unsigned long long);
     else if (unit == 4) LAUNCH(unsigned int);
