@@ -7,6 +7,8 @@
 // Reference counterparts (cuda/src/kernels.cu): embed_gather_kernel :1198,
 // rmsnorm_kernel :1152 with residual_add_kernel :649, rope_qk_kernel :1244 with the
 // page writes of crates/allpaca-core/src/kv_tier.rs:1101-1203, silu_mul_kernel :775.
+#include <algorithm>
+
 #include "common.cuh"
 
 // ---------------------------------------------------------------------------
@@ -456,8 +458,11 @@ AP_EXPORT int ap_clear_page_tails(void* pages, int elem_bytes, long long run_str
            (run_stride * elem_bytes) % (unit * 2) == 0 && (page_stride * elem_bytes) % (unit * 2) == 0)
         unit *= 2;
     const int scale = (int)(unit / elem_bytes);
-    // many CTAs to a row where few rows ask (a step of single rows), few where most rows are not the first of a page
-    dim3 grid(T, T <= 64 ? 32 : 8);
+    // Up to 32 CTAs to a row where few rows ask (a step of single rows), up to 8 where most rows are not the first of a page, and none beyond a
+    // warp to each plane.  64 rows of 512 planes, us, with 8 CTAs to a row and with 32: no row begins a page 1.5 and 2.1, one does 6.0 and 4.2 (pages of 128
+    // slots 35 and 18), all do 23.7 and 20.8; 8 planes, which one CTA clears: 1.4 instead of 2.1, all rows 2.3 instead of 3.0.
+    const long long plane_ctas = ((long long)runs * outer + CLEAR_WARPS - 1) / CLEAR_WARPS;
+    dim3 grid(T, (unsigned)std::min(plane_ctas, T <= 64 ? 32LL : 8LL));
     const unsigned warps = grid.y * CLEAR_WARPS;
 #define LAUNCH(TT)                                                                                            \
     clear_page_tails_kernel<TT><<<grid, CLEAR_WARPS * 32, 0, stream>>>((TT*)pages, (size_t)(run_stride / scale),          \
