@@ -10,7 +10,7 @@
 //   the eight CTAs of a cluster, which add up through distributed shared memory; else a CTA walks all of K and keeps
 //   the finished runs' sum beside the current one.
 // * beyond, tiles of 64 to 176 rows x 96, 112 or 128 columns, always a cluster of eight per tile: up to 11 x 14 outputs to a thread (a
-//   byte read from shared memory serves 6.2 multiply-adds; at 8 x 8 the reads take as long as the arithmetic).
+//   number read from shared memory serves 6.2 multiply-adds, at 8 x 8, where the reads take as long as the arithmetic, 4).
 //
 // Measured (one B200, weights rotating over more than L2; in brackets the 64 x 64 tiles of gemm_simt.cu, which load 4 bytes
 // at a time), us:
@@ -389,12 +389,57 @@ bool gemm_f32_takes(const void* a, const void* w, long long K, long long lda, lo
     return K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
 }
 
+// The tile of a product of more than 32 rows, by what its clusters take (one B200, tenths of a us at K = 2048; the same ratios at K = 512 and 8192).
+// 33 clusters of 8 run at once, two CTAs to an SM (the last of them often only in the next round), and a round takes `full`; up to 10 clusters have an SM to a CTA and take
+// `alone`, up to 14 something between.  Of 4 x 16 outputs a thread 48 clusters run at once, three to an SM, and a last round that is not full
+// takes as much less as one alone.  The tile that leaves the fewest rows empty (the larger of two equals) is taken unless another is 2 %
+// cheaper: 173 rows x 3072 one round of 11 x 12 in place of two of 6 x 16 (63 us against 99), x 16384 five of 11 x 14 in place of eight (354 against
+// 397); 448 rows x 16384 stay with 4 x 16 (888 us; 6 x 16 983), 144 rows x 1024 take it (39; 6 x 16 49).  Of 1213 products measured (33 to 2048 rows,
+// 256 to 16384 columns, K of 512 to 8192) the tile so chosen takes 0.5 % longer than the best one on average, 11 % at most; ten take 3 to 8 %
+// longer than with the fewest empty rows, all of them together 8 % less.  Every tile gives the same bits.
+struct F32Tile { int rm, cn, full, alone; };
+static const F32Tile f32_tiles[] = {{8, 16, 620, 390}, {6, 16, 500, 330}, {4, 16, 0, 0},    {8, 12, 490, 325},
+                                    {10, 12, 575, 375}, {11, 12, 630, 400}, {11, 14, 720, 450}};
+
+static long long f32_tile_cost(long long M, long long N, const F32Tile& t) {
+    const long long clusters = ((M + 16 * t.rm - 1) / (16 * t.rm)) * ((N + 8 * t.cn - 1) / (8 * t.cn));
+    if (t.rm == 4) {
+        const int rest = (int)(clusters % 48);
+        return clusters / 48 * 500 + (rest == 0 ? 0 : rest <= 10 ? 280 : rest <= 14 ? 300 : rest <= 17 ? 380 : rest <= 24 ? 430 : rest <= 33 ? 510 : 540);
+    }
+    return clusters <= 10 ? t.alone : clusters <= 14 ? t.full * 85 / 100 : t.full * (clusters / 33 + 1);
+}
+
+static const F32Tile& f32_tile(int M, int N) {
+    int pick = 0;
+    for (int i = 1; i < 3; ++i) {
+        const auto rows = [M](const F32Tile& t) { return ((long long)M + 16 * t.rm - 1) / (16 * t.rm) * (16 * t.rm); };
+        if (rows(f32_tiles[i]) < rows(f32_tiles[pick])) pick = i;
+    }
+    long long least = f32_tile_cost(M, N, f32_tiles[pick]) * 98 / 100;
+    for (int i = 0; i < 7; ++i) {
+        const long long cost = f32_tile_cost(M, N, f32_tiles[i]);
+        if (cost < least && ((long long)M + 16 * f32_tiles[i].rm - 1) / (16 * f32_tiles[i].rm) <= 65535) {
+            least = cost;
+            pick = i;
+        }
+    }
+    return f32_tiles[pick];
+}
+
+// the outputs to a thread of the tile that a product of M rows and N columns takes (rows x 100 + columns); 0: the few-rows kernel's
+AP_EXPORT int ap_gemm_f32_tile(int M, int N) {
+    if (M <= F32_FEW_ROWS || N <= 0) return 0;
+    const F32Tile& t = f32_tile(M, N);
+    return t.rm * 100 + t.cn;
+}
+
 int gemm_f32(const float* a, const float* w, float* out, int M, int N, int K, long long lda, long long ldw, long long ldc,
              cudaStream_t stream) {
     const int tiles_n = (N + F32_BN - 1) / F32_BN;
     CUtensorMap tw, ta;
-    AP_REQUIRE(f32_make_map(&tw, w, N, K, ldw, F32_BN), "gemm_f32: cannot encode the weight's tensor map");
     if (M <= F32_FEW_ROWS) {
+        AP_REQUIRE(f32_make_map(&tw, w, N, K, ldw, F32_BN), "gemm_f32: cannot encode the weight's tensor map");
         const int a_rows = (M + 7) / 8 * 8;
         AP_REQUIRE(f32_make_map(&ta, a, M, K, lda, a_rows), "gemm_f32: cannot encode the rows' tensor map");
         const size_t smem = F32_FEW_STAGES * (size_t)(F32_W_BYTES + F32_FEW_ROWS * F32_BK * 4) + 2 * F32_FEW_STAGES * 8 + 16 + 1024;
@@ -414,23 +459,7 @@ int gemm_f32(const float* a, const float* w, float* out, int M, int N, int K, lo
         FEW(8);
 #undef FEW
     }
-    // A round of clusters takes about 28 + outputs to a thread, whatever K (us at K = 2048, one round: 4 x 16 outputs 38, 6 x 16 50, 8 x 16 61,
-    // 8 x 12 48, 10 x 12 57, 11 x 12 62, 11 x 14 71), and 34 clusters of 8 run at once (more than 272 CTAs of two to an SM make a second
-    // round), so the tile with the least of rounds x (28 + outputs) is taken, one of 128 columns unless another has 6 % less (512 rows x 16384:
-    // 968 us in 8 x 16, 985 in 11 x 14, which the rule alone would prefer by 5 %): 173 rows x 3072 one round of 11 x 12 instead of two of
-    // 6 x 16 (62 against 98 us), x 16384 five of 11 x 14 instead of eight (353 against 396).  Every tile gives the same bits.
-    static const int shapes[][2] = {{8, 16}, {6, 16}, {4, 16}, {8, 12}, {10, 12}, {11, 12}, {11, 14}};
-    int rm = 8, cn = 16;
-    long long least = -1;
-    for (const auto& s : shapes) {
-        const long long clusters = (long long)((M + 16 * s[0] - 1) / (16 * s[0])) * ((N + 8 * s[1] - 1) / (8 * s[1]));
-        const long long cost = (clusters + 33) / 34 * (28 + s[0] * s[1]) * (s[1] == 16 ? 94 : 100);
-        if (least < 0 || cost < least) {
-            least = cost;
-            rm = s[0];
-            cn = s[1];
-        }
-    }
+    const int rm = f32_tile(M, N).rm, cn = f32_tile(M, N).cn;
     const dim3 grid((unsigned)((N + 8 * cn - 1) / (8 * cn)) * F32_SEGS, (unsigned)((M + 16 * rm - 1) / (16 * rm)));
     AP_REQUIRE(grid.y <= 65535, "gemm: %d rows exceed the grid of the CUDA-core kernel", M);
     AP_REQUIRE(f32_make_map(&tw, w, N, K, ldw, 8 * cn), "gemm_f32: cannot encode the weight's tensor map");

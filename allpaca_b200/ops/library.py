@@ -75,6 +75,8 @@ _CORE_SIGNATURES = {
     # int ap_causal_conv(in, ld_in, col0, in_bias, w, bias, act, state, state_stride, seq_start, positions,
     #                    state_slots, out, T, nseq, C, taps, stream)
     "ap_causal_conv": [_P, _L, _I, _P, _P, _P, _I, _P, _L, _P, _P, _P, _P, _I, _I, _I, _I, _P],
+    # int ap_gemm_f32_tile(M, N): outputs to a thread, rows x 100 + columns
+    "ap_gemm_f32_tile": [_I, _I],
     # int ap_ssm_gates(dt_raw, ld_dt, dt_bias, a_log, dt, decay, T, heads, stream); ap_ssm_skip(y, x, ld_x, d_skip, seq_start, T, nseq, heads,
     #                                                                                                  vdim, stream)
     "ap_ssm_gates": [_P, _L, _P, _P, _P, _P, _I, _I, _P],

@@ -1,4 +1,4 @@
-"""The 32-bit product against a 64-bit one at the edges of its two kernels (up to 32 rows, tiles of 64, 96 and 128 rows; a
+"""The 32-bit product against a 64-bit one at the edges of its two kernels (up to 32 rows, tiles of 64 to 176 rows; a
 tile's K over a cluster or over one CTA), and one order of sums for every number of rows."""
 import pytest
 import torch
@@ -9,8 +9,9 @@ ROWS = [1, 4, 5, 8, 9, 16, 17, 24, 25, 32, 33, 64, 65, 96, 97, 128, 129, 173, 25
 
 
 # N: one tile, a ragged second one, more tiles than the cluster form is used for; K: less than one block, a ragged last
-# block, runs of unequal length, empty runs
-@pytest.mark.parametrize("N,K", [(128, 32), (130, 4), (97, 100), (256, 256), (300, 1000), (129, 2052), (38000, 96)])
+# block, runs of unequal length, empty runs.  Beyond 32 rows the first six take tiles of 64 and 96 rows, the last ones the others too
+@pytest.mark.parametrize("N,K", [(128, 32), (130, 4), (97, 100), (256, 256), (300, 1000), (129, 2052), (38000, 96), (2503, 1000),
+                                 (3505, 2052)])
 def test_rows_of_any_batch(N, K):
     from allpaca_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(N + K)

@@ -1,16 +1,19 @@
-"""The 32-bit product's tiles beyond 32 rows, each at sizes for which the rule takes it (ragged rows and columns among them): the bits of
-single rows, which another kernel forms, and the 64-bit sums."""
+"""The 32-bit product's tiles beyond 32 rows, each at sizes for which the rule takes it (ragged rows and columns among them), with fewer
+blocks of K to a CTA than the operand ring holds and with three times as many: the bits of single rows, which another kernel forms, and the 64-bit
+sums."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
-# outputs to a thread: 4 x 16, 6 x 16, 8 x 12, 8 x 16, 10 x 12, 11 x 14, 11 x 12, then several row tiles
-@pytest.mark.parametrize("M, N", [(33, 1000), (65, 2503), (97, 2503), (97, 3505), (129, 2503), (129, 3505), (161, 2503),
-                                  (300, 3072), (353, 3000)])
-def test_every_tile_has_the_bits_of_single_rows(M, N, K=260):
+# outputs to a thread as rows x 100 + columns; the last ones with several row tiles
+@pytest.mark.parametrize("M, N, tile", [(33, 1000, 416), (65, 2503, 616), (97, 2503, 812), (97, 3505, 816), (129, 2503, 1012), (129, 3505, 1114),
+                                        (161, 2503, 1112), (300, 3072, 1012), (353, 3000, 812), (512, 1000, 816), (700, 3072, 1112)])
+@pytest.mark.parametrize("K", [260, 2052])
+def test_every_tile_has_the_bits_of_single_rows(M, N, tile, K):
     from allpaca_b200 import ops
+    assert ops.core().ap_gemm_f32_tile(M, N) == tile
     g = torch.Generator(device="cuda").manual_seed(M + N)
     a = torch.randn(M, K, generator=g, device="cuda")
     w = torch.randn(N, K, generator=g, device="cuda")
