@@ -490,8 +490,11 @@ def bench_recurrent(args) -> dict:
     }
     # the state-space recurrence with the same state per head: B and C of D numbers, one group per head
     xbc = [rnd(T, H * V + 2 * H * D) for _ in range(copies)]
-    cases["ssm_scan"] = (lambda i: ops.ssm_scan(xbc[i % copies], a, dt_bias, a_log, consts, state, seq_start, positions,
-                                                slots, y, S, H, H, D, V), io)
+    cases["ssm_scan, token after token"] = (lambda i: ops.ssm_scan(xbc[i % copies], a, dt_bias, a_log, consts, state, seq_start, positions,
+                                                                   slots, y, S, H, H, D, V), io)
+    cases["ssm_scan, as a bfloat16 engine runs it"] = (
+        lambda i: ops.ssm_scan(xbc[i % copies], a, dt_bias, a_log, consts, state, seq_start, positions, slots, y, S, H, H, D, V,
+                               workspace=ws, longest=n), io)
     gate = [rnd(T, H * V) for _ in range(copies)]
     out = torch.empty(T, H * V, device=dev, dtype=torch.bfloat16)
     nw = torch.ones(V, device=dev)
@@ -506,7 +509,7 @@ def bench_recurrent(args) -> dict:
     copy = torch.empty(T, W, device=dev, dtype=torch.bfloat16)
     w32, gb = torch.ones(W, device=dev), rnd(W)
     cases["gated_postnorm"] = (lambda i: ops.gated_postnorm(xs[i % wc], w32, args.groups, 1e-6, alpha=2.0, delta=ds[i % wc],
-                                                            gate=gs[i % wc], gate_bias=gb, copy=copy), T * W * 18)
+                                                            gate=gs[i % wc], gate_bias=gb, copy=copy, settled=True), T * W * 18)
     cases["norm_residual"] = (lambda i: ops.norm_residual(xs[i % wc], ds[i % wc], w32, 1e-6, 0.5, copy), T * W * 14)
     cases["add_rmsnorm"] = (lambda i: ops.add_rmsnorm(xs[i % wc], w32.to(torch.bfloat16), 1e-6, copy, delta=ds[i % wc]),
                             T * W * 14)
