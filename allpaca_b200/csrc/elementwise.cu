@@ -639,7 +639,7 @@ rope_kv_store_bf16x8_kernel(const bf16* __restrict__ in, bf16* __restrict__ q_ou
 
 // The same for a step of many rows, a thread taking the same eight pairs of RUN neighbouring heads (or RUN runs of V, as far apart as the
 // row has threads for V): the row's cosines and sines, twice a pair's own bytes, are read once for them, and the heads' loads are in flight together.  Traffic
-// bounds it then: 2048 rows of 32 + 8 + 8 heads of 128 15.6 -> 12.1 us (4.2 TB/s of 25 MB in, 25 MB out; the table comes from L2).
+// bounds it then: 2048 rows of 32 + 8 + 8 heads of 128 12.4 -> 11.0 us (4.6 TB/s of 25 MB in, 25 MB out; the table comes from L2).
 #define ROPE_RUN 4
 __global__ void __launch_bounds__(ROPE_THREADS)
 rope_kv_store_rows_kernel(const bf16* __restrict__ in, bf16* __restrict__ q_out, bf16* __restrict__ cache,
