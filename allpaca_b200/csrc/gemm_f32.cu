@@ -395,17 +395,17 @@ bool gemm_f32_takes(const void* a, const void* w, long long K, long long lda, lo
 // takes as much less as one alone.  The tile that leaves the fewest rows empty (the larger of two equals) is taken unless another is 2 %
 // cheaper: 173 rows x 3072 one round of 11 x 12 in place of two of 6 x 16 (63 us against 99), x 16384 five of 11 x 14 in place of eight (354 against
 // 397); 448 rows x 16384 stay with 4 x 16 (888 us; 6 x 16 983), 144 rows x 1024 take it (39; 6 x 16 49).  Of 1213 products measured (33 to 2048 rows,
-// 256 to 16384 columns, K of 512 to 8192) the tile so chosen takes 0.5 % longer than the best one on average, 11 % at most; ten take 3 to 8 %
+// 256 to 16384 columns, K of 512 to 8192) the tile so chosen takes 0.3 % longer than the best one on average, 10 % at most; 15 take 3 to 10 %
 // longer than with the fewest empty rows, all of them together 8 % less.  Every tile gives the same bits.
 struct F32Tile { int rm, cn, full, alone; };
-static const F32Tile f32_tiles[] = {{8, 16, 620, 390}, {6, 16, 500, 330}, {4, 16, 0, 0},    {8, 12, 490, 325},
-                                    {10, 12, 575, 375}, {11, 12, 630, 400}, {11, 14, 720, 450}};
+static const F32Tile f32_tiles[] = {{8, 16, 615, 390}, {6, 16, 500, 330}, {4, 16, 0, 0},    {8, 12, 485, 325},
+                                    {10, 12, 585, 375}, {11, 12, 640, 400}, {11, 14, 715, 450}};
 
 static long long f32_tile_cost(long long M, long long N, const F32Tile& t) {
     const long long clusters = ((M + 16 * t.rm - 1) / (16 * t.rm)) * ((N + 8 * t.cn - 1) / (8 * t.cn));
     if (t.rm == 4) {
         const int rest = (int)(clusters % 48);
-        return clusters / 48 * 500 + (rest == 0 ? 0 : rest <= 10 ? 280 : rest <= 14 ? 300 : rest <= 17 ? 380 : rest <= 24 ? 430 : rest <= 33 ? 510 : 540);
+        return clusters / 48 * 500 + (rest == 0 ? 0 : rest <= 10 ? 280 : rest <= 14 ? 300 : rest <= 17 ? 380 : rest <= 24 ? 410 : rest <= 33 ? 530 : 540);
     }
     return clusters <= 10 ? t.alone : clusters <= 14 ? t.full * 85 / 100 : t.full * (clusters / 33 + 1);
 }

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 # outputs to a thread as rows x 100 + columns; the last ones with several row tiles
-@pytest.mark.parametrize("M, N, tile", [(33, 1000, 416), (65, 2503, 616), (97, 2503, 812), (97, 3505, 816), (129, 2503, 1012), (129, 3505, 1114),
+@pytest.mark.parametrize("M, N, tile", [(33, 1000, 416), (65, 3505, 616), (65, 2503, 812), (97, 2503, 812), (97, 3505, 816), (129, 2503, 1012), (129, 3505, 1114),
                                         (161, 2503, 1112), (300, 3072, 1012), (353, 3000, 812), (512, 1000, 816), (700, 3072, 1112)])
 @pytest.mark.parametrize("K", [260, 2052])
 def test_every_tile_has_the_bits_of_single_rows(M, N, tile, K):
